@@ -71,6 +71,7 @@ struct Params {
     const double* cheb;    // [n_grid][1 + phi*NS][kChebN] coefficients (NULL: direct)
     const double* cheb_mid;
     const double* cheb_half;
+    const double* tgrid;   // mixed form: n_grid x kChebG Chebyshev values at the grid points
     // Weighted x-sums of every table row r (grid rows, the ones row n_grid, the null rows
     // n_grid+1+f), produced for the whole chunk by two FP64 GEMMs:
     //   CL[j*ldcl + r*(C+phi) + a] = sum_i h_r,i x_ij w_a,i  (a < C)
@@ -388,225 +389,6 @@ __device__ __forceinline__ double eval_logl(const Params& p, const double* x, co
     return REML ? reml_logl<C>(pb, log_iab, logdet, p) : mle_logl<C>(pb, logdet, p);
 }
 
-// Chebyshev series sum_j c_j T_j(t) by Clenshaw's recurrence.
-__device__ __forceinline__ double cheb_eval(const double* __restrict__ c, double t) {
-    double b1 = 0.0, b2 = 0.0;
-    const double t2 = 2.0 * t;
-#pragma unroll 5
-    for (int j = kChebN - 1; j >= 1; --j) {
-        const double b0 = fma(t2, b1, c[j] - b2);
-        b2 = b1;
-        b1 = b0;
-    }
-    return fma(t, b1, c[0] - b2);
-}
-
-// Mixed form: the c+2 x-dependent sums at log-lambda `s` from the SNP's global Chebyshev
-// coefficients (chunk GEMM rows 1..kChebG), by Clenshaw's recurrence.  Every lane
-// computes the same values (broadcast loads), so the warp stays uniform.
-template <int C>
-__device__ __forceinline__ void series_xsums(const Params& p, int64_t j, int f, double s,
-                                             double (&xs)[Lay<C>::NX]) {
-    using L = Lay<C>;
-    const int64_t cp = C + p.phi;
-    const double* __restrict__ cl = p.CL + j * p.ldcl;
-    const double* __restrict__ cq = p.CQ + j * p.ldcq;
-    const double tt = (s - p.gmid) * p.ginv;
-    const double t2 = 2.0 * tt;
-    double b1[L::NX], b2[L::NX];
-#pragma unroll
-    for (int q = 0; q < L::NX; ++q) b1[q] = b2[q] = 0.0;
-#pragma unroll 4
-    for (int k = kChebG - 1; k >= 1; --k) {
-        const double* rl = cl + (1 + k) * cp;
-        double c[L::NX];
-#pragma unroll
-        for (int a = 0; a < C; ++a) c[a] = __ldg(rl + a);
-        c[C] = __ldg(cq + 1 + k);
-        c[C + 1] = __ldg(rl + C + f);
-#pragma unroll
-        for (int q = 0; q < L::NX; ++q) {
-            const double b0 = fma(t2, b1[q], c[q] - b2[q]);
-            b2[q] = b1[q];
-            b1[q] = b0;
-        }
-    }
-    const double* rl = cl + cp;
-    double c[L::NX];
-#pragma unroll
-    for (int a = 0; a < C; ++a) c[a] = __ldg(rl + a);
-    c[C] = __ldg(cq + 1);
-    c[C + 1] = __ldg(rl + C + f);
-#pragma unroll
-    for (int q = 0; q < L::NX; ++q) xs[q] = fma(tt, b1[q], c[q] - b2[q]);
-}
-
-// ---------------------------------------------------------------- warp-cooperative series
-// Chebyshev values for a series summed across the warp: lane l gets T_l(x) (l = 0..31)
-// and every lane T_32(x), by the doubling identity T_{a+b} = 2 T_a T_b - T_{a-b} (round r
-// fills lanes 2^r+1 .. 2^(r+1) from lanes already known).
-__device__ __forceinline__ void lane_cheb(double x, double& tl, double& t32) {
-    const int lane = threadIdx.x & 31;
-    tl = lane == 0 ? 1.0 : x;
-#pragma unroll
-    for (int r = 0; r < 5; ++r) {
-        const int a = 1 << r;
-        const bool act = lane > a && lane <= 2 * a;
-        const double ta = __shfl_sync(0xffffffffu, tl, a);
-        const double tb = __shfl_sync(0xffffffffu, tl, act ? lane - a : 0);
-        const double tc = __shfl_sync(0xffffffffu, tl, act ? 2 * a - lane : 0);
-        if (act) tl = fma(2.0 * ta, tb, -tc);
-    }
-    const double t16 = __shfl_sync(0xffffffffu, tl, 16);
-    t32 = fma(2.0 * t16, t16, -1.0);
-}
-
-// T_k(x) for the coefficients a lane owns: k = lane + 32 i, i < kCoefPerLane.
-struct LaneT {
-    double t[kCoefPerLane];
-};
-__device__ __forceinline__ LaneT lane_cheb_global(double x) {
-    const int lane = threadIdx.x & 31;
-    double tl, t32;
-    lane_cheb(x, tl, t32);
-    const double tm = __shfl_sync(0xffffffffu, tl, (32 - lane) & 31);  // T_{32-l}
-    LaneT r;
-    r.t[0] = tl;
-    r.t[1] = fma(2.0 * t32, tl, -(lane == 0 ? t32 : tm));  // T_{l+32}
-#pragma unroll
-    for (int i = 2; i < kCoefPerLane; ++i)
-        r.t[i] = fma(2.0 * t32, r.t[i - 1], -r.t[i - 2]);   // T_{l+32i}
-    return r;
-}
-
-// Per-(SNP, phenotype) coefficients of the global x-sum series, spread over the warp
-// (lane l holds k = l + 32 i of every series), loaded once per SNP.
-template <int C>
-struct GlobalCoef {
-    double c[Lay<C>::NX][kCoefPerLane];
-};
-template <int C>
-__device__ __forceinline__ GlobalCoef<C> load_global_coef(const Params& p, int64_t j, int f) {
-    const int lane = threadIdx.x & 31;
-    const int64_t cp = C + p.phi;
-    GlobalCoef<C> g;
-#pragma unroll
-    for (int i = 0; i < kCoefPerLane; ++i) {
-        const int64_t r = 1 + lane + 32 * i;
-        const double* rl = p.CL + j * p.ldcl + r * cp;
-#pragma unroll
-        for (int a = 0; a < C; ++a) g.c[a][i] = __ldg(rl + a);
-        g.c[C][i] = __ldg(p.CQ + j * p.ldcq + r);
-        g.c[C + 1][i] = __ldg(rl + C + f);
-    }
-    return g;
-}
-
-// The c+2 x-dependent sums at log-lambda s; identical bits in every lane.
-template <int C>
-__device__ __forceinline__ void coop_xsums(const Params& p, const GlobalCoef<C>& g, double s,
-                                           double (&xs)[Lay<C>::NX]) {
-    const LaneT T = lane_cheb_global((s - p.gmid) * p.ginv);
-#pragma unroll
-    for (int q = 0; q < Lay<C>::NX; ++q) {
-        double v = g.c[q][0] * T.t[0];
-#pragma unroll
-        for (int i = 1; i < kCoefPerLane; ++i) v = fma(g.c[q][i], T.t[i], v);
-        xs[q] = warp_sum(v);
-    }
-}
-
-// Per-bracket expansions of log|H^-1| and the x-free sums of phenotype f (degree 24 over
-// the golden bracket of grid index `best`): lane j < kChebN holds coefficient j.
-template <int C>
-struct BracketCoef {
-    double c[1 + Lay<C>::NS];
-    double mid, inv_half;
-};
-template <int C>
-__device__ __forceinline__ BracketCoef<C> load_bracket_coef(const Params& p, int best, int f) {
-    using L = Lay<C>;
-    const int lane = threadIdx.x & 31;
-    const int nf = 1 + p.phi * L::NS;
-    const double* cb = p.cheb + (int64_t)best * nf * kChebN;
-    BracketCoef<C> b;
-    b.c[0] = lane < kChebN ? __ldg(cb + lane) : 0.0;
-#pragma unroll
-    for (int k = 0; k < L::NS; ++k)
-        b.c[1 + k] = lane < kChebN ? __ldg(cb + (1 + f * L::NS + k) * kChebN + lane) : 0.0;
-    b.mid = p.cheb_mid[best];
-    b.inv_half = 1.0 / p.cheb_half[best];
-    return b;
-}
-
-// log|H^-1| and the x-free sums at log-lambda s inside the bracket; identical bits in
-// every lane.
-template <int C>
-__device__ __forceinline__ void coop_shared(const BracketCoef<C>& b, double s, double& logdet,
-                                            double (&shared)[Lay<C>::NS]) {
-    double tl, t32;
-    lane_cheb((s - b.mid) * b.inv_half, tl, t32);
-    logdet = warp_sum(b.c[0] * tl);
-#pragma unroll
-    for (int k = 0; k < Lay<C>::NS; ++k) shared[k] = warp_sum(b.c[1 + k] * tl);
-}
-
-// Mixed-form log-likelihood at log-lambda s with no length-n pass: the x-dependent sums
-// from the SNP's global series, log|H^-1| and the x-free sums from the bracket's expansions
-// (exact FP64 node values).  The golden-section probes use it; the final evaluation at
-// the optimum takes the same steps in lmm_pairs_kernel, where direct_fix may replace the
-// x-dependent sums by direct ones at large lambda.  pb receives the Pab rows.
-template <int C, bool REML>
-__device__ __forceinline__ double coop_eval(const Params& p, const GlobalCoef<C>& g,
-                                            const BracketCoef<C>& b, double s,
-                                            const double (&log_iab)[C + 1], PabOut<C>& pb) {
-    using L = Lay<C>;
-    double xs[L::NX], shared[L::NS], logdet;
-    coop_xsums<C>(p, g, s, xs);
-    coop_shared<C>(b, s, logdet, shared);
-    double row0[L::NI];
-    assemble<C>(row0, shared, xs);
-    pb = pab_reduce<C>(row0);
-    return REML ? reml_logl<C>(pb, log_iab, logdet, p) : mle_logl<C>(pb, logdet, p);
-}
-
-template <int C, bool REML>
-__device__ __forceinline__ double coop_logl(const Params& p, const GlobalCoef<C>& g,
-                                            const BracketCoef<C>& b, double s,
-                                            const double (&log_iab)[C + 1]) {
-    PabOut<C> pb;
-    return coop_eval<C, REML>(p, g, b, s, log_iab, pb);
-}
-
-// Golden-section refinement (_golden_section_refine, likelihood_jax.py:419-488) on the
-// mixed-form likelihood; returns the optimum's log-lambda (a + b) / 2 and the bracket's
-// expansions for the final evaluation.
-template <int C, bool REML>
-__device__ double golden_coop(const Params& p, const GlobalCoef<C>& g, int best, int f,
-                              const double (&log_iab)[C + 1], BracketCoef<C>& bc) {
-    const int lo = best - 1 > 0 ? best - 1 : 0;
-    const int hi = best + 1 < p.n_grid - 1 ? best + 1 : p.n_grid - 1;
-    bc = load_bracket_coef<C>(p, best, f);
-    auto probe = [&](double s) { return coop_logl<C, REML>(p, g, bc, s, log_iab); };
-    double a = p.loglam[lo], b = p.loglam[hi];
-    double c = __dsub_rn(b, __dmul_rn(kPhi, __dsub_rn(b, a)));
-    double d = __dadd_rn(a, __dmul_rn(kPhi, __dsub_rn(b, a)));
-    double fc = probe(c);
-    double fd = probe(d);
-    for (int it = 0; it < p.n_iter; ++it) {
-        const bool keep_left = fc > fd;
-        const double na = keep_left ? a : c;
-        const double nb = keep_left ? d : b;
-        const double nc = __dsub_rn(nb, __dmul_rn(kPhi, __dsub_rn(nb, na)));
-        const double nd = __dadd_rn(na, __dmul_rn(kPhi, __dsub_rn(nb, na)));
-        const double nl = probe(keep_left ? nc : nd);
-        const double nfc = keep_left ? nl : fd;
-        const double nfd = keep_left ? fc : nl;
-        a = na; b = nb; c = nc; d = nd; fc = nfc; fd = nfd;
-    }
-    return __dmul_rn(__dadd_rn(a, b), 0.5);
-}
-
 // Grid bracket + golden section (_golden_section_refine, likelihood_jax.py:419-488).
 template <int C, bool REML>
 __device__ void golden(const Params& p, const double* x, const double* y, int best,
@@ -636,190 +418,7 @@ __device__ void golden(const Params& p, const double* x, const double* y, int be
     logl_out = eval_logl<C, REML>(p, x, y, log_opt, log_iab, &pb_out);
 }
 
-// ---------------------------------------------------------------- two pairs per warp
-// The mixed-form search with one (SNP, phenotype) pair per half-warp and exactly the values
-// of the one-pair-per-warp form above: lane l (< 16) of a half stands in for that form's
-// lanes l ("v0") and l + 16 ("v1").  It holds both lanes' Chebyshev values, coefficients
-// and partial sums, built by the same formulas from the same inputs, and folds them with
-// the first (offset-16) step of the warp butterfly; the other four steps run across the
-// half.  Every value and the order of every sum match, so results are bit-identical, while
-// the per-probe scalar work (Pab recursion, logs, golden-section bookkeeping) that every
-// lane repeats now serves two pairs per instruction.
 constexpr unsigned kFull = 0xffffffffu;
-
-__device__ __forceinline__ double fold_sum(double p0, double p1) {
-    double v = __dadd_rn(p0, p1);  // offset 16: v_l + v_{l^16} (never contracted into an FMA)
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    return v;
-}
-
-// lane_cheb's T_l and T_{l+16} (32-lane doubling rounds) and T_32.
-__device__ __forceinline__ void lane_cheb_v(double x, double& t0, double& t1, double& t32) {
-    const int lane = threadIdx.x & 15;
-    double tl = lane == 0 ? 1.0 : x;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {  // a = 1, 2, 4, 8 (lanes above 16 are idle in these rounds)
-        const int a = 1 << r;
-        const bool act = lane > a && lane <= 2 * a;
-        const double ta = __shfl_sync(kFull, tl, a, 16);
-        const double tb = __shfl_sync(kFull, tl, act ? lane - a : 0, 16);
-        const double tc = __shfl_sync(kFull, tl, act ? 2 * a - lane : 0, 16);
-        if (act) tl = fma(2.0 * ta, tb, -tc);
-    }
-    const double t8 = __shfl_sync(kFull, tl, 8, 16);
-    const double t16 = fma(2.0 * t8, t8, -1.0);  // lane 16 at a = 8: 2 T_8 T_8 - T_0
-    const double tmir = __shfl_sync(kFull, tl, (16 - lane) & 15, 16);  // T_{16-l}
-    t0 = tl;
-    t1 = lane == 0 ? t16 : fma(2.0 * t16, tl, -tmir);  // lanes 17..31 at a = 16
-    t32 = fma(2.0 * t16, t16, -1.0);
-}
-
-struct LaneTV {
-    double t0[kCoefPerLane], t1[kCoefPerLane];
-};
-__device__ __forceinline__ LaneTV lane_cheb_global_v(double x) {
-    const int lane = threadIdx.x & 15;
-    double t0, t1, t32;
-    lane_cheb_v(x, t0, t1, t32);
-    const double a = __shfl_sync(kFull, t0, (16 - lane) & 15, 16);  // T_{16-l}
-    const double b = __shfl_sync(kFull, t1, (16 - lane) & 15, 16);  // T_{32-l}
-    LaneTV r;
-    r.t0[0] = t0;
-    r.t1[0] = t1;
-    r.t0[1] = fma(2.0 * t32, t0, -(lane == 0 ? t32 : b));  // T_{l+32}
-    r.t1[1] = fma(2.0 * t32, t1, -(lane == 0 ? t1 : a));   // T_{l+48}
-#pragma unroll
-    for (int i = 2; i < kCoefPerLane; ++i) {
-        r.t0[i] = fma(2.0 * t32, r.t0[i - 1], -r.t0[i - 2]);
-        r.t1[i] = fma(2.0 * t32, r.t1[i - 1], -r.t1[i - 2]);
-    }
-    return r;
-}
-
-template <int C>
-struct GlobalCoefV {
-    GlobalCoef<C> v0, v1;
-};
-template <int C>
-__device__ __forceinline__ GlobalCoefV<C> load_global_coef_v(const Params& p, int64_t j, int f) {
-    const int lane = threadIdx.x & 15;
-    const int64_t cp = C + p.phi;
-    GlobalCoefV<C> g;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        GlobalCoef<C>& gg = h ? g.v1 : g.v0;
-#pragma unroll
-        for (int i = 0; i < kCoefPerLane; ++i) {
-            const int64_t r = 1 + lane + 16 * h + 32 * i;
-            const double* rl = p.CL + j * p.ldcl + r * cp;
-#pragma unroll
-            for (int a = 0; a < C; ++a) gg.c[a][i] = __ldg(rl + a);
-            gg.c[C][i] = __ldg(p.CQ + j * p.ldcq + r);
-            gg.c[C + 1][i] = __ldg(rl + C + f);
-        }
-    }
-    return g;
-}
-
-template <int C>
-__device__ __forceinline__ void coop_xsums_v(const Params& p, const GlobalCoefV<C>& g, double s,
-                                             double (&xs)[Lay<C>::NX]) {
-    const LaneTV T = lane_cheb_global_v((s - p.gmid) * p.ginv);
-#pragma unroll
-    for (int q = 0; q < Lay<C>::NX; ++q) {
-        double v0 = g.v0.c[q][0] * T.t0[0], v1 = g.v1.c[q][0] * T.t1[0];
-#pragma unroll
-        for (int i = 1; i < kCoefPerLane; ++i) {
-            v0 = fma(g.v0.c[q][i], T.t0[i], v0);
-            v1 = fma(g.v1.c[q][i], T.t1[i], v1);
-        }
-        xs[q] = fold_sum(v0, v1);
-    }
-}
-
-template <int C>
-struct BracketCoefV {
-    BracketCoef<C> v0, v1;
-};
-template <int C>
-__device__ __forceinline__ BracketCoefV<C> load_bracket_coef_v(const Params& p, int best, int f) {
-    using L = Lay<C>;
-    const int lane = threadIdx.x & 15;
-    const int nf = 1 + p.phi * L::NS;
-    const double* cb = p.cheb + (int64_t)best * nf * kChebN;
-    BracketCoefV<C> b;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        BracketCoef<C>& bb = h ? b.v1 : b.v0;
-        const int jj = lane + 16 * h;
-        bb.c[0] = jj < kChebN ? __ldg(cb + jj) : 0.0;
-#pragma unroll
-        for (int k = 0; k < L::NS; ++k)
-            bb.c[1 + k] = jj < kChebN ? __ldg(cb + (1 + f * L::NS + k) * kChebN + jj) : 0.0;
-        bb.mid = p.cheb_mid[best];
-        bb.inv_half = 1.0 / p.cheb_half[best];
-    }
-    return b;
-}
-
-template <int C>
-__device__ __forceinline__ void coop_shared_v(const BracketCoefV<C>& b, double s, double& logdet,
-                                              double (&shared)[Lay<C>::NS]) {
-    double t0, t1, t32;
-    lane_cheb_v((s - b.v0.mid) * b.v0.inv_half, t0, t1, t32);
-    logdet = fold_sum(b.v0.c[0] * t0, b.v1.c[0] * t1);
-#pragma unroll
-    for (int k = 0; k < Lay<C>::NS; ++k) shared[k] = fold_sum(b.v0.c[1 + k] * t0, b.v1.c[1 + k] * t1);
-}
-
-template <int C, bool REML>
-__device__ __forceinline__ double coop_eval_v(const Params& p, const GlobalCoefV<C>& g,
-                                              const BracketCoefV<C>& b, double s,
-                                              const double (&log_iab)[C + 1], PabOut<C>& pb) {
-    using L = Lay<C>;
-    double xs[L::NX], shared[L::NS], logdet;
-    coop_xsums_v<C>(p, g, s, xs);
-    coop_shared_v<C>(b, s, logdet, shared);
-    double row0[L::NI];
-    assemble<C>(row0, shared, xs);
-    pb = pab_reduce<C>(row0);
-    return REML ? reml_logl<C>(pb, log_iab, logdet, p) : mle_logl<C>(pb, logdet, p);
-}
-
-template <int C, bool REML>
-__device__ __forceinline__ double coop_logl_v(const Params& p, const GlobalCoefV<C>& g,
-                                              const BracketCoefV<C>& b, double s,
-                                              const double (&log_iab)[C + 1]) {
-    PabOut<C> pb;
-    return coop_eval_v<C, REML>(p, g, b, s, log_iab, pb);
-}
-
-template <int C, bool REML>
-__device__ double golden_coop_v(const Params& p, const GlobalCoefV<C>& g, int best, int f,
-                                const double (&log_iab)[C + 1], BracketCoefV<C>& bc) {
-    const int lo = best - 1 > 0 ? best - 1 : 0;
-    const int hi = best + 1 < p.n_grid - 1 ? best + 1 : p.n_grid - 1;
-    bc = load_bracket_coef_v<C>(p, best, f);
-    auto probe = [&](double s) { return coop_logl_v<C, REML>(p, g, bc, s, log_iab); };
-    double a = p.loglam[lo], b = p.loglam[hi];
-    double c = __dsub_rn(b, __dmul_rn(kPhi, __dsub_rn(b, a)));
-    double d = __dadd_rn(a, __dmul_rn(kPhi, __dsub_rn(b, a)));
-    double fc = probe(c);
-    double fd = probe(d);
-    for (int it = 0; it < p.n_iter; ++it) {
-        const bool keep_left = fc > fd;
-        const double na = keep_left ? a : c;
-        const double nb = keep_left ? d : b;
-        const double nc = __dsub_rn(nb, __dmul_rn(kPhi, __dsub_rn(nb, na)));
-        const double nd = __dadd_rn(na, __dmul_rn(kPhi, __dsub_rn(nb, na)));
-        const double nl = probe(keep_left ? nc : nd);
-        const double nfc = keep_left ? nl : fd;
-        const double nfd = keep_left ? fc : nl;
-        a = na; b = nb; c = nc; d = nd; fc = nfc; fd = nfd;
-    }
-    return __dmul_rn(__dadd_rn(a, b), 0.5);
-}
 
 // jnp.argmax semantics: first maximum, NaN wins (first NaN).
 struct ArgMax {
@@ -986,34 +585,40 @@ __device__ __forceinline__ void direct_fix(const Params& p, int64_t j, int f, bo
     }
 }
 
-// 4 warps per block; with one covariate at least 5 blocks per SM (<= 102 registers, 20
-// resident warps to hide FP64 and shuffle latency), fewer for wider covariate sets whose
-// per-warp state would otherwise spill.
+// Statistics of the REML optimum (Wald): beta, se, the F statistic (NaN: no test;
+// lmm_fpvalue_kernel turns it into the p-value), lambda and the log-likelihood.
+template <int C>
+__device__ __forceinline__ void write_wald(const Params& p, const PabOut<C>& pb, double logl,
+                                           double lam, int64_t o, bool writer) {
+    bool valid;
+    double beta, tau, se;
+    const double px_yy = clamp_pyy(pb.yy1);
+    beta_se<C>(pb, px_yy, p.df, valid, beta, tau, se);
+    const double fstat = (pb.yy - px_yy) * tau;
+    if (writer) {
+        if (p.out.lambda_remle) p.out.lambda_remle[o] = lam;
+        if (p.out.logl_h1) p.out.logl_h1[o] = logl;
+        if (p.out.beta) p.out.beta[o] = beta;
+        if (p.out.se) p.out.se[o] = se;
+        if (p.out.p_wald) p.out.p_wald[o] = valid ? fstat : jnan();
+    }
+}
+
+// 4 warps per block; as many blocks per SM as the per-warp state allows without spills.
 constexpr int kPairsThreads = 128;
 template <int C>
 struct PairsOccupancy {
     static constexpr int kMinBlocks = C == 1 ? 4 : (C == 2 ? 3 : 2);  // C = 1: 125 registers, no spill
-    // two pairs per warp: each lane holds two virtual lanes' state (C = 1: 160 registers,
-    // no spill; 4 blocks at 128 registers measured within 0.5 %)
-    static constexpr int kMinBlocksHalf = 3;
 };
 
-// One (SNP, phenotype) pair per group of GW lanes: a warp (GW = 32), or a half-warp in the
-// mixed form with one covariate column (GW = 16, the bit-identical two-pairs-per-warp
-// helpers above).  Every lane of a warp runs the same control flow: a group past the last
-// pair repeats the last pair and writes nothing.
-template <int C, bool INTERP, int GW>
-__global__ void __launch_bounds__(kPairsThreads, GW == 16 ? PairsOccupancy<C>::kMinBlocksHalf
-                                                            : PairsOccupancy<C>::kMinBlocks)
+// Plain form: one (SNP, phenotype) pair per warp, every probe a direct FP64 pass over x.
+template <int C>
+__global__ void __launch_bounds__(kPairsThreads, PairsOccupancy<C>::kMinBlocks)
     lmm_pairs_kernel(const Params p) {
     using L = Lay<C>;
-    static_assert(GW == 32 || (INTERP && GW == 16), "half-warp pairs are a mixed-form path");
-    const int64_t npairs = p.m * p.phi;
-    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if ((tid & ~31ll) / GW >= npairs) return;  // the whole warp is idle
-    const bool valid_pair = tid / GW < npairs;
-    const int64_t wid = valid_pair ? tid / GW : npairs - 1;
-    const int lane = threadIdx.x & (GW - 1);
+    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    if (wid >= p.m * p.phi) return;
+    const int lane = threadIdx.x & 31;
     const int64_t j = wid / p.phi;
     const int f = (int)(wid % p.phi);
     const double* __restrict__ x = p.G + j * p.ldg;
@@ -1033,21 +638,13 @@ __global__ void __launch_bounds__(kPairsThreads, GW == 16 ? PairsOccupancy<C>::k
         xs[C + 1] = cl[C + f];
     };
 
-    // mixed form: this SNP's global series coefficients, spread over the warp
-    GlobalCoef<C> gc;
-    GlobalCoefV<C> gcv;
-    if constexpr (INTERP && GW == 16)
-        gcv = load_global_coef_v<C>(p, j, f);
-    else if (INTERP)
-        gc = load_global_coef<C>(p, j, f);
-
     // ---------------- phase 1: H = 1 (Iab) and H = H0 (score)
     double log_iab[C + 1];
 #pragma unroll
     for (int i = 0; i <= C; ++i) log_iab[i] = 0.0;
     if (need_reml) {
         double xs[L::NX], row0[L::NI];
-        row_xsums(INTERP ? 0 : p.n_grid, xs);
+        row_xsums(p.n_grid, xs);
         assemble<C>(row0, p.S + (int64_t)p.n_grid * srow + (int64_t)f * L::NS, xs);
         const PabOut<C> pb = pab_reduce<C>(row0);
 #pragma unroll
@@ -1055,19 +652,14 @@ __global__ void __launch_bounds__(kPairsThreads, GW == 16 ? PairsOccupancy<C>::k
     }
     if (need_score) {
         double xs[L::NX], row0[L::NI];
-        if constexpr (INTERP && GW == 16)
-            coop_xsums_v<C>(p, gcv, log(p.lam0[f]), xs);
-        else if (INTERP)
-            coop_xsums<C>(p, gc, log(p.lam0[f]), xs);
-        else
-            row_xsums(p.n_grid + 1 + f, xs);
+        row_xsums(p.n_grid + 1 + f, xs);
         assemble<C>(row0, p.S + (int64_t)(p.n_grid + 1 + f) * srow + (int64_t)f * L::NS, xs);
         const PabOut<C> pb = pab_reduce<C>(row0);
         bool valid;
         double beta, tau, se;
         beta_se<C>(pb, clamp_pyy(pb.yy1), p.df, valid, beta, tau, se);
         const double fstat = p.n_d * (pb.xy * pb.xy) / (pb.yy * (valid ? pb.xx : 1.0));
-        if (lane == 0 && valid_pair) {
+        if (lane == 0) {
             // the F statistic (NaN: no test); lmm_fpvalue_kernel turns it into the p-value
             if (p.out.p_score) p.out.p_score[o] = valid ? fstat : jnan();
             if (p.mode == 3) {
@@ -1076,110 +668,47 @@ __global__ void __launch_bounds__(kPairsThreads, GW == 16 ? PairsOccupancy<C>::k
             }
         }
     }
-    if (!need_reml && !need_mle) {
-        if constexpr (INTERP) {  // score only: the large-lambda rewrite happens here
-            double xs_m[L::NX], xs_r[L::NX];
-            direct_fix<C, GW>(p, j, f, valid_pair, need_score, false, false, 0.0, 0.0, xs_m, xs_r);
-        }
-        return;
-    }
+    if (!need_reml && !need_mle) return;
 
     // ---------------- phase 2: shared lambda grid
     ArgMax best_reml, best_mle;
-    // mixed form: lanes take grid points lane, lane+GW, ... from the series, then merge
-    for (int g = INTERP ? lane : 0; g < p.n_grid; g += INTERP ? GW : 1) {
+    for (int g = 0; g < p.n_grid; ++g) {
         double xs[L::NX], row0[L::NI];
-        if (INTERP)
-            series_xsums<C>(p, j, f, p.loglam[g], xs);
-        else
-            row_xsums(g, xs);
+        row_xsums(g, xs);
         assemble<C>(row0, p.S + (int64_t)g * srow + (int64_t)f * L::NS, xs);
         const PabOut<C> pb = pab_reduce<C>(row0);
         const double ldh = p.logdet[g];
         if (need_reml) best_reml.push(g, reml_logl<C>(pb, log_iab, ldh, p));
         if (need_mle) best_mle.push(g, mle_logl<C>(pb, ldh, p));
     }
-    if (INTERP) {
-        best_reml.warp_reduce<GW>();
-        best_mle.warp_reduce<GW>();
-    }
 
     // ---------------- phase 3: golden sections + statistics
-    double lam_m = 0.0, logl_m = 0.0, lam_r = 0.0, logl_r = 0.0;
-    double s_m = 0.0, s_r = 0.0;  // mixed form: log-lambda of the optima
-    PabOut<C> pb_r;
-    if constexpr (INTERP) {
-        // final evaluations at the optima: x-dependent sums from the series (or, at large
-        // lambda, directly), x-free sums and log|H^-1| from the bracket's expansions
-        double xs_m[L::NX], xs_r[L::NX], sh_m[L::NS], sh_r[L::NS], ld_m = 0.0, ld_r = 0.0;
-        if constexpr (GW == 16) {
-            BracketCoefV<C> bm, br;
-            if (need_mle) s_m = golden_coop_v<C, false>(p, gcv, best_mle.idx, f, log_iab, bm);
-            if (need_reml) s_r = golden_coop_v<C, true>(p, gcv, best_reml.idx, f, log_iab, br);
-            if (need_mle) {
-                coop_xsums_v<C>(p, gcv, s_m, xs_m);
-                coop_shared_v<C>(bm, s_m, ld_m, sh_m);
-            }
-            if (need_reml) {
-                coop_xsums_v<C>(p, gcv, s_r, xs_r);
-                coop_shared_v<C>(br, s_r, ld_r, sh_r);
-            }
-        } else {
-            BracketCoef<C> bm, br;
-            if (need_mle) s_m = golden_coop<C, false>(p, gc, best_mle.idx, f, log_iab, bm);
-            if (need_reml) s_r = golden_coop<C, true>(p, gc, best_reml.idx, f, log_iab, br);
-            if (need_mle) {
-                coop_xsums<C>(p, gc, s_m, xs_m);
-                coop_shared<C>(bm, s_m, ld_m, sh_m);
-            }
-            if (need_reml) {
-                coop_xsums<C>(p, gc, s_r, xs_r);
-                coop_shared<C>(br, s_r, ld_r, sh_r);
-            }
+    if (need_mle) {
+        double lam, logl;
+        PabOut<C> pb;
+        golden<C, false>(p, x, y, best_mle.idx, log_iab, lam, logl, pb);
+        if (lane == 0) {
+            if (p.out.lambda_mle) p.out.lambda_mle[o] = lam;
+            if (p.out.logl_mle) p.out.logl_mle[o] = logl;
+            const double stat = jmax(2.0 * (logl - p.logl0[f]), 0.0);
+            if (p.out.p_lrt) p.out.p_lrt[o] = chi2_1_sf(stat);
         }
-        lam_m = exp(s_m);
-        lam_r = exp(s_r);
-        direct_fix<C, GW>(p, j, f, valid_pair, need_score, need_mle, need_reml, s_m, s_r, xs_m,
-                          xs_r);
-        double row0[L::NI];
-        if (need_mle) {
-            assemble<C>(row0, sh_m, xs_m);
-            const PabOut<C> pb = pab_reduce<C>(row0);
-            logl_m = mle_logl<C>(pb, ld_m, p);
-        }
-        if (need_reml) {
-            assemble<C>(row0, sh_r, xs_r);
-            pb_r = pab_reduce<C>(row0);
-            logl_r = reml_logl<C>(pb_r, log_iab, ld_r, p);
-        }
-    } else {
-        if (need_mle) {
-            PabOut<C> pb;
-            golden<C, false>(p, x, y, best_mle.idx, log_iab, lam_m, logl_m, pb);
-        }
-        if (need_reml) golden<C, true>(p, x, y, best_reml.idx, log_iab, lam_r, logl_r, pb_r);
-    }
-    if (need_mle && lane == 0 && valid_pair) {
-        if (p.out.lambda_mle) p.out.lambda_mle[o] = lam_m;
-        if (p.out.logl_mle) p.out.logl_mle[o] = logl_m;
-        const double stat = jmax(2.0 * (logl_m - p.logl0[f]), 0.0);
-        if (p.out.p_lrt) p.out.p_lrt[o] = chi2_1_sf(stat);
     }
     if (need_reml) {
-        bool valid;
-        double beta, tau, se;
-        const double px_yy = clamp_pyy(pb_r.yy1);
-        beta_se<C>(pb_r, px_yy, p.df, valid, beta, tau, se);
-        const double fstat = (pb_r.yy - px_yy) * tau;
-        if (lane == 0 && valid_pair) {
-            if (p.out.lambda_remle) p.out.lambda_remle[o] = lam_r;
-            if (p.out.logl_h1) p.out.logl_h1[o] = logl_r;
-            if (p.out.beta) p.out.beta[o] = beta;
-            if (p.out.se) p.out.se[o] = se;
-            if (p.out.p_wald) p.out.p_wald[o] = valid ? fstat : jnan();  // F, as for p_score
-        }
+        double lam, logl;
+        PabOut<C> pb;
+        golden<C, true>(p, x, y, best_reml.idx, log_iab, lam, logl, pb);
+        write_wald<C>(p, pb, logl, lam, o, lane == 0);
     }
 }
+
+}  // namespace lmm
+}  // namespace jb
+
+#include "jb_lmm_search.cuh"
+
+namespace jb {
+namespace lmm {
 
 // ---------------------------------------------------------------- tables
 // H rows: grid lambda_g = exp(loglam[g]) for g < n_grid, then the null lambda0[f];
@@ -1488,6 +1017,21 @@ __global__ void lmm_series_dct_kernel(double* __restrict__ ccos) {
     ccos[k + (int64_t)j * kChebG] = k == 0 ? 0.5 * c : c;
 }
 
+// Chebyshev values of the global series at the grid points: tg[g * kChebG + k] = T_k(t_g).
+__global__ void lmm_grid_cheb_kernel(int n_grid, double mid, double inv_half,
+                                     const double* __restrict__ loglam, double* __restrict__ tg) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= n_grid) return;
+    const double x = (loglam[g] - mid) * inv_half;
+    double t0 = 1.0, t1 = x;
+    for (int k = 0; k < kChebG; ++k) {
+        tg[(int64_t)g * kChebG + k] = t0;
+        const double t2 = fma(2.0 * x, t1, -t0);
+        t0 = t1;
+        t1 = t2;
+    }
+}
+
 // GEMM operands of the mixed form: row 0 is the ones row (h = 1), row 1 + k holds the
 // Chebyshev coefficient k of h_i(t) (already in Asq rows 1..kChebG from the transform
 // GEMM); A_lin[r*(C+phi) + a] = Asq[r] * w_a, A_lin[r*(C+phi) + C + f] = Asq[r] * y_f.
@@ -1704,7 +1248,8 @@ __global__ void null_mle_kernel(int64_t n, const double* W, int64_t ldw, const d
 
 // ---------------------------------------------------------------- host helpers
 struct WsLayout {
-    int64_t loglam, logdet, H, S, cheb, cmid, chalf, cvals, alin, asq, asqt, hn, ccos, blas, total;
+    int64_t loglam, logdet, H, S, cheb, cmid, chalf, tgrid, cvals, alin, asq, asqt, hn, ccos, blas,
+        total;
 };
 
 inline int64_t align256(int64_t b) { return (b + 255) / 256 * 256; }
@@ -1736,6 +1281,8 @@ inline WsLayout ws_layout(int64_t n, int c, int phi, int n_grid) {
     off += align256(8 * (int64_t)n_grid);
     w.chalf = off;
     off += align256(8 * (int64_t)n_grid);
+    w.tgrid = off;
+    off += align256(8 * (int64_t)n_grid * kChebG);
     w.cvals = off;
     off += align256(8 * (int64_t)n_grid * nf * kChebN);
     const int64_t rows = table_rows(phi, n_grid);
@@ -1890,18 +1437,12 @@ int32_t launch_sq_sums(const double* AT, int64_t rows, const double* X, int64_t 
 template <int C>
 int32_t launch_pairs(const Params& p, cudaStream_t st) {
     const int64_t pairs = p.m * p.phi;
-    if constexpr (C == 1) {
-        if (p.cheb)  // two pairs per warp (bit-identical to one per warp)
-            lmm_pairs_kernel<C, true, 16>
-                <<<(unsigned)ceil_div(pairs * 16, kPairsThreads), kPairsThreads, 0, st>>>(p);
-        else
-            lmm_pairs_kernel<C, false, 32>
-                <<<(unsigned)ceil_div(pairs * 32, kPairsThreads), kPairsThreads, 0, st>>>(p);
-    } else if (p.cheb)
-        lmm_pairs_kernel<C, true, 32><<<(unsigned)ceil_div(pairs * 32, kPairsThreads), kPairsThreads, 0, st>>>(p);
+    if (p.cheb)
+        lmm_search_kernel<C><<<(unsigned)ceil_div(pairs * Search<C>::LP, Search<C>::kThreads),
+                               Search<C>::kThreads, 0, st>>>(p);
     else
-        lmm_pairs_kernel<C, false, 32><<<(unsigned)ceil_div(pairs * 32, kPairsThreads), kPairsThreads, 0, st>>>(p);
-    JB_LAUNCH_CHECK("lmm_pairs_kernel");
+        lmm_pairs_kernel<C><<<(unsigned)ceil_div(pairs * 32, kPairsThreads), kPairsThreads, 0, st>>>(p);
+    JB_LAUNCH_CHECK("lmm search");
     // p-values of the tests this mode ran (other outputs stay untouched)
     double* v0 = (p.mode == 1 || p.mode == 4) ? p.out.p_wald : nullptr;
     double* v1 = (p.mode == 3 || p.mode == 4) ? p.out.p_score : nullptr;
@@ -1952,6 +1493,10 @@ int32_t launch_prepare(int64_t n, int phi, int n_grid, const double* evals, cons
         lmm_series_nodes_kernel<<<dim3(ny, kChebG), 256, 0, st>>>(n, 0.5 * (lo + hi), 0.5 * (hi - lo),
                                                                    evals, hn);
         JB_LAUNCH_CHECK("lmm_series_nodes_kernel");
+        lmm_grid_cheb_kernel<<<(n_grid + 31) / 32, 32, 0, st>>>(
+            n_grid, 0.5 * (lo + hi), 1.0 / (0.5 * (hi - lo)), loglam,
+            reinterpret_cast<double*>(ws + L.tgrid));
+        JB_LAUNCH_CHECK("lmm_grid_cheb_kernel");
         lmm_series_dct_kernel<<<kChebG, kChebG, 0, st>>>(ccos);
         JB_LAUNCH_CHECK("lmm_series_dct_kernel");
         cublasHandle_t h = cublas_handle();
@@ -2161,6 +1706,7 @@ int32_t jb_lmm_chunk(int32_t lmm_mode, int32_t precision, int64_t n, int32_t n_c
     p.cheb = precision >= 1 ? reinterpret_cast<const double*>(ws + L.cheb) : nullptr;
     p.cheb_mid = reinterpret_cast<const double*>(ws + L.cmid);
     p.cheb_half = reinterpret_cast<const double*>(ws + L.chalf);
+    p.tgrid = reinterpret_cast<const double*>(ws + L.tgrid);
     p.lam0 = lam0;
     JB_CHECK_ARG(precision == 0 || lmm_mode == 1 || lam0 != nullptr,
                  "jb_lmm_chunk: the mixed form needs lam0 in modes 2-4");
