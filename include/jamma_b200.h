@@ -323,7 +323,8 @@ typedef struct jb_lmm_out {
  * -- the squared sums sum_i h_i x_i^2 by one fused kernel that reads each rotated genotype
  * once and squares it on chip (FP64, fixed summation order), the linear sums by a cuBLAS
  * DGEMM (precision 0 and 1) or by jb_lmm_chunk_series_i8 (precision 2).  The chunk's
- * precision must match the one its workspace was prepared with (0 with 0; 1 or 2 with 1).
+ * precision must match the one its workspace was prepared with (0 with 0; 1 or 2 with 1;
+ * 3 with 3).
  * precision: 0 = every likelihood evaluation is a direct FP64 reduction over n (plain
  * form; grid, ones and null rows by DGEMM);
  * 1 = mixed form: the c+2 genotype-dependent sums are a degree-95 Chebyshev series in
@@ -334,7 +335,11 @@ typedef struct jb_lmm_out {
  * genotypes).  Needs 1e-5 <= l_min < l_max <= 1e5 and
  * 1 + 1e5 * min(eval) > 0.5 (no pole of 1/(lambda eval + 1) near the domain);
  * 2 = as 1, with the linear series sums already placed in chunk_workspace by
- * jb_lmm_chunk_series_i8 for the same chunk (only the squared sums use a DGEMM).
+ * jb_lmm_chunk_series_i8 for the same chunk (only the squared sums use a DGEMM);
+ * 3 = plain form, guided: the grid's and the golden sections' decisions are taken on the
+ * series of precision 1 while they differ by more than the series' error bound, the others
+ * and the final evaluations by direct FP64 reductions, so the optima are those of precision
+ * 0; conditions as for 1, and n_grid >= 16.
  */
 int64_t jb_lmm_workspace_size(int64_t n, int32_t n_cvt, int32_t phi, int32_t n_grid);
 

@@ -24,7 +24,14 @@
 #include "jb_common.cuh"
 #include "jb_rotate_i8.cuh"
 
+namespace jb {
+namespace tc {
+int num_sms();
+}
+}  // namespace jb
+
 #include <cmath>
+#include <type_traits>
 
 namespace jb {
 namespace lmm {
@@ -86,6 +93,10 @@ struct Params {
     int64_t ldcq;
     const double* lam0;  // null-model lambda per phenotype (modes 2-4)
     double gmid, ginv;   // domain centre and 1 / half-width of the global series
+    // guided plain form: 2 states per pair (MLE, REML), and the searches left open
+    struct SearchState* state;
+    int64_t* open_list;
+    unsigned long long* open_count;
 };
 
 constexpr int kChebN = 25;  // interpolation nodes (degree 24) per bracket
@@ -1307,7 +1318,7 @@ inline WsLayout ws_layout(int64_t n, int c, int phi, int n_grid) {
 }
 
 struct ChunkLayout {
-    int64_t sqp, cl, cq, blas, total;
+    int64_t sqp, cl, cq, state, open, blas, total;
 };
 
 // Partial squared sums of sq_sums_kernel's sample ranges: the largest over the row counts a
@@ -1333,6 +1344,10 @@ inline ChunkLayout chunk_layout(int64_t n, int c, int phi, int n_grid, int64_t m
     off += align256(8 * rows * (c + phi) * m);
     L.cq = off;
     off += align256(8 * rows * m);
+    L.state = off;
+    off += align256(2 * (int64_t)sizeof(SearchState) * phi * m);
+    L.open = off;  // counter, then the list
+    off += align256(256 + 2 * (int64_t)sizeof(int64_t) * phi * m);
     L.blas = off;  // cuBLAS workspace of this chunk's DGEMMs (fixed size: same kernels alone or
     off += kCublasWorkspaceBytes;  // beside other streams' work, so results do not depend on it)
     L.total = off;
@@ -1437,11 +1452,30 @@ int32_t launch_sq_sums(const double* AT, int64_t rows, const double* X, int64_t 
 template <int C>
 int32_t launch_pairs(const Params& p, cudaStream_t st) {
     const int64_t pairs = p.m * p.phi;
-    if (p.cheb)
-        lmm_search_kernel<C><<<(unsigned)ceil_div(pairs * Search<C>::LP, Search<C>::kThreads),
-                               Search<C>::kThreads, 0, st>>>(p);
-    else
-        lmm_pairs_kernel<C><<<(unsigned)ceil_div(pairs * 32, kPairsThreads), kPairsThreads, 0, st>>>(p);
+    const unsigned groups = (unsigned)ceil_div(pairs * Search<C>::LP, Search<C>::kThreads);
+    const unsigned warps = (unsigned)ceil_div(pairs * 32, kPairsThreads);
+    if (p.state) {
+        if (p.mode != 3) {
+            JB_CUDA(cudaMemsetAsync(p.open_count, 0, sizeof(*p.open_count), st));
+            lmm_search_kernel<C, true><<<groups, Search<C>::kThreads, 0, st>>>(p);
+            JB_LAUNCH_CHECK("lmm_search_kernel");
+            const int64_t sms = tc::num_sms();
+            lmm_open_kernel<C><<<(unsigned)(2 * pairs < sms ? 2 * pairs : sms), kOpenThreads, 0, st>>>(
+                p, kOpenPerSm * sms);
+            JB_LAUNCH_CHECK("lmm_open_kernel");
+            if (2 * pairs > kOpenPerSm * sms) {
+                const int64_t blocks = sms * PairsOccupancy<C>::kMinBlocks;
+                lmm_close_kernel<C><<<(unsigned)(warps < blocks ? warps : blocks), kPairsThreads, 0, st>>>(
+                    p, kOpenPerSm * sms);
+                JB_LAUNCH_CHECK("lmm_close_kernel");
+            }
+        }
+        lmm_finish_kernel<C><<<warps, kPairsThreads, 0, st>>>(p);
+    } else if (p.cheb) {
+        lmm_search_kernel<C, false><<<groups, Search<C>::kThreads, 0, st>>>(p);
+    } else {
+        lmm_pairs_kernel<C><<<warps, kPairsThreads, 0, st>>>(p);
+    }
     JB_LAUNCH_CHECK("lmm search");
     // p-values of the tests this mode ran (other outputs stay untouched)
     double* v0 = (p.mode == 1 || p.mode == 4) ? p.out.p_wald : nullptr;
@@ -1463,7 +1497,8 @@ int32_t launch_pairs(const Params& p, cudaStream_t st) {
 template <int C>
 int32_t launch_prepare(int64_t n, int phi, int n_grid, const double* evals, const double* W,
                        int64_t ldw, const double* Y, int64_t ldy, const double* lam0,
-                       double l_min, double l_max, uint8_t* ws, cudaStream_t st, bool interp) {
+                       double l_min, double l_max, uint8_t* ws, cudaStream_t st, bool interp,
+                       bool sums_only) {
     const WsLayout L = ws_layout(n, C, phi, n_grid);
     double* loglam = reinterpret_cast<double*>(ws + L.loglam);
     double* logdet = reinterpret_cast<double*>(ws + L.logdet);
@@ -1478,6 +1513,7 @@ int32_t launch_prepare(int64_t n, int phi, int n_grid, const double* evals, cons
     const int rows_s = n_grid + 1 + (lam0 ? phi : 0);
     lmm_shared_kernel<C><<<dim3(rows_s, phi), 256, 0, st>>>(n, n_grid, phi, W, ldw, Y, ldy, H, S);
     JB_LAUNCH_CHECK("lmm_shared_kernel");
+    if (sums_only) return JB_OK;  // guided plain form, score test only
     const unsigned ny = (unsigned)(ceil_div(n, 256) < 64 ? ceil_div(n, 256) : 64);
     double* Alin = reinterpret_cast<double*>(ws + L.alin);
     double* Asq = reinterpret_cast<double*>(ws + L.asq);
@@ -1555,7 +1591,8 @@ int32_t jb_lmm_prepare(int32_t lmm_mode, int32_t precision, int64_t n, int32_t n
                        const double* Uty, int64_t ldy, const double* lam0, double l_min,
                        double l_max, int32_t n_grid, void* workspace, int64_t workspace_bytes,
                        uintptr_t stream) {
-    JB_CHECK_ARG(precision == 0 || precision == 1, "jb_lmm_prepare: precision must be 0 or 1");
+    JB_CHECK_ARG(precision == 0 || precision == 1 || precision == 3,
+                 "jb_lmm_prepare: precision must be 0, 1 or 3");
     JB_CHECK_ARG(lmm_mode >= 1 && lmm_mode <= 4, "jb_lmm_prepare: lmm_mode must be 1..4");
     JB_CHECK_ARG(n > 0 && phi >= 1 && n_grid >= 2, "jb_lmm_prepare: bad sizes");
     JB_CHECK_ARG(n_cvt >= 1 && n_cvt <= kMaxCvt, "jb_lmm_prepare: n_cvt must be in 1..%d", kMaxCvt);
@@ -1567,15 +1604,16 @@ int32_t jb_lmm_prepare(int32_t lmm_mode, int32_t precision, int64_t n, int32_t n
                  "jb_lmm_prepare: workspace too small");
     JB_CHECK_ARG(phi <= 65535, "jb_lmm_prepare: too many phenotypes");
     JB_CHECK_ARG(precision == 0 || (l_min >= kDomainLo * (1 - 1e-12) && l_max <= kDomainHi * (1 + 1e-12)),
-                 "jb_lmm_prepare: the mixed form needs 1e-5 <= l_min < l_max <= 1e5");
+                 "jb_lmm_prepare: the series need 1e-5 <= l_min < l_max <= 1e5");
     cudaStream_t st = as_stream(stream);
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     const double* l0 = lmm_mode == 1 ? nullptr : lam0;
+    const bool series = precision != 0, sums_only = precision == 3 && lmm_mode == 3;
     switch (n_cvt) {
-        case 1: return launch_prepare<1>(n, phi, n_grid, evals, UtW, ldw, Uty, ldy, l0, l_min, l_max, ws, st, precision == 1);
-        case 2: return launch_prepare<2>(n, phi, n_grid, evals, UtW, ldw, Uty, ldy, l0, l_min, l_max, ws, st, precision == 1);
-        case 3: return launch_prepare<3>(n, phi, n_grid, evals, UtW, ldw, Uty, ldy, l0, l_min, l_max, ws, st, precision == 1);
-        case 4: return launch_prepare<4>(n, phi, n_grid, evals, UtW, ldw, Uty, ldy, l0, l_min, l_max, ws, st, precision == 1);
+        case 1: return launch_prepare<1>(n, phi, n_grid, evals, UtW, ldw, Uty, ldy, l0, l_min, l_max, ws, st, series, sums_only);
+        case 2: return launch_prepare<2>(n, phi, n_grid, evals, UtW, ldw, Uty, ldy, l0, l_min, l_max, ws, st, series, sums_only);
+        case 3: return launch_prepare<3>(n, phi, n_grid, evals, UtW, ldw, Uty, ldy, l0, l_min, l_max, ws, st, series, sums_only);
+        case 4: return launch_prepare<4>(n, phi, n_grid, evals, UtW, ldw, Uty, ldy, l0, l_min, l_max, ws, st, series, sums_only);
     }
     return JB_E_UNSUPPORTED;
 }
@@ -1702,16 +1740,17 @@ int32_t jb_lmm_chunk(int32_t lmm_mode, int32_t precision, int64_t n, int32_t n_c
     p.c_reml = 0.5 * df * (std::log(df) - std::log(2 * M_PI) - 1.0);
     p.c_mle = 0.5 * (double)n * (std::log((double)n) - std::log(2 * M_PI) - 1.0);
     p.out = out;
-    JB_CHECK_ARG(precision >= 0 && precision <= 2, "jb_lmm_chunk: precision must be 0, 1 or 2");
+    JB_CHECK_ARG(precision >= 0 && precision <= 3, "jb_lmm_chunk: precision must be 0 to 3");
     p.cheb = precision >= 1 ? reinterpret_cast<const double*>(ws + L.cheb) : nullptr;
     p.cheb_mid = reinterpret_cast<const double*>(ws + L.cmid);
     p.cheb_half = reinterpret_cast<const double*>(ws + L.chalf);
     p.tgrid = reinterpret_cast<const double*>(ws + L.tgrid);
     p.lam0 = lam0;
+    JB_CHECK_ARG(precision != 3 || n_grid >= 16, "jb_lmm_chunk: precision 3 needs n_grid >= 16");
     JB_CHECK_ARG(precision == 0 || lmm_mode == 1 || lam0 != nullptr,
-                 "jb_lmm_chunk: the mixed form needs lam0 in modes 2-4");
+                 "jb_lmm_chunk: precision 1 to 3 needs lam0 in modes 2-4");
     JB_CHECK_ARG(precision == 0 || (l_min >= kDomainLo * (1 - 1e-12) && l_max <= kDomainHi * (1 + 1e-12)),
-                 "jb_lmm_chunk: the mixed form needs 1e-5 <= l_min < l_max <= 1e5");
+                 "jb_lmm_chunk: the series need 1e-5 <= l_min < l_max <= 1e5");
     {
         const double lo = std::log(kDomainLo), hi = std::log(kDomainHi);
         p.gmid = 0.5 * (lo + hi);
@@ -1724,10 +1763,13 @@ int32_t jb_lmm_chunk(int32_t lmm_mode, int32_t precision, int64_t n, int32_t n_c
     uint8_t* cws = static_cast<uint8_t*>(chunk_workspace);
     double* CL = reinterpret_cast<double*>(cws + CLy.cl);
     double* CQ = reinterpret_cast<double*>(cws + CLy.cq);
+    p.state = precision == 3 ? reinterpret_cast<SearchState*>(cws + CLy.state) : nullptr;
+    p.open_count = reinterpret_cast<unsigned long long*>(cws + CLy.open);
+    p.open_list = reinterpret_cast<int64_t*>(cws + CLy.open + 256);
     // FP64 form: grid rows, ones row, null rows (only when prepared); mixed: ones + series
     const int rows = precision >= 1 ? 1 + kChebG : n_grid + 1 + (lmm_mode == 1 ? 0 : phi);
     const int rows_lin = rows * (n_cvt + phi);
-    {
+    if (precision != 3 || lmm_mode != 3) {  // the guided form's score test sums directly
         if (precision != 2) {  // precision 2: CL already formed by jb_lmm_chunk_series_i8
             cublasHandle_t h = cublas_handle();
             if (!h) {

@@ -203,11 +203,47 @@ __device__ __forceinline__ double group_reml(const PabOut<C>& pb, const double (
     return __dsub_rn(f, __dmul_rn(__dmul_rn(0.5, p.df), lpyy));
 }
 
+// A golden section as the plain form's search leaves it (see lmm_open_kernel): bracket [a, b]
+// before decision `step`, and the log-lambdas sc < sd of its two inner values.  step =
+// n_iter: every decision is taken; step = -1: none, not even the grid's.
+struct SearchState {
+    double a, b, sc, sd, step;
+};
+
+// Where a search of the plain form reports: its state, and the list of searches left open.
+struct SearchReport {
+    SearchState* state = nullptr;  // null: this lane does not report
+    int64_t id = 0;
+    int64_t* list = nullptr;
+    unsigned long long* count = nullptr;
+    __device__ __forceinline__ void put(const SearchState& st, bool open) const {
+        if (!state) return;
+        *state = st;
+        if (open) list[atomicAdd(count, 1ull)] = id;
+    }
+};
+
 // One golden section (_golden_section_refine, likelihood_jax.py:419-488) as a sequence of
 // probes: c, d, then one per step; probe number n_iter + 2 is the optimum (a + b) / 2.
+// GUIDE: the probes are approximations of direct evaluations, their differences certain to
+// GuideTau.  The first decision between values closer than that (or NaN) is left open: the
+// state before it is reported, and the steps after it are without effect.
+struct GuideTau {
+    double whole;  // error of a probe's value
+    double slope;  // of a difference, per unit of log-lambda between the probes
+    double floor;  // the part that does not shrink with that distance (rounding)
+    __device__ __forceinline__ double of(double dist) const {
+        return floor + fmin(whole, slope * dist);
+    }
+};
+
+template <bool GUIDE>
 struct Golden {
     double a, b, c, d, fc, fd, s;  // s: the next probe
     bool left;                     // it replaces c (fc), else d (fd)
+    double sc, sd;                 // GUIDE: where fc and fd were evaluated
+    GuideTau tau;
+    bool certain;
     __device__ __forceinline__ void start(const Params& p, int best) {
         const int lo = best - 1 > 0 ? best - 1 : 0;
         const int hi = best + 1 < p.n_grid - 1 ? best + 1 : p.n_grid - 1;
@@ -217,15 +253,21 @@ struct Golden {
         fc = fd = 0.0;
         s = c;
         left = true;
+        sc = sd = 0.0;
+        certain = true;
     }
     __device__ __forceinline__ void inner() {
         c = __dsub_rn(b, __dmul_rn(kPhi, __dsub_rn(b, a)));
         d = __dadd_rn(a, __dmul_rn(kPhi, __dsub_rn(b, a)));
     }
     // takes the value at probe `it` and sets the next one
-    __device__ __forceinline__ void take(double f, int it, int n_iter) {
+    __device__ __forceinline__ void take(double f, int it, int n_iter, const SearchReport& out) {
         fc = left ? f : fc;
         fd = left ? fd : f;
+        if (GUIDE) {
+            sc = left ? s : sc;
+            sd = left ? sd : s;
+        }
         if (it == 0) {
             s = d;
             left = false;
@@ -233,7 +275,12 @@ struct Golden {
         }
         if (it > n_iter) {
             s = __dmul_rn(__dadd_rn(a, b), 0.5);
+            if (GUIDE && certain) out.put(SearchState{a, b, sc, sd, (double)n_iter}, false);
             return;
+        }
+        if (GUIDE && certain && !(fabs(fc - fd) > tau.of(fabs(sd - sc)))) {
+            certain = false;
+            out.put(SearchState{a, b, sc, sd, (double)(it - 1)}, true);
         }
         left = fc > fd;
         a = left ? a : c;
@@ -241,12 +288,94 @@ struct Golden {
         const double keep = left ? fc : fd;
         fc = keep;  // the one that the next probe replaces is overwritten
         fd = keep;
+        if (GUIDE) {
+            const double at = left ? sc : sd;
+            sc = at;
+            sd = at;
+        }
         inner();
         s = left ? c : d;
     }
 };
 
+// GUIDE: how far a probe's log-likelihood can be from its direct evaluation, over the golden
+// bracket of grid index `best`.  The series leave an absolute error in the x-dependent sums
+// (~1e-13 of the size that they have at lambda -> 0), which counts
+//   * by A = sum w0^2 / sum h w0^2, the factor by which the weighted sums have shrunk there,
+//   * by G = sum h x^2 / P_xx, the cancellation against the covariates (an uncentred, nearly
+//     constant genotype): sqrt(G) in P_xy, G in P_xx; 1 for a genotype of zeros, whose
+//     series vanish,
+//   * by the SNP's z score, through xy^2 / xx.
+// Measured over n = 500 to 20 000, h2 = 0 to 0.9 and allele frequencies 0.01 to 0.99 the
+// difference of series and direct log-likelihoods stays below 1/15 of `whole`.  It is the
+// truncated terms of degree 96 and up, so between close probes it cancels: its slope in log
+// lambda is at most 96 / 11.5 per sqrt(1 - t^2) (t the point in the domain scaled to
+// [-1, 1]), 27 for |t| < 0.95 and 96^2 / 11.5 = 801 anywhere.  What stays is rounding: 1/100
+// of `whole` (one rounding against ~1e-13) and the direct sums' own, a few ulp of a value of
+// size 1.4 n.  Anything not finite, or a bound that no longer tells golden steps apart, makes
+// the pair's search direct from the grid on.
 template <int C>
+__device__ __forceinline__ GuideTau guide_tau(const Params& p, const PairCoef<C>& g, int best,
+                                              int f, int r) {
+    using L = Lay<C>;
+    const int64_t srow = (int64_t)p.phi * L::NS;
+    const double* s0 = p.S + (int64_t)best * srow + (int64_t)f * L::NS;
+    double xs[L::NX], row0[L::NI];
+    grid_xsums<C>(p, g, best, r, xs);
+    assemble<C>(row0, s0, xs);
+    const PabOut<C> pb = pab_reduce<C>(row0);
+    const double A = p.S[(int64_t)p.n_grid * srow + (int64_t)f * L::NS] / s0[0];
+    const double xx = row0[L::idx(C, C)];
+    const double G = xx == 0.0 ? 1.0 : xx / pb.xx;
+    const double z2 = p.n_d * fmax(pb.yy - pb.yy1, 0.0) / pb.yy1;
+    double whole = 2.0 * A * (1e-9 * sqrt(G) * (1.0 + 0.05 * sqrt(z2)) + 2e-13 * G * (1.0 + z2));
+    if (!(A > 0.0 && G >= 0.5 && whole < 1e-2)) whole = __longlong_as_double(0x7ff0000000000000ll);
+    const double t = (p.loglam[best] - p.gmid) * p.ginv;
+    return GuideTau{whole, whole * (fabs(t) < 0.95 ? 30.0 : 900.0), 0.01 * whole + 1e-14 * p.n_d};
+}
+
+// Maximum of the grid's values with its lead over the next largest.
+struct ArgMaxLead {
+    int idx = -1;
+    double v = 0.0, v2 = 0.0;
+    bool nan = false;
+    __device__ __forceinline__ void push(int i, double x) {
+        nan = nan || isnan(x);
+        if (idx < 0) {
+            idx = i;
+            v = x;
+            v2 = -__longlong_as_double(0x7ff0000000000000ll);
+        } else if (x > v) {
+            idx = i;
+            v2 = v;
+            v = x;
+        } else {
+            v2 = x > v2 ? x : v2;
+        }
+    }
+    template <int GW>
+    __device__ __forceinline__ void warp_reduce() {  // over groups of GW lanes
+#pragma unroll
+        for (int o = GW / 2; o > 0; o >>= 1) {
+            const int oi = __shfl_xor_sync(kFull, idx, o);
+            const double ov = __shfl_xor_sync(kFull, v, o), ov2 = __shfl_xor_sync(kFull, v2, o);
+            nan = __shfl_xor_sync(kFull, (int)nan, o) != 0 || nan;
+            if (oi < 0) continue;
+            if (idx < 0 || ov > v || (ov == v && oi < idx)) {
+                v2 = idx >= 0 && v > ov2 ? v : ov2;
+                v = ov;
+                idx = oi;
+            } else {
+                v2 = ov > v2 ? ov : v2;
+            }
+        }
+    }
+};
+
+// GUIDE = false: the mixed form, search and statistics.  GUIDE = true: the plain form's
+// decisions, as far as they are certain (modes 1, 2 and 4); lmm_open_kernel and
+// lmm_finish_kernel take over.
+template <int C, bool GUIDE>
 __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
     lmm_search_kernel(const Params p) {
     using L = Lay<C>;
@@ -262,7 +391,7 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
     const int f = (int)(wid % p.phi);
     const bool need_reml = p.mode == 1 || p.mode == 4;
     const bool need_mle = p.mode == 2 || p.mode == 4;
-    const bool need_score = p.mode == 3 || p.mode == 4;
+    const bool need_score = !GUIDE && (p.mode == 3 || p.mode == 4);
     const int64_t o = (int64_t)f * p.m + j;
     const int64_t srow = (int64_t)p.phi * L::NS;  // stride of one S row
     const bool writer = r == 0 && valid_pair;
@@ -304,14 +433,14 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
             }
         }
     }
-    if (!need_reml && !need_mle) {  // score only: the large-lambda rewrite happens here
+    if (!GUIDE && !need_reml && !need_mle) {  // score only: the large-lambda rewrite
         double xs_m[L::NX], xs_r[L::NX];
         direct_fix<C, LP>(p, j, f, valid_pair, need_score, false, false, 0.0, 0.0, xs_m, xs_r);
         return;
     }
 
     // ---------------- shared lambda grid, LP points at a time
-    ArgMax best_reml, best_mle;
+    std::conditional_t<GUIDE, ArgMaxLead, ArgMax> best_reml, best_mle;
 #pragma unroll 1
     for (int g0 = 0; g0 < p.n_grid; g0 += LP) {
         double xs[L::NX];
@@ -332,15 +461,30 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
             if (need_mle) best_mle.push(k, mle_logl<C>(pb, ldh, p));
         }
     }
-    best_reml.warp_reduce<LP>();
-    best_mle.warp_reduce<LP>();
+    best_reml.template warp_reduce<LP>();
+    best_mle.template warp_reduce<LP>();
 
     // ---------------- golden sections, both searches in step
     const int bm = need_mle ? best_mle.idx : best_reml.idx;
     const int br = need_reml ? best_reml.idx : best_mle.idx;
-    Golden gm, gr;
+    Golden<GUIDE> gm, gr;
     gm.start(p, bm);
     gr.start(p, br);
+    SearchReport out_m, out_r;
+    if constexpr (GUIDE) {
+        if (writer) {
+            out_m = SearchReport{p.state + 2 * wid, 2 * wid, p.open_list, p.open_count};
+            out_r = SearchReport{p.state + 2 * wid + 1, 2 * wid + 1, p.open_list, p.open_count};
+        }
+        // the grid's decision: its values are as certain as the probes'
+        auto settle = [&](Golden<GUIDE>& gs, const ArgMaxLead& best, int at, const SearchReport& out) {
+            gs.tau = guide_tau<C>(p, g, at, f, r);
+            gs.certain = !best.nan && best.v - best.v2 > 4.0 * (gs.tau.whole + gs.tau.floor);
+            if (!gs.certain) out.put(SearchState{0.0, 0.0, 0.0, 0.0, -1.0}, true);
+        };
+        if (need_mle) settle(gm, best_mle, bm, out_m);
+        if (need_reml) settle(gr, best_reml, br, out_r);
+    }
     double xs_m[L::NX], xs_r[L::NX], sh_m[L::NS], sh_r[L::NS], ld_m = 0.0, ld_r = 0.0;
     PabOut<C> pb_m, pb_r;
 #pragma unroll 1
@@ -361,16 +505,17 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
                 ld_r = ld_m;
             }
         }
-        if (it == p.n_iter + 2) break;
+        if (!GUIDE && it == p.n_iter + 2) break;
         double row0[L::NI];
         if (need_mle) {
             assemble<C>(row0, sh_m, xs_m);
-            gm.take(mle_logl<C>(pab_reduce<C>(row0), ld_m, p), it, p.n_iter);
+            gm.take(mle_logl<C>(pab_reduce<C>(row0), ld_m, p), it, p.n_iter, out_m);
         }
         if (need_reml) {
             assemble<C>(row0, sh_r, xs_r);
-            gr.take(group_reml<C>(pab_reduce<C>(row0), log_iab, ld_r, p, r), it, p.n_iter);
+            gr.take(group_reml<C>(pab_reduce<C>(row0), log_iab, ld_r, p, r), it, p.n_iter, out_r);
         }
+        if (GUIDE && it == p.n_iter + 1) return;
     }
 
     // ---------------- statistics at the optima; at large lambda from direct x-sums
@@ -390,6 +535,416 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
         assemble<C>(row0, sh_r, xs_r);
         const PabOut<C> pb = pab_reduce<C>(row0);
         write_wald<C>(p, pb, reml_logl<C>(pb, log_iab, ld_r, p), exp(gr.s), o, writer);
+    }
+}
+
+// ---------------------------------------------------------------- plain form, guided
+// The plain form's golden sections would take a direct FP64 pass over x per probe (46 passes
+// with a logarithm and a reciprocal per sample and pair in mode 4), although nearly every
+// decision is far from a tie.  So lmm_search_kernel<C, true> takes the decisions that its
+// series approximations settle beyond their error (guide_tau), lmm_open_kernel takes the few
+// others by direct evaluations (lmm_close_kernel when they are many), and lmm_finish_kernel
+// makes one direct pass per pair for the
+// evaluations at the optima, whose sums the statistics use, and the score test.  Both form
+// their sums term by term in the order of eval_full, so every decision and every value is
+// the one that a search of direct evaluations gives.
+// Measured, search of direct evaluations -> search + open + close + finish: 8192 SNPs, n =
+// 1940, Wald 1976 -> 264 us; 2048 SNPs, three covariate columns, n = 10 000, every test 8294
+// -> 796 us; 2048 SNPs, n = 20 000, every test 10 536 -> 832 us (and 0.4 ms more for the 97
+// rows of series sums in place of 52 grid rows).  The gain shrinks where the likelihood is
+// flat: lambda at its upper bound, n = 20 000: 19.7 -> 13 ms for 2000 SNPs x 2 phenotypes.
+
+// One search by all threads of a CTA: tiles of kOpenTile samples staged in shared memory.
+constexpr int kOpenThreads = 256, kOpenTile = 512;
+template <int C>
+struct OpenSmem {
+    double col[Lay<C>::R][kOpenTile];  // W columns, x, y
+    double h[kOpenTile], ld[kOpenTile];
+    double sum[32];
+};
+
+// Log-likelihood at log-lambda s by all threads of the CTA, with eval_full's values: the
+// weights and logarithms of a tile of samples are formed by all threads, then each warp adds
+// up some of the NI + 1 sums over the tile as eval_full's one warp does.  The next tile's
+// loads are in flight meanwhile.
+template <int C, bool REML>
+__device__ double block_logl(const Params& p, const double* __restrict__ x,
+                             const double* __restrict__ y, double s,
+                             const double (&log_iab)[C + 1], OpenSmem<C>& sm) {
+    using L = Lay<C>;
+    constexpr int kWarps = kOpenThreads / 32, kSlots = (L::NI + kWarps) / kWarps;
+    constexpr int kPer = kOpenTile / kOpenThreads;  // samples of a tile per thread
+    static_assert(L::NI + 1 <= 32, "sums of a pair");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double lam = exp(s);
+    int ca[kSlots], cb[kSlots];  // this warp's sums: columns a <= b; log|H| is sum NI
+    double acc[kSlots];
+#pragma unroll
+    for (int q = 0; q < kSlots; ++q) {
+        acc[q] = 0.0;
+        ca[q] = cb[q] = 0;
+#pragma unroll
+        for (int a = 0; a < L::R; ++a)
+#pragma unroll
+            for (int b = a; b < L::R; ++b)
+                if (L::idx(a, b) == warp + q * kWarps) {
+                    ca[q] = a;
+                    cb[q] = b;
+                }
+    }
+    double ev[kPer], col[kPer][L::R];
+    auto fetch = [&](int64_t base) {
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) {
+            const int64_t i = base + threadIdx.x + e * kOpenThreads;
+            if (i >= p.n) continue;
+            ev[e] = __ldg(p.evals + i);
+#pragma unroll
+            for (int a = 0; a < C; ++a) col[e][a] = __ldg(p.W + a * p.ldw + i);
+            col[e][C] = x[i];
+            col[e][C + 1] = __ldg(y + i);
+        }
+    };
+    fetch(0);
+    for (int64_t base = 0; base < p.n; base += kOpenTile) {
+        const int len = (int)(p.n - base < kOpenTile ? p.n - base : kOpenTile);
+        __syncthreads();  // the previous tile (or call) has been read
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) {
+            const int i = threadIdx.x + e * kOpenThreads;
+            if (i >= len) continue;
+            const double v = __dadd_rn(__dmul_rn(lam, ev[e]), 1.0);
+            sm.h[i] = __drcp_rn(v);
+            sm.ld[i] = log(fabs(v));
+#pragma unroll
+            for (int a = 0; a < L::R; ++a) sm.col[a][i] = col[e][a];
+        }
+        __syncthreads();
+        if (base + kOpenTile < p.n) fetch(base + kOpenTile);
+#pragma unroll
+        for (int q = 0; q < kSlots; ++q) {
+            const int k = warp + q * kWarps;  // warp-uniform
+            const double *pa = sm.col[ca[q]], *pb = sm.col[cb[q]];
+            double t = acc[q];
+            if (k < L::NI) {
+#pragma unroll 8
+                for (int i = lane; i < len; i += 32) t = fma(sm.h[i] * pa[i], pb[i], t);
+            } else if (k == L::NI) {
+#pragma unroll 8
+                for (int i = lane; i < len; i += 32) t += sm.ld[i];
+            }
+            acc[q] = t;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kSlots; ++q) {
+        const double v = warp_sum(acc[q]);
+        if (lane == 0 && warp + q * kWarps <= L::NI) sm.sum[warp + q * kWarps] = v;
+    }
+    __syncthreads();
+    double row0[L::NI];
+#pragma unroll
+    for (int k = 0; k < L::NI; ++k) row0[k] = sm.sum[k];
+    const PabOut<C> pb2 = pab_reduce<C>(row0);
+    return REML ? reml_logl<C>(pb2, log_iab, sm.sum[L::NI], p) : mle_logl<C>(pb2, sm.sum[L::NI], p);
+}
+
+// Iab's logarithms of a pair (H = 1: the chunk's ones row).
+template <int C>
+__device__ __forceinline__ void pair_log_iab(const Params& p, int64_t j, int f,
+                                             double (&log_iab)[C + 1]) {
+    using L = Lay<C>;
+    double xs[L::NX], row0[L::NI];
+    const double* cl = p.CL + j * p.ldcl;
+#pragma unroll
+    for (int a = 0; a < C; ++a) xs[a] = cl[a];
+    xs[C] = p.CQ[j * p.ldcq];
+    xs[C + 1] = cl[C + f];
+    assemble<C>(row0, p.S + ((int64_t)p.n_grid * p.phi + f) * L::NS, xs);
+    const PabOut<C> pb = pab_reduce<C>(row0);
+#pragma unroll
+    for (int i = 0; i <= C; ++i) log_iab[i] = pb.diag[i] > 0 ? log(pb.diag[i]) : 0.0;
+}
+
+// Takes the open decisions of a search: `probe` evaluates a log-likelihood directly,
+// `grid_best` picks the grid point.  Returns the optimum (a + b) / 2.
+template <class Probe, class Grid>
+__device__ __forceinline__ double close_golden(const Params& p, const SearchState& st, Probe probe,
+                                               Grid grid_best) {
+    double a = st.a, b = st.b, sc = st.sc, sd = st.sd;
+    int it = (int)st.step;
+    if (it < 0) {  // the grid as well
+        const int best = grid_best();
+        a = p.loglam[best - 1 > 0 ? best - 1 : 0];
+        b = p.loglam[best + 1 < p.n_grid - 1 ? best + 1 : p.n_grid - 1];
+        sc = __dsub_rn(b, __dmul_rn(kPhi, __dsub_rn(b, a)));
+        sd = __dadd_rn(a, __dmul_rn(kPhi, __dsub_rn(b, a)));
+        it = 0;
+    }
+    if (it < p.n_iter) {
+        double c = __dsub_rn(b, __dmul_rn(kPhi, __dsub_rn(b, a)));
+        double d = __dadd_rn(a, __dmul_rn(kPhi, __dsub_rn(b, a)));
+        double fc = 0.0, fd = 0.0, s = sc;
+        bool left = true;
+        for (int e = 0;; ++e) {  // one copy of the evaluation: both inner values, then the steps
+            const double f = probe(s);
+            fc = left ? f : fc;
+            fd = left ? fd : f;
+            if (e == 0) {
+                s = sd;
+                left = false;
+                continue;
+            }
+            left = fc > fd;
+            a = left ? a : c;
+            b = left ? d : b;
+            if (++it == p.n_iter) break;
+            const double keep = left ? fc : fd;
+            fc = keep;
+            fd = keep;
+            c = __dsub_rn(b, __dmul_rn(kPhi, __dsub_rn(b, a)));
+            d = __dadd_rn(a, __dmul_rn(kPhi, __dsub_rn(b, a)));
+            s = left ? c : d;
+        }
+    }
+    return __dmul_rn(__dadd_rn(a, b), 0.5);
+}
+
+// The grid point of a search whose grid decision is open, from the tabulated H rows: x-sums
+// of kRun points a pass by THREADS threads, added up over the warps in `red`.
+template <int C, bool REML, int THREADS>
+__device__ __forceinline__ int direct_grid(const Params& p, const double* __restrict__ x,
+                                           const double* __restrict__ y, int f,
+                                           const double (&log_iab)[C + 1], double* red) {
+    using L = Lay<C>;
+    constexpr int kRun = 4, kWarps = THREADS / 32;
+    const int tid = THREADS == 32 ? threadIdx.x & 31 : threadIdx.x;
+    ArgMax best;
+#pragma unroll 1
+    for (int g0 = 0; g0 < p.n_grid; g0 += kRun) {
+        double acc[kRun][L::NX];
+#pragma unroll
+        for (int e = 0; e < kRun; ++e)
+#pragma unroll
+            for (int q = 0; q < L::NX; ++q) acc[e][q] = 0.0;
+        for (int64_t i = tid; i < p.n; i += THREADS) {
+            const double xv = x[i], yv = __ldg(y + i);
+            double w[C];
+#pragma unroll
+            for (int q = 0; q < C; ++q) w[q] = __ldg(p.W + q * p.ldw + i);
+#pragma unroll
+            for (int e = 0; e < kRun; ++e) {
+                const int g = g0 + e < p.n_grid ? g0 + e : p.n_grid - 1;
+                const double t = __ldg(p.H + (int64_t)g * p.n + i) * xv;
+#pragma unroll
+                for (int q = 0; q < C; ++q) acc[e][q] = fma(t, w[q], acc[e][q]);
+                acc[e][C] = fma(t, xv, acc[e][C]);
+                acc[e][C + 1] = fma(t, yv, acc[e][C + 1]);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < kRun; ++e) {
+            double xs[L::NX], row0[L::NI];
+#pragma unroll
+            for (int q = 0; q < L::NX; ++q) xs[q] = warp_sum(acc[e][q]);
+            if (THREADS > 32) {
+                __syncthreads();
+                if ((tid & 31) == 0)
+#pragma unroll
+                    for (int q = 0; q < L::NX; ++q) red[q * kWarps + (tid >> 5)] = xs[q];
+                __syncthreads();
+#pragma unroll
+                for (int q = 0; q < L::NX; ++q) {
+                    xs[q] = red[q * kWarps];
+                    for (int w = 1; w < kWarps; ++w) xs[q] += red[q * kWarps + w];
+                }
+            }
+            if (g0 + e >= p.n_grid) continue;
+            assemble<C>(row0, p.S + ((int64_t)(g0 + e) * p.phi + f) * L::NS, xs);
+            const PabOut<C> pb = pab_reduce<C>(row0);
+            const double ldh = p.logdet[g0 + e];
+            best.push(g0 + e, REML ? reml_logl<C>(pb, log_iab, ldh, p) : mle_logl<C>(pb, ldh, p));
+        }
+    }
+    return best.idx;
+}
+
+// Few open searches (the usual chunk: a fraction of a percent): one CTA takes one at a time,
+// so that they do not make a long tail of one warp each.  With more of them than
+// kOpenPerSm per SM the CTAs' synchronisation costs more than it saves, and lmm_close_kernel
+// takes them, one warp each.
+constexpr int kOpenPerSm = 4;
+
+template <int C, bool REML>
+__device__ __noinline__ double open_search(const Params& p, int64_t wid, OpenSmem<C>& sm) {
+    const int64_t j = wid / p.phi;
+    const int f = (int)(wid % p.phi);
+    const double* __restrict__ x = p.G + j * p.ldg;
+    const double* __restrict__ y = p.Y + (int64_t)f * p.ldy;
+    double log_iab[C + 1];
+#pragma unroll
+    for (int i = 0; i <= C; ++i) log_iab[i] = 0.0;
+    if (REML) pair_log_iab<C>(p, j, f, log_iab);
+    return close_golden(
+        p, p.state[2 * wid + (REML ? 1 : 0)],
+        [&](double s) { return block_logl<C, REML>(p, x, y, s, log_iab, sm); },
+        [&] { return direct_grid<C, REML, kOpenThreads>(p, x, y, f, log_iab, sm.h); });
+}
+
+template <int C>
+__global__ void __launch_bounds__(kOpenThreads, 1) lmm_open_kernel(const Params p, int64_t most) {
+    __shared__ OpenSmem<C> sm;
+    const int64_t count = *p.open_count;
+    if (count > most) return;
+    for (int64_t e = blockIdx.x; e < count; e += gridDim.x) {
+        const int64_t at = p.open_list[e];  // 2 pair + (1: REML)
+        const double s = at & 1 ? open_search<C, true>(p, at >> 1, sm)
+                                : open_search<C, false>(p, at >> 1, sm);
+        __syncthreads();  // every thread has read the state
+        if (threadIdx.x == 0) p.state[at] = SearchState{s, s, s, s, (double)p.n_iter};
+    }
+}
+
+template <int C, bool REML>
+__device__ __noinline__ double close_search(const Params& p, int64_t wid) {
+    const int64_t j = wid / p.phi;
+    const int f = (int)(wid % p.phi);
+    const double* __restrict__ x = p.G + j * p.ldg;
+    const double* __restrict__ y = p.Y + (int64_t)f * p.ldy;
+    double log_iab[C + 1];
+#pragma unroll
+    for (int i = 0; i <= C; ++i) log_iab[i] = 0.0;
+    if (REML) pair_log_iab<C>(p, j, f, log_iab);
+    return close_golden(
+        p, p.state[2 * wid + (REML ? 1 : 0)],
+        [&](double s) { return eval_logl<C, REML>(p, x, y, s, log_iab, nullptr); },
+        [&] { return direct_grid<C, REML, 32>(p, x, y, f, log_iab, nullptr); });
+}
+
+template <int C>
+__global__ void __launch_bounds__(kPairsThreads, PairsOccupancy<C>::kMinBlocks)
+    lmm_close_kernel(const Params p, int64_t most) {
+    const int64_t count = *p.open_count;
+    if (count <= most) return;
+    const int64_t nw = (int64_t)gridDim.x * kPairsThreads / 32;
+    for (int64_t e = ((int64_t)blockIdx.x * kPairsThreads + threadIdx.x) / 32; e < count; e += nw) {
+        const int64_t at = p.open_list[e];
+        const double s = at & 1 ? close_search<C, true>(p, at >> 1) : close_search<C, false>(p, at >> 1);
+        __syncwarp();  // every lane has read the state
+        if ((threadIdx.x & 31) == 0) p.state[at] = SearchState{s, s, s, s, (double)p.n_iter};
+    }
+}
+
+// One pass over x per pair, one warp each: the sums at the MLE and REML optima and the score
+// test's sums at the null lambda (its H row is tabulated).  Bound by FP64 issue: a logarithm,
+// a reciprocal and, with one covariate column, 9 multiply-adds per sample and optimum.
+template <int C>
+__global__ void __launch_bounds__(kPairsThreads, PairsOccupancy<C>::kMinBlocks)
+    lmm_finish_kernel(const Params p) {
+    using L = Lay<C>;
+    constexpr int U = C <= 2 ? 4 : 2;  // samples in flight
+    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    if (wid >= p.m * p.phi) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t j = wid / p.phi;
+    const int f = (int)(wid % p.phi);
+    const double* __restrict__ x = p.G + j * p.ldg;
+    const double* __restrict__ y = p.Y + (int64_t)f * p.ldy;
+    const double* __restrict__ h0 = p.H + (int64_t)(p.n_grid + f) * p.n;
+    const int64_t o = (int64_t)f * p.m + j;
+    const bool on[2] = {p.mode == 2 || p.mode == 4, p.mode == 1 || p.mode == 4};  // MLE, REML
+    const bool score = p.mode == 3 || p.mode == 4;
+    double s[2] = {0.0, 0.0}, lam[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        if (on[q]) s[q] = __dmul_rn(__dadd_rn(p.state[2 * wid + q].a, p.state[2 * wid + q].b), 0.5);
+        lam[q] = exp(s[q]);
+    }
+    double acc[2][L::NI], ld[2] = {0.0, 0.0}, xs0[L::NX];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int k = 0; k < L::NI; ++k) acc[q][k] = 0.0;
+#pragma unroll
+    for (int k = 0; k < L::NX; ++k) xs0[k] = 0.0;
+    for (int64_t i0 = lane; i0 < p.n; i0 += 32 * U) {
+        double ev[U], hv[U], vec[U][L::R];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {  // past the end: a sample without weight
+            const int64_t i = i0 + 32 * u;
+            const bool in = i < p.n;
+            ev[u] = in ? __ldg(p.evals + i) : 0.0;
+            hv[u] = in && score ? __ldg(h0 + i) : 0.0;
+#pragma unroll
+            for (int a = 0; a < C; ++a) vec[u][a] = in ? __ldg(p.W + a * p.ldw + i) : 0.0;
+            vec[u][C] = in ? x[i] : 0.0;
+            vec[u][C + 1] = in ? __ldg(y + i) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (!on[q]) continue;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const double v = __dadd_rn(__dmul_rn(lam[q], ev[u]), 1.0);
+                const double h = __drcp_rn(v);
+                ld[q] += log(fabs(v));
+#pragma unroll
+                for (int a = 0; a < L::R; ++a) {
+                    const double t = h * vec[u][a];
+#pragma unroll
+                    for (int b = a; b < L::R; ++b)
+                        acc[q][L::idx(a, b)] = fma(t, vec[u][b], acc[q][L::idx(a, b)]);
+                }
+            }
+        }
+        if (score) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const double t = hv[u] * vec[u][C];
+#pragma unroll
+                for (int a = 0; a < C; ++a) xs0[a] = fma(t, vec[u][a], xs0[a]);
+                xs0[C] = fma(t, vec[u][C], xs0[C]);
+                xs0[C + 1] = fma(t, vec[u][C + 1], xs0[C + 1]);
+            }
+        }
+    }
+    if (score) {
+        double row0[L::NI];
+#pragma unroll
+        for (int k = 0; k < L::NX; ++k) xs0[k] = warp_sum(xs0[k]);
+        assemble<C>(row0, p.S + ((int64_t)(p.n_grid + 1 + f) * p.phi + f) * L::NS, xs0);
+        const PabOut<C> pb = pab_reduce<C>(row0);
+        bool valid;
+        double beta, tau, se;
+        beta_se<C>(pb, clamp_pyy(pb.yy1), p.df, valid, beta, tau, se);
+        const double fstat = p.n_d * (pb.xy * pb.xy) / (pb.yy * (valid ? pb.xx : 1.0));
+        if (lane == 0) {
+            if (p.out.p_score) p.out.p_score[o] = valid ? fstat : jnan();
+            if (p.mode == 3) {
+                if (p.out.beta) p.out.beta[o] = beta;
+                if (p.out.se) p.out.se[o] = se;
+            }
+        }
+    }
+    if (on[0]) {
+        double row0[L::NI];
+#pragma unroll
+        for (int k = 0; k < L::NI; ++k) row0[k] = warp_sum(acc[0][k]);
+        const double logl = mle_logl<C>(pab_reduce<C>(row0), warp_sum(ld[0]), p);
+        if (lane == 0) {
+            if (p.out.lambda_mle) p.out.lambda_mle[o] = lam[0];
+            if (p.out.logl_mle) p.out.logl_mle[o] = logl;
+            const double stat = jmax(2.0 * (logl - p.logl0[f]), 0.0);
+            if (p.out.p_lrt) p.out.p_lrt[o] = chi2_1_sf(stat);
+        }
+    }
+    if (on[1]) {
+        double row0[L::NI], log_iab[C + 1];
+        pair_log_iab<C>(p, j, f, log_iab);
+#pragma unroll
+        for (int k = 0; k < L::NI; ++k) row0[k] = warp_sum(acc[1][k]);
+        const PabOut<C> pb = pab_reduce<C>(row0);
+        write_wald<C>(p, pb, reml_logl<C>(pb, log_iab, warp_sum(ld[1]), p), lam[1], o, lane == 0);
     }
 }
 

@@ -35,6 +35,10 @@ MAX_CVT = 4
 NULL_L_MIN, NULL_L_MAX, NULL_N_GRID, NULL_N_ITER = 1e-5, 1e5, 50, 20
 # log-lambda domain of the mixed form's series tables (jb_lmm_prepare precision 1)
 SERIES_L_MIN, SERIES_L_MAX = 1e-5, 1e5
+# The FP64 form's guided search: fewest grid points at which the degree-24 bracket expansions
+# truncate below 1e-15, and fewest samples at which it is the faster one (4000 SNPs x 2
+# phenotypes, every test, direct -> guided: n = 300 1.4 -> 2.5 ms, n = 500 1.9 -> 0.7 ms)
+GUIDE_MIN_GRID, GUIDE_MIN_SAMPLES = 16, 400
 
 
 def eigh_device(K: torch.Tensor, threshold: float = 1e-10) -> tuple[torch.Tensor, torch.Tensor]:
@@ -135,11 +139,18 @@ class DeviceCohort:
         # The interpolated search expands 1/(lambda*eval + 1) in log lambda over the fixed
         # domain [1e-5, 1e5]: it needs the user's range inside that domain and no pole of
         # the weights near it; otherwise every probe is evaluated directly in FP64.
+        # The FP64 form stays a search of direct evaluations (search 0), with the decisions
+        # that are far from a tie taken on the same series where these hold and its golden
+        # brackets are narrow enough for their expansions to reach rounding level.
         ev_min = float(self.evals.min().item())
-        self.search = 1 if (precision == "mixed" and 1.0 + SERIES_L_MAX * ev_min > 0.5
-                            and self.l_min >= SERIES_L_MIN and self.l_max <= SERIES_L_MAX) else 0
+        series = (1.0 + SERIES_L_MAX * ev_min > 0.5
+                  and self.l_min >= SERIES_L_MIN and self.l_max <= SERIES_L_MAX)
+        self.search = 1 if precision == "mixed" and series else 0
+        self.guided = (precision == "fp64" and series and self.n_grid >= GUIDE_MIN_GRID
+                       and n >= GUIDE_MIN_SAMPLES)
+        self._form = 3 if self.guided else self.search  # native precision argument
         self.ws = workspace(_native.load().jb_lmm_workspace_size(n, c, phi, self.n_grid))
-        _native.call("jb_lmm_prepare", lmm_mode, self.search, n, c, phi, ptr(self.evals), ptr(self.UtW), n,
+        _native.call("jb_lmm_prepare", lmm_mode, self._form, n, c, phi, ptr(self.evals), ptr(self.UtW), n,
                      ptr(self.Uty), n, ptr(self.lam0), self.l_min, self.l_max, self.n_grid,
                      ptr(self.ws), self.ws.numel(), st)
         # Mixed form with the series search: the linear genotype sums of each chunk come
@@ -174,7 +185,7 @@ class DeviceCohort:
         out = out if out is not None else self.alloc_out(m)
         o = _native.LmmOut(**{k: ptr(out.get(k)) for k in OUT_KEYS})
         cws = self.chunk_workspace(m)
-        precision = self.search
+        precision = self._form
         if self._series_for is not None and self._series_for == (m, UtG.data_ptr()):
             precision = 2  # linear sums already formed from this chunk's int8 calls
         self._series_for = None
@@ -273,7 +284,8 @@ class ChunkGraph:
         n_file = n if n_file is None else n_file
         self.cohort, self.m, self.n_file, self.sample_idx = cohort, m, n_file, sample_idx
         self.has_missing = bool(has_missing)
-        self.packed = torch.zeros((m, (n_file + 3) // 4), dtype=torch.uint8, device="cuda")
+        # "no copies" calls: without prefill the warm-up tests all-zero genotypes
+        self.packed = torch.full((m, (n_file + 3) // 4), 255, dtype=torch.uint8, device="cuda")
         self.means = torch.zeros((m,), dtype=torch.float64, device="cuda")
         self.codes = torch.zeros((m, cohort.code_ld), dtype=torch.int8, device="cuda")
         self.counts = torch.zeros((m, 4), dtype=torch.int32, device="cuda")
