@@ -287,6 +287,26 @@ int32_t jb_rotate_i8(const void* ozaki_ws, int64_t n, const int8_t* codes, int64
                      uintptr_t stream);
 int32_t jb_rotate_status(const void* workspace, int32_t* out, uintptr_t stream);
 
+/*
+ * FP64 rotation of genotype calls on INT8 tensor cores: X = U^T G to FP64 accuracy, for calls
+ * that are small integers (decoded codes, 3 = missing, mean-imputed with mean[j] without
+ * centring).  jb_split_f64_prepare writes U (n x n, column-major, ldu) once per cohort as
+ * seven exact int8 digit planes (base 254, a power-of-two scale per eigenvector; remainder
+ * below 3e-17 max|U_col|); jb_rotate_codes_f64 sums every digit product exactly in int32
+ * and adds the seven in FP64.  has_missing = 0 says that the chunk holds no missing call and
+ * halves the work; a missing call found all the same is imputed as with has_missing = 1.
+ * Workspace: jb_rotate_codes_f64_workspace_size(n, m) bytes, its first int32 a pipeline status
+ * word as for jb_rotate_i8 (jb_rotate_status).  n < 2^23.
+ */
+int64_t jb_split_f64_workspace_size(int64_t n);
+int32_t jb_split_f64_prepare(const double* U, int64_t n, int64_t ldu, void* planes,
+                             int64_t planes_bytes, uintptr_t stream);
+int64_t jb_rotate_codes_f64_workspace_size(int64_t n, int64_t m);
+int32_t jb_rotate_codes_f64(const void* planes, int64_t n, const int8_t* codes,
+                            int64_t ld_codes, int64_t m, const double* mean,
+                            int32_t has_missing, double* X, int64_t ldx, void* workspace,
+                            int64_t workspace_bytes, uintptr_t stream);
+
 /* ------------------------------------------------------------------ association */
 
 /* Output arrays of jb_lmm_chunk; each is phi x m (phenotype-major, ld = m) or NULL. */

@@ -94,6 +94,10 @@ SIGNATURES: dict[str, tuple] = {
     "jb_rotate_i8_workspace_size": (_i64, [_i64, _i64]),
     "jb_rotate_i8": (_i32, [_p, _i64, _p, _i64, _i64, _p, _i32, _p, _i64, _p, _i64, _u]),
     "jb_rotate_status": (_i32, [_p, _p, _u]),
+    "jb_split_f64_workspace_size": (_i64, [_i64]),
+    "jb_split_f64_prepare": (_i32, [_p, _i64, _i64, _p, _i64, _u]),
+    "jb_rotate_codes_f64_workspace_size": (_i64, [_i64, _i64]),
+    "jb_rotate_codes_f64": (_i32, [_p, _i64, _p, _i64, _i64, _p, _i32, _p, _i64, _p, _i64, _u]),
     "jb_null_mle": (
         _i32,
         [_i64, _i32, _i32, _p, _p, _i64, _p, _i64, _f64, _f64, _i32, _i32, _p, _p, _u],

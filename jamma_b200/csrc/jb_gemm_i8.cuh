@@ -5,7 +5,7 @@
 // A and B are K-major int8 matrices described by TMA tensor maps (128-byte K boxes,
 // 128B swizzle).  One CTA per SM walks a tile list; its 6 warps split the work:
 //   warp 0      TMA producer: fills a STAGES-deep ring of (A, B) K-slices;
-//   warp 1      allocates TMEM (2 accumulators x BN columns) and, from one thread,
+//   warp 1      allocates TMEM (2 accumulators of BN <= 256 columns) and, from one thread,
 //               issues tcgen05.mma (M=128, N=BN, K=32) into the current accumulator,
 //               committing each consumed stage back to the producer and each finished
 //               tile to the epilogue;
@@ -13,6 +13,7 @@
 //               (warp w owns TMEM lanes 32*(w%4)..+31 = tile rows), hand the values to
 //               the Epi functor, then release the accumulator.
 // Integer accumulation is exact, so results do not depend on K order or tiling.
+// A launch with a gate returns at once unless *gate == gate_value.
 #pragma once
 
 #include "jb_tc.cuh"
@@ -55,8 +56,12 @@ struct Tile {
 template <int BN, int STAGES, class Epi>
 __global__ void __launch_bounds__(kThreads, 1)
     i8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                   const Tile* __restrict__ tiles, int n_tiles, int num_kb, Epi epi, int* err) {
+                   const Tile* __restrict__ tiles, int n_tiles, int num_kb, Epi epi, int* err,
+                   const int* gate = nullptr, int gate_value = 0) {
     using S = GemmSmem<BN, STAGES, Epi::kSmem>;
+    constexpr int kTmemCols = 512, kAcc = 256;  // two accumulators, 256 columns apart
+    static_assert(BN <= kAcc, "accumulator columns");
+    if (gate && *gate != gate_value) return;  // the same decision in every CTA
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -89,7 +94,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
     }
-    if (warp == 1) tmem_alloc(tmem_slot, 2 * BN);
+    if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -126,7 +131,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int t = blockIdx.x; t < n_tiles && !*abort; t += gridDim.x) {
                 if (!mbar_wait(&tempty[acc], acc_phase ^ 1, abort, err, 2, wait_ns)) break;
                 tc_fence_after();
-                const uint32_t d = tmem_base + (uint32_t)(acc * BN);
+                const uint32_t d = tmem_base + (uint32_t)(acc * kAcc);
                 for (int kb = 0; kb < num_kb; ++kb) {
                     if (!mbar_wait(&full[stage], phase, abort, err, 3, wait_ns)) break;
                     tc_fence_after();
@@ -163,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!proceed) break;
             tc_fence_after();
             const Tile tl = tiles[t];
-            epi.run(tl.mb, tl.nb, tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(acc * BN), q,
+            epi.run(tl.mb, tl.nb, tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(acc * kAcc), q,
                     lane, epi_smem);
             tc_fence_before();
             mbar_arrive(&tempty[acc]);
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 1) tmem_dealloc(tmem_base, 2 * BN);
+    if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
 // ---------------------------------------------------------------- CTA-pair variant

@@ -693,7 +693,7 @@ int32_t jb_gram_i8(const int8_t* Z, int64_t n, int64_t p, int64_t ldz, int32_t* 
     GramEpi epi{C, ldc, (int)n};
     const int grid = n_tiles < num_sms() ? n_tiles : num_sms();
     const int num_kb = (int)ceil_div(p, kBK);
-    kern<<<grid, kThreads, GramSmem::TOTAL, st>>>(ta, tb, tiles, n_tiles, num_kb, epi, status);
+    kern<<<grid, kThreads, GramSmem::TOTAL, st>>>(ta, tb, tiles, n_tiles, num_kb, epi, status, nullptr, 0);
     JB_LAUNCH_CHECK("i8_gemm_kernel<gram>");
     return JB_OK;
 }
@@ -752,6 +752,7 @@ int32_t jb_test_pipeline_timeout(int32_t skip_loads, int64_t wait_limit_ns) {
     const unsigned long long lim = (unsigned long long)wait_limit_ns;
     JB_CUDA(pipeline_test_mode(skip_loads ? 1 : 0, lim));
     JB_CUDA(rotate_pipeline_test_mode(skip_loads ? 1 : 0, lim));
+    JB_CUDA(rotate_f64_pipeline_test_mode(skip_loads ? 1 : 0, lim));
     return JB_OK;
 }
 
@@ -938,7 +939,7 @@ int32_t jb_kinship_i8_corrections_tc(const int8_t* codes, int64_t ld_codes, cons
     const int n_tiles = MB * NB;
     KinREpi epi{RT, ldr, (int)n};
     kern<<<n_tiles < num_sms() ? n_tiles : num_sms(), kThreads, GramSmem::TOTAL, st>>>(
-        ta, tb, tiles, n_tiles, (int)ceil_div(m, kBK), epi, status);
+        ta, tb, tiles, n_tiles, (int)ceil_div(m, kBK), epi, status, nullptr, 0);
     JB_LAUNCH_CHECK("i8_gemm_kernel<kinship R>");
     // T/2 from the per-SNP missing lists
     return kin_missing_terms(codes, ld_codes, n, m, mu, RT, ldr, L, ws, false, st);

@@ -1,0 +1,356 @@
+// FP64 eigenvector rotation x~ = U^T g of genotype calls on INT8 tensor cores.
+//
+// Calls are small integers, so U^T g needs no FP64 multiplier: each eigenvector u_i (column i
+// of U) is scaled by a power of two s_i (s_i 127 >= max |u_i| > s_i 63.5) and written in seven
+// signed base-254 digits, U_ki = s_i sum_{t<7} q_t(k,i) 254^-t.  Every step of the split is
+// exact in FP64; what is left over is below s_i 254^-6 / 2, i.e. 3e-17 of max |u_i| -- less
+// than the rounding of U itself.  Each digit product accumulates exactly in int32 on tcgen05
+// (kind::i8) and the epilogue adds the seven products in FP64, so the result carries a few
+// roundings of its own size, where an FP64 GEMM carries those of n partial sums (measured
+// against exact sums, n = 20 000: see jb_rotate_codes_f64's test).
+//
+// Missing calls are mean-imputed without centring (src/jamma/lmm/runner_streaming.py:
+// 427-434), g_j = z_j + mu_j m_j with m_j the missing mask: x~ = U^T z + mu_j U^T m.
+//
+// Bound by the INT8 pipe: 7 products for the calls and 7 for the masks, 28 n^2 m operations
+// against 2 n^2 m on the FP64 pipe, at ~90 times its rate.
+//
+// Tiles: SNPs on M, digits on N.  An A tile is 128 rows: the calls of 64 SNPs and their masks,
+// or the calls of 128 SNPs; a B tile is the 7 x 32 = 224 digit rows of 32 eigenvectors (digit
+// t of eigenvector 32 b + e at row 224 b + 32 t + e).  All digits of an output then lie in one
+// TMEM lane, 32 columns apart, and the epilogue thread of that lane adds them in registers;
+// only the mask sums cross between lanes, through shared memory, on the way to the transposed
+// store.  N = 224 runs at the full rate of M = 128 tiles.
+#include "jb_common.cuh"
+#include "jb_gemm_i8.cuh"
+#include "jb_rotate_i8.cuh"
+
+namespace jb {
+namespace tc {
+
+int32_t make_map_i8(CUtensorMap* map, const void* base, int64_t rows, int64_t k, int64_t ld,
+                    int box_rows);
+int num_sms();
+
+constexpr int kXDigits = 7;
+constexpr int kXBN = 32 * kXDigits;   // digit rows of 32 eigenvectors
+constexpr int kXStages = 4;
+constexpr int kXLd = 33;              // padded row of the epilogue's output tile
+constexpr int kXEpiSmem = 128 * kXLd * 8;
+constexpr double kXBase = 254.0;
+using XSmem = GemmSmem<kXBN, kXStages, kXEpiSmem>;
+
+// ---------------------------------------------------------------- digit split
+// One CTA per eigenvector: its scale, then its seven digit rows.  scale[i] = s_i, 0 for a
+// zero eigenvector (no digits), NaN if an element is not finite (every output of that row
+// becomes NaN, as in a GEMM).
+__global__ void __launch_bounds__(256) xsplit_kernel(const double* __restrict__ U, int64_t n,
+                                                     int64_t ldu, int8_t* __restrict__ A,
+                                                     int64_t lda, double* __restrict__ scale) {
+    const int64_t i = blockIdx.x;
+    const double* __restrict__ col = U + i * ldu;
+    double mx = 0.0;
+    bool bad = false;
+    for (int64_t k = threadIdx.x; k < n; k += blockDim.x) {
+        const double a = fabs(col[k]);
+        bad = bad || !(a <= 1.7976931348623157e308);
+        mx = fmax(mx, a);
+    }
+    __shared__ double red[8];
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    bad = __syncthreads_or(bad);
+    for (int w = 0; w < 8; ++w) mx = fmax(mx, red[w]);
+    // 2^e with 63.5 < mx 2^e <= 127
+    int e = 0;
+    const bool zero = bad || !(mx > 0.0);
+    if (!zero) {
+        frexp(mx, &e);  // mx = f 2^e, f in [1/2, 1)
+        e = 7 - e;      // mx 2^e in [64, 128)
+        if (scalbn(mx, e) > 127.0) --e;
+    }
+    if (threadIdx.x == 0)
+        scale[i] = bad ? __longlong_as_double(0x7ff8000000000000ll) : (zero ? 0.0 : scalbn(1.0, -e));
+    int8_t* __restrict__ rows = A + ((i / 32) * kXBN + (i % 32)) * lda;
+    for (int64_t k = 4 * (int64_t)threadIdx.x; k < lda; k += 4 * (int64_t)blockDim.x) {
+        uint32_t w[kXDigits];
+#pragma unroll
+        for (int t = 0; t < kXDigits; ++t) w[t] = 0u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (k + q >= n || zero) continue;
+            double a = scalbn(col[k + q], e);  // |a| <= 127, exact
+#pragma unroll
+            for (int t = 0; t < kXDigits; ++t) {
+                const double r = rint(a);
+                w[t] |= (uint32_t)(uint8_t)(int8_t)(int)r << (8 * q);
+                a = (a - r) * kXBase;  // exact: |a - r| <= 1/2 drops 7 leading bits, 254 adds 7
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < kXDigits; ++t)
+            *reinterpret_cast<uint32_t*>(rows + 32 * t * lda + k) = w[t];
+    }
+}
+
+// ---------------------------------------------------------------- A operand
+// Block b of 64 SNPs: rows [128 b, +64) the calls (missing -> 0), rows [128 b + 64, +64) the
+// masks; 16 bytes of each per thread.  SNPs and samples past the end read as call 0.
+__global__ void __launch_bounds__(256) xpack_kernel(const int8_t* __restrict__ codes, int64_t ldc,
+                                                    int64_t n, int64_t m, int8_t* __restrict__ A,
+                                                    int64_t lda, const int* gate) {
+    if (gate && !*gate) return;
+    const int64_t j = blockIdx.x;
+    int8_t* z = A + ((j / 64) * 128 + j % 64) * lda;
+    int8_t* mk = z + 64 * lda;
+    const bool vec = (reinterpret_cast<uintptr_t>(codes) & 15) == 0 && (ldc & 15) == 0;
+    for (int64_t k = 16 * (int64_t)threadIdx.x; k < lda; k += 16 * (int64_t)blockDim.x) {
+        uint32_t c[4] = {0u, 0u, 0u, 0u}, v[4], u[4];
+        if (j < m) {
+            const int8_t* row = codes + j * ldc + k;
+            if (vec && k + 16 <= n) {
+                const uint4 q = __ldg(reinterpret_cast<const uint4*>(row));
+                c[0] = q.x;
+                c[1] = q.y;
+                c[2] = q.z;
+                c[3] = q.w;
+            } else {
+                for (int q = 0; q < 16; ++q)
+                    if (k + q < n) c[q >> 2] |= (uint32_t)(uint8_t)row[q] << (8 * (q & 3));
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t m3 = __vcmpeq4(c[q], 0x03030303u);
+            v[q] = c[q] & ~m3;
+            u[q] = m3 & 0x01010101u;
+        }
+        *reinterpret_cast<uint4*>(z + k) = make_uint4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<uint4*>(mk + k) = make_uint4(u[0], u[1], u[2], u[3]);
+    }
+}
+
+// *found = 1 if a call is missing (callers may promise that none is; the promise is checked,
+// since an unmarked missing call would count as a call of 3).
+__global__ void __launch_bounds__(256) xfind_missing_kernel(const int8_t* __restrict__ codes,
+                                                            int64_t ldc, int64_t n, int64_t m,
+                                                            int* found) {
+    bool any = false;
+    for (int64_t j = blockIdx.x; j < m; j += gridDim.x) {
+        const int8_t* row = codes + j * ldc;  // 16-byte aligned rows (see jb_rotate_codes_f64)
+        for (int64_t k = 16 * (int64_t)threadIdx.x; k < n; k += 16 * (int64_t)blockDim.x) {
+            if (k + 16 <= n) {
+                const uint4 q = __ldg(reinterpret_cast<const uint4*>(row + k));
+                any = any || (__vcmpeq4(q.x, 0x03030303u) | __vcmpeq4(q.y, 0x03030303u) |
+                              __vcmpeq4(q.z, 0x03030303u) | __vcmpeq4(q.w, 0x03030303u)) != 0u;
+            } else {
+                for (int64_t i = k; i < n; ++i) any = any || row[i] == 3;
+            }
+        }
+    }
+    if (__syncthreads_or(any) && threadIdx.x == 0) *found = 1;
+}
+
+// ---------------------------------------------------------------- epilogue
+template <bool PAIRED>
+struct XEpi {
+    static constexpr int kSmem = kXEpiSmem;
+    double* X;            // x~ (n x m, column-major, ld ldx)
+    int64_t ldx;
+    const double* scale;  // per eigenvector
+    const double* mu;     // per SNP (PAIRED)
+    int n, m;
+    __device__ __forceinline__ void run(int mb, int nb, uint32_t taddr, int q, int lane,
+                                        uint8_t* smem) const {
+        double* S = reinterpret_cast<double*>(smem);  // [row][kXLd]
+        constexpr int kRows = PAIRED ? 64 : 128;      // SNPs of the tile
+        constexpr double w1 = 1.0 / kXBase;
+        const int row = 32 * q + lane;                // TMEM lane
+        const int i0 = nb * 32;
+        // V[e] = sum_t C_t 254^-t, smallest digit first (Horner's rule from the last digit)
+        double v[32];
+        {
+            uint32_t c[32];
+            tmem_ld32(taddr + 32 * (kXDigits - 1), c);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) v[e] = (double)(int32_t)c[e];
+        }
+#pragma unroll 1
+        for (int t = kXDigits - 2; t >= 0; --t) {
+            uint32_t c[32];
+            tmem_ld32(taddr + (uint32_t)(32 * t), c);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) v[e] = fma(v[e], w1, (double)(int32_t)c[e]);
+        }
+        if (PAIRED) {
+            if (q >= 2) {  // mask sums of SNP row - 64
+#pragma unroll
+                for (int e = 0; e < 32; ++e) S[(row - 64) * kXLd + e] = v[e];
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (q < 2) {
+                const int j = mb * 64 + row;
+                const double u = j < m ? __ldg(mu + j) : 0.0;
+#pragma unroll
+                for (int e = 0; e < 32; ++e) {
+                    const double vm = S[row * kXLd + e];
+                    const double sc = i0 + e < n ? __ldg(scale + i0 + e) : 0.0;
+                    S[row * kXLd + e] = sc * (vm != 0.0 ? fma(u, vm, v[e]) : v[e]);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+                S[row * kXLd + e] = (i0 + e < n ? __ldg(scale + i0 + e) : 0.0) * v[e];
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        // row by row: 32 consecutive eigenvectors of one SNP per warp store
+#pragma unroll 4
+        for (int s = 0; s < kRows / 4; ++s) {
+            const int rr = q * (kRows / 4) + s;
+            const int64_t j = (int64_t)mb * kRows + rr;
+            if (j < m && i0 + lane < n) X[j * ldx + i0 + lane] = S[rr * kXLd + lane];
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");  // the next tile rewrites S
+    }
+};
+
+cudaError_t rotate_f64_pipeline_test_mode(int skip_loads, unsigned long long wait_limit_ns) {
+    return pipeline_test_mode(skip_loads, wait_limit_ns);
+}
+
+namespace {
+struct XPlanes {
+    int64_t lda, rows, a_off, s_off, total;
+};
+XPlanes xplanes(int64_t n) {
+    XPlanes L;
+    L.lda = (n + 127) / 128 * 128;
+    L.rows = ceil_div(n, 32) * kXBN;
+    L.a_off = 0;
+    L.s_off = ((L.rows * L.lda + 255) / 256) * 256;
+    L.total = L.s_off + ((n * 8 + 255) / 256) * 256;
+    return L;
+}
+// Chunk scratch: status and found words, one tile list per form, the packed A operand.
+struct XChunk {
+    int64_t status, found, tiles, tiles2, a_off, lda, total;
+};
+XChunk xchunk(int64_t n, int64_t m) {
+    XChunk L;
+    const int64_t NB = ceil_div(n, 32), MB = ceil_div(m, 64);
+    auto a256 = [](int64_t x) { return (x + 255) / 256 * 256; };
+    L.lda = (n + 127) / 128 * 128;
+    L.status = 0;
+    L.found = 128;
+    L.tiles = 256;
+    L.tiles2 = L.tiles + a256(MB * NB * (int64_t)sizeof(Tile));
+    L.a_off = L.tiles2 + a256(ceil_div(m, 128) * NB * (int64_t)sizeof(Tile));
+    L.total = L.a_off + MB * 128 * L.lda;
+    return L;
+}
+
+// Tile groups: 16 SNP blocks x 9 eigenvector blocks are about one wave of CTAs, whose
+// operand slices are then shared in L2.
+constexpr int kXGroupM = 16, kXGroupN = 9;
+
+template <bool PAIRED>
+int32_t launch_x(const int8_t* A, int64_t a_rows, int64_t lda, const int8_t* digits,
+                 const XPlanes& P, const double* scale, int64_t n, int64_t m, const double* mean,
+                 double* X, int64_t ldx, Tile* tiles, int* status, const int* gate, int gate_value,
+                 cudaStream_t st) {
+    const int MB = (int)ceil_div(m, PAIRED ? 64 : 128), NB = (int)ceil_div(n, 32);
+    CUtensorMap ta, tb;
+    int32_t rc = make_map_i8(&ta, A, a_rows, n, lda, kBM);
+    if (rc) return rc;
+    rc = make_map_i8(&tb, digits, P.rows, n, P.lda, kXBN);
+    if (rc) return rc;
+    rc = launch_group_tiles(MB, NB, kXGroupM, kXGroupN, tiles, st);
+    if (rc) return rc;
+    auto kern = i8_gemm_kernel<kXBN, kXStages, XEpi<PAIRED>>;
+    JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XSmem::TOTAL));
+    const int64_t n_tiles = (int64_t)MB * NB;
+    XEpi<PAIRED> epi{X, ldx, scale, mean, (int)n, (int)m};
+    kern<<<(unsigned)(n_tiles < num_sms() ? n_tiles : num_sms()), kThreads, XSmem::TOTAL, st>>>(
+        ta, tb, tiles, (int)n_tiles, (int)ceil_div(n, kBK), epi, status, gate, gate_value);
+    JB_LAUNCH_CHECK("i8_gemm_kernel<rotate f64>");
+    return JB_OK;
+}
+}  // namespace
+
+}  // namespace tc
+}  // namespace jb
+
+using namespace jb;
+using namespace jb::tc;
+
+extern "C" {
+
+int64_t jb_split_f64_workspace_size(int64_t n) {
+    if (n <= 0) return -1;
+    return xplanes(n).total;
+}
+
+int32_t jb_split_f64_prepare(const double* U, int64_t n, int64_t ldu, void* planes,
+                             int64_t planes_bytes, uintptr_t stream) {
+    JB_CHECK_ARG(n > 0 && ldu >= n && U, "jb_split_f64_prepare: bad arguments");
+    JB_CHECK_ARG(n < (1ll << 23), "jb_split_f64_prepare: n too large for exact int32 digit sums");
+    const XPlanes P = xplanes(n);
+    JB_CHECK_ARG(planes && planes_bytes >= P.total, "jb_split_f64_prepare: workspace too small");
+    uint8_t* ws = static_cast<uint8_t*>(planes);
+    cudaStream_t st = as_stream(stream);
+    if (n % 32) {  // digit rows of the last block past the last eigenvector
+        const int64_t first = (P.rows - kXBN) * P.lda;
+        JB_CUDA(cudaMemsetAsync(ws + P.a_off + first, 0, (size_t)(kXBN * P.lda), st));
+    }
+    xsplit_kernel<<<(unsigned)n, 256, 0, st>>>(U, n, ldu, reinterpret_cast<int8_t*>(ws + P.a_off), P.lda,
+                                               reinterpret_cast<double*>(ws + P.s_off));
+    JB_LAUNCH_CHECK("xsplit_kernel");
+    return JB_OK;
+}
+
+int64_t jb_rotate_codes_f64_workspace_size(int64_t n, int64_t m) {
+    if (n <= 0 || m <= 0) return -1;
+    return xchunk(n, m).total;
+}
+
+int32_t jb_rotate_codes_f64(const void* planes, int64_t n, const int8_t* codes, int64_t ld_codes,
+                            int64_t m, const double* mean, int32_t has_missing, double* X,
+                            int64_t ldx, void* workspace, int64_t workspace_bytes,
+                            uintptr_t stream) {
+    JB_CHECK_ARG(n > 0 && m >= 0 && ld_codes >= n && ldx >= n, "jb_rotate_codes_f64: bad shape");
+    JB_CHECK_ARG(n < (1ll << 23) && m < (1ll << 31), "jb_rotate_codes_f64: size too large");
+    if (m == 0) return JB_OK;
+    JB_CHECK_ARG(planes && codes && X && mean, "jb_rotate_codes_f64: null pointer");
+    const XChunk L = xchunk(n, m);
+    JB_CHECK_ARG(workspace && workspace_bytes >= L.total, "jb_rotate_codes_f64: workspace too small");
+    JB_CHECK_ARG(ceil_div(m, 64) * ceil_div(n, 32) < (1ll << 31), "jb_rotate_codes_f64: size too large");
+    const XPlanes P = xplanes(n);
+    const uint8_t* pw = static_cast<const uint8_t*>(planes);
+    const int8_t* digits = reinterpret_cast<const int8_t*>(pw + P.a_off);
+    const double* scale = reinterpret_cast<const double*>(pw + P.s_off);
+    uint8_t* ws = static_cast<uint8_t*>(workspace);
+    int* status = reinterpret_cast<int*>(ws + L.status);
+    int* found = reinterpret_cast<int*>(ws + L.found);
+    int8_t* A = reinterpret_cast<int8_t*>(ws + L.a_off);
+    cudaStream_t st = as_stream(stream);
+    JB_CUDA(cudaMemsetAsync(ws, 0, 256, st));  // status and found
+    const int* gate = nullptr;
+    // without missing calls the codes are the A operand themselves (if TMA can read them);
+    // should one be missing after all, the launches after it run instead
+    if (!has_missing && ld_codes % 16 == 0 && (reinterpret_cast<uintptr_t>(codes) & 15) == 0) {
+        gate = found;
+        xfind_missing_kernel<<<(unsigned)(m < 4 * num_sms() ? m : 4 * num_sms()), 256, 0, st>>>(
+            codes, ld_codes, n, m, found);
+        JB_LAUNCH_CHECK("xfind_missing_kernel");
+        const int32_t rc = launch_x<false>(codes, m, ld_codes, digits, P, scale, n, m, nullptr, X, ldx,
+                                           reinterpret_cast<Tile*>(ws + L.tiles2), status, gate, 0, st);
+        if (rc) return rc;
+    }
+    xpack_kernel<<<(unsigned)(ceil_div(m, 64) * 64), 256, 0, st>>>(codes, ld_codes, n, m, A, L.lda, gate);
+    JB_LAUNCH_CHECK("xpack_kernel");
+    return launch_x<true>(A, ceil_div(m, 64) * 128, L.lda, digits, P, scale, n, m, mean, X, ldx,
+                          reinterpret_cast<Tile*>(ws + L.tiles), status, gate, 1, st);
+}
+
+}  // extern "C"

@@ -316,13 +316,13 @@ int32_t rotate_i8_gemm(const uint8_t* ozaki_ws, int64_t n_out, int64_t n_k, cons
         JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      RotSmem::TOTAL));
         RotEpi<true> epi{X, ldx, smax, mean, (int)n_out, (int)m};
-        kern<<<grid, kThreads, RotSmem::TOTAL, st>>>(ta, tb, tiles, n_tiles, num_kb, epi, status);
+        kern<<<grid, kThreads, RotSmem::TOTAL, st>>>(ta, tb, tiles, n_tiles, num_kb, epi, status, nullptr, 0);
     } else {
         auto kern = i8_gemm_kernel<kRotBN, kRotStages, RotEpi<false>>;
         JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      RotSmem::TOTAL));
         RotEpi<false> epi{X, ldx, smax, nullptr, (int)n_out, (int)m};
-        kern<<<grid, kThreads, RotSmem::TOTAL, st>>>(ta, tb, tiles, n_tiles, num_kb, epi, status);
+        kern<<<grid, kThreads, RotSmem::TOTAL, st>>>(ta, tb, tiles, n_tiles, num_kb, epi, status, nullptr, 0);
     }
     JB_LAUNCH_CHECK("i8_gemm_kernel<rotate>");
     return JB_OK;

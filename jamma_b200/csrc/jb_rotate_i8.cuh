@@ -39,6 +39,7 @@ int32_t rotate_i8_gemm(const uint8_t* ozaki_ws, int64_t n_out, int64_t n_k, cons
 // Test hooks of the rotation kernels' bounded waits (this translation unit's copy of the
 // GEMM core's hooks; see jb_test_pipeline_timeout).
 cudaError_t rotate_pipeline_test_mode(int skip_loads, unsigned long long wait_limit_ns);
+cudaError_t rotate_f64_pipeline_test_mode(int skip_loads, unsigned long long wait_limit_ns);
 
 }  // namespace tc
 }  // namespace jb

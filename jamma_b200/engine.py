@@ -35,6 +35,9 @@ MAX_CVT = 4
 NULL_L_MIN, NULL_L_MAX, NULL_N_GRID, NULL_N_ITER = 1e-5, 1e5, 50, 20
 # log-lambda domain of the mixed form's series tables (jb_lmm_prepare precision 1)
 SERIES_L_MIN, SERIES_L_MAX = 1e-5, 1e5
+# The FP64 form rotates calls from seven INT8 digit planes (7 n^2 bytes beside U's 8 n^2) up to
+# this many samples
+EXACT_MAX_SAMPLES = 65536
 # The FP64 form's guided search: fewest grid points at which the degree-24 bracket expansions
 # truncate below 1e-15, and fewest samples at which it is the faster one (4000 SNPs x 2
 # phenotypes, every test, direct -> guided: n = 300 1.4 -> 2.5 ms, n = 500 1.9 -> 0.7 ms)
@@ -72,6 +75,15 @@ def ozaki_split(U: torch.Tensor) -> torch.Tensor:
     return oz
 
 
+def exact_split(U: torch.Tensor) -> torch.Tensor:
+    """Seven exact INT8 digit planes of column-major eigenvectors U (n, n) for the FP64
+    rotation of genotype calls."""
+    n = U.shape[0]
+    planes = workspace(_native.load().jb_split_f64_workspace_size(n))
+    _native.call("jb_split_f64_prepare", ptr(U), n, n, ptr(planes), planes.numel(), stream_handle())
+    return planes
+
+
 class DeviceCohort:
     """One cohort's resident state for association testing.
 
@@ -82,6 +94,8 @@ class DeviceCohort:
         covariates: (n, c) host matrix W (c in 1..4), or None for an intercept.
         phenotypes: (n,) or (n, phi) host phenotypes (already restricted to analysed
             samples; every phenotype shares the sample set).
+        ozaki: digit planes of the eigenvectors shared with other users of the cohort
+            (:func:`ozaki_split` for "mixed", :func:`exact_split` for "fp64").
     """
 
     def __init__(self, eigenvalues, eigenvectors, covariates, phenotypes, lmm_mode=1,
@@ -127,13 +141,16 @@ class DeviceCohort:
             _native.call("jb_null_mle", n, c, phi, ptr(self.evals), ptr(self.UtW), n, ptr(self.Uty),
                          n, NULL_L_MIN, NULL_L_MAX, NULL_N_GRID, NULL_N_ITER, ptr(self.lam0),
                          ptr(self.logl0), st)
+        # digit planes of U for the rotation of calls: four in the mixed form, seven exact
+        # ones in the FP64 form (where U^T G is a GEMM without them)
         self.ozaki = None
         if precision == "mixed":
-            if ozaki is not None:  # digit planes shared with other users of the same cohort
-                self.ozaki = ozaki
-            else:
-                self.ozaki = ozaki_split(self.U)
-        self.code_ld = (n + 127) // 128 * 128 if precision == "mixed" else n
+            self.ozaki = ozaki if ozaki is not None else ozaki_split(self.U)
+        elif n <= EXACT_MAX_SAMPLES:
+            shared = (ozaki is not None
+                      and ozaki.numel() == _native.load().jb_split_f64_workspace_size(n))
+            self.ozaki = ozaki if shared else exact_split(self.U)
+        self.code_ld = (n + 127) // 128 * 128 if self.ozaki is not None else n
         self._rot_ws = None
         self._chunk_ws = None
         # The interpolated search expands 1/(lambda*eval + 1) in log lambda over the fixed
@@ -229,6 +246,19 @@ class DeviceCohort:
             self._series_for = (m, out.data_ptr())
         return out
 
+    def rotate_codes_f64(self, codes: torch.Tensor, means: torch.Tensor, has_missing: bool = True,
+                         out: torch.Tensor | None = None) -> torch.Tensor:
+        """FP64 form: U^T G (m, n) of decoded codes from the exact digit planes."""
+        m, ld = codes.shape
+        need = _native.load().jb_rotate_codes_f64_workspace_size(self.n, m)
+        if self._rot_ws is None or self._rot_ws.numel() < need:
+            self._rot_ws = workspace(need)
+        out = out if out is not None else empty((m, self.n))
+        _native.call("jb_rotate_codes_f64", ptr(self.ozaki), self.n, ptr(codes), ld, m, ptr(means),
+                     int(bool(has_missing)), ptr(out), self.n, ptr(self._rot_ws),
+                     self._rot_ws.numel(), stream_handle())
+        return out
+
     def rotate_status(self) -> int:
         st = np.zeros(1, dtype=np.int32)
         if self._rot_ws is not None:
@@ -240,18 +270,18 @@ class DeviceCohort:
         """Decoded int8 codes (m, ld) + per-SNP imputation means (m,) -> statistics."""
         m, ld = codes.shape
         bufs = bufs if bufs is not None else {}
+        UtG = bufs.get("UtG")
+        UtG = UtG[:m] if UtG is not None and UtG.shape[0] >= m else None
         if self.precision == "mixed":
-            UtG = bufs.get("UtG")
-            UtG = UtG[:m] if UtG is not None and UtG.shape[0] >= m else None
             return self.associate_rotated(self.rotate_codes_i8(codes, means, has_missing, UtG), out)
+        if self.ozaki is not None:
+            return self.associate_rotated(self.rotate_codes_f64(codes, means, has_missing, UtG), out)
         G = bufs.get("G")
         if G is None or G.shape[0] < m:
             G = empty((m, self.n))
         G = G[:m]
         _native.call("jb_impute_f64", ptr(codes), ld, self.n, m, ptr(means), ptr(G), self.n,
                      stream_handle())
-        UtG = bufs.get("UtG")
-        UtG = UtG[:m] if UtG is not None and UtG.shape[0] >= m else None
         return self.associate_genotypes(G, out, UtG)
 
 
@@ -291,7 +321,7 @@ class ChunkGraph:
         self.counts = torch.zeros((m, 4), dtype=torch.int32, device="cuda")
         self.out = cohort.alloc_out(m)
         self.bufs = {"UtG": empty((m, n))}
-        if cohort.precision != "mixed":
+        if cohort.ozaki is None:
             self.bufs["G"] = empty((m, n))
         caller = torch.cuda.current_stream()
         side = torch.cuda.Stream()

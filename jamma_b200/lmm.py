@@ -220,7 +220,7 @@ def associate_records(cohort: eng.DeviceCohort, records, n_file: int, sample_idx
         collect(*pending)
         pending = (b, s, e)
     collect(*pending)
-    if cohort.precision == "mixed" and (status := cohort.rotate_status()):
+    if status := cohort.rotate_status():  # 0 where the rotation was a GEMM
         raise RuntimeError(f"INT8 rotation pipeline reported status {status} (a bounded "
                            "tensor-core pipeline wait ran out)")
     return res

@@ -93,7 +93,7 @@ def _eigh_workspace_bytes(n: int) -> int:
 
 
 def job_device_bytes(n: int, phi: int, n_cvt: int, chunk: int, resident: bool,
-                     n_snps: int = 0) -> int:
+                     n_snps: int = 0, precision: str = "mixed") -> int:
     """Device bytes a job holds while it runs (cohort state counted when not resident).
 
     A job that builds its cohort also needs, at the peak of its set-up, the largest of the
@@ -103,14 +103,17 @@ def job_device_bytes(n: int, phi: int, n_cvt: int, chunk: int, resident: bool,
     lib = _native.load()
     b = lib.jb_lmm_workspace_size(n, n_cvt, phi, 50) + lib.jb_lmm_chunk_workspace_size(
         n, n_cvt, phi, 50, chunk)
-    b += lib.jb_rotate_i8_workspace_size(n, chunk) + chunk * n * 8 + chunk * ((n + 127) // 128 * 128)
+    exact = precision == "fp64" and n <= eng.EXACT_MAX_SAMPLES
+    rot_ws = lib.jb_rotate_codes_f64_workspace_size if exact else lib.jb_rotate_i8_workspace_size
+    b += rot_ws(n, chunk) + chunk * n * 8 + chunk * ((n + 127) // 128 * 128)
     b += 9 * phi * chunk * 8 + 2 * n * (n_cvt + phi) * 8
     b += lib.jb_lmm_series_workspace_size(n, n_cvt, phi)
     if not resident:
         nn = n * n
         build = max(n * ((n_snps + 127) // 128 * 128) + 12 * nn, 20 * nn,
                     8 * nn + _eigh_workspace_bytes(n))
-        b += build + lib.jb_ozaki_workspace_size(n) + n * 8
+        planes = lib.jb_split_f64_workspace_size if exact else lib.jb_ozaki_workspace_size
+        b += build + planes(n) + n * 8
     return int(b)
 
 
@@ -215,7 +218,8 @@ class GwasServer:
             with self._lock:
                 known = job.cohort_id in self.cohorts or job.cohort_id in self._building
                 need = job_device_bytes(job.n_samples, phi, c, self.chunk, known,
-                                        n_snps=int(np.shape(job.packed)[0]))
+                                        n_snps=int(np.shape(job.packed)[0]),
+                                        precision=self.precision)
                 self._evict_for(need)
                 if self.used + self._resident_bytes() + need > self.budget:
                     if not self.active and not self.preparing:
@@ -275,7 +279,10 @@ class GwasServer:
             del acc
             with self._device_sync_lock:  # the large-n solver synchronises the device
                 evals, U = eng.eigh_device(K)
-            oz = eng.ozaki_split(U) if self.precision == "mixed" else None
+            if self.precision == "mixed":
+                oz = eng.ozaki_split(U)
+            else:
+                oz = eng.exact_split(U) if n <= eng.EXACT_MAX_SAMPLES else None
             torch.cuda.current_stream().synchronize()  # resident state complete for other streams
             return _Resident(evals, U, oz)
 
