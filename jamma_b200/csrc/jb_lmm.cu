@@ -1449,15 +1449,43 @@ int32_t launch_sq_sums(const double* AT, int64_t rows, const double* X, int64_t 
     return JB_OK;
 }
 
+// Lanes per pair of the series search: the most with which all pairs are resident at once (2
+// CTAs per SM), where the chain of steps of one pair sets the time; beyond one wave the
+// fewest, which do the least work.  Measured, every test, one covariate column, 16 / 8 / 4
+// lanes: 1000 pairs 76 / 80 / 105 us, 4000 pairs 144 / 87 / 108 us, 8192 pairs 259 / 158 /
+// 118 us; two columns, 16 / 8 lanes: 2000 pairs 91 / 101 us, 8192 pairs 298 / 204 us.
+inline int search_lanes(int64_t pairs, int c) {
+    const int64_t threads = (int64_t)2 * tc::num_sms() * kSearchThreads;
+    if (pairs * 16 <= threads) return 16;
+    return c > 1 || pairs * 8 <= threads ? 8 : 4;
+}
+
+template <int C, int LP, bool GUIDE>
+void launch_search_as(const Params& p, cudaStream_t st) {
+    const int64_t threads = p.m * p.phi * LP;
+    lmm_search_kernel<C, LP, GUIDE>
+        <<<(unsigned)ceil_div(threads, kSearchThreads), kSearchThreads, 0, st>>>(p);
+}
+
+template <int C, bool GUIDE>
+void launch_search(const Params& p, cudaStream_t st) {
+    const int lanes = search_lanes(p.m * p.phi, C);
+    if (lanes == 16)
+        launch_search_as<C, 16, GUIDE>(p, st);
+    else if (C == 1 && lanes == 4)
+        launch_search_as<C, C == 1 ? 4 : 8, GUIDE>(p, st);
+    else
+        launch_search_as<C, 8, GUIDE>(p, st);
+}
+
 template <int C>
 int32_t launch_pairs(const Params& p, cudaStream_t st) {
     const int64_t pairs = p.m * p.phi;
-    const unsigned groups = (unsigned)ceil_div(pairs * Search<C>::LP, Search<C>::kThreads);
     const unsigned warps = (unsigned)ceil_div(pairs * 32, kPairsThreads);
     if (p.state) {
         if (p.mode != 3) {
             JB_CUDA(cudaMemsetAsync(p.open_count, 0, sizeof(*p.open_count), st));
-            lmm_search_kernel<C, true><<<groups, Search<C>::kThreads, 0, st>>>(p);
+            launch_search<C, true>(p, st);
             JB_LAUNCH_CHECK("lmm_search_kernel");
             const int64_t sms = tc::num_sms();
             lmm_open_kernel<C><<<(unsigned)(2 * pairs < sms ? 2 * pairs : sms), kOpenThreads, 0, st>>>(
@@ -1472,7 +1500,7 @@ int32_t launch_pairs(const Params& p, cudaStream_t st) {
         }
         lmm_finish_kernel<C><<<warps, kPairsThreads, 0, st>>>(p);
     } else if (p.cheb) {
-        lmm_search_kernel<C, false><<<groups, Search<C>::kThreads, 0, st>>>(p);
+        launch_search<C, false>(p, st);
     } else {
         lmm_pairs_kernel<C><<<warps, kPairsThreads, 0, st>>>(p);
     }

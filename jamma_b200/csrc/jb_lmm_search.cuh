@@ -8,8 +8,10 @@
 // same order of every sum whatever LP is, so the group size only trades registers against
 // repeated work: the coefficients of a pair take 3 (C + 2) 32 / LP doubles of each lane, and
 // the per-probe scalar work (Pab recursion, golden-section steps) is repeated by every lane.
-//   * LP = 4 for one covariate column (72 coefficient doubles, 8 pairs per warp), LP = 8 for
-//     two to four (48 to 72 doubles, 4 pairs per warp);
+//   * LP = 4 for one covariate column (72 coefficient doubles, 8 pairs per warp) and 8 for
+//     two to four (48 to 72 doubles, 4 pairs per warp) do the least work per pair; LP = 16
+//     (12 to 36 doubles) has the shortest chain of steps per pair, for chunks whose pairs
+//     cannot fill the GPU otherwise (search_lanes);
 //   * offsets of the butterfly that stay within a lane need no shuffle;
 //   * the logarithms of one likelihood are taken by different lanes of the group;
 //   * grid points are shared out one per lane after their sums, so that their Pab recursions
@@ -25,13 +27,7 @@
 namespace jb {
 namespace lmm {
 
-template <int C>
-struct Search {
-    static constexpr int LP = C == 1 ? 4 : 8;  // lanes per pair
-    static constexpr int V = 32 / LP;          // virtual lanes per lane
-    static constexpr int kThreads = 128;
-    static constexpr int kMinBlocks = 2;       // up to 255 registers
-};
+constexpr int kSearchThreads = 128;  // 2 CTAs per SM: up to 255 registers
 
 // Chebyshev values of a group: t[v] = T_{r + LP v}(x), m[v] = T_{LP - r + LP v}(x) (r the
 // lane within the group), by the doubling identity T_{a+b} = 2 T_a T_b - T_{a-b} with a the
@@ -40,25 +36,23 @@ template <int LP>
 __device__ __forceinline__ double cheb_group(double x, int r, double (&t)[32 / LP],
                                              double (&m)[32 / LP]) {
     constexpr int V = 32 / LP;
-    static_assert(LP == 4 || LP == 8, "group of 4 or 8 lanes");
+    static_assert(LP == 4 || LP == 8 || LP == 16, "group of 4, 8 or 16 lanes");
     const double t2 = fma(2.0 * x, x, -1.0);
     const double t3 = fma(2.0 * t2, x, -x);
-    const double t4 = fma(2.0 * t2, t2, -1.0);
+    double ta = fma(2.0 * t2, t2, -1.0);  // T_4
     const int q = r & 3;
-    const double lo = q == 0 ? 1.0 : (q == 1 ? x : (q == 2 ? t2 : t3));  // T_q
-    const double hi = q == 0 ? t4 : (q == 1 ? t3 : (q == 2 ? t2 : x));   // T_{4-q}
-    double ta;
-    if (LP == 4) {
-        t[0] = lo;
-        m[0] = hi;
-        ta = t4;
-    } else {
-        const bool up = r >= 4;
-        const double v = fma(2.0 * t4, up ? lo : hi, -(up ? hi : lo));
-        t[0] = up ? v : lo;
-        m[0] = up ? hi : v;
-        ta = fma(2.0 * t4, t4, -1.0);
+    double lo = q == 0 ? 1.0 : (q == 1 ? x : (q == 2 ? t2 : t3));  // T_q
+    double hi = q == 0 ? ta : (q == 1 ? t3 : (q == 2 ? t2 : x));   // T_{4-q}
+#pragma unroll
+    for (int a = 4; a < LP; a *= 2) {  // lo = T_{r mod 2a}, hi = T_{2a - r mod 2a}
+        const bool up = (r & a) != 0;
+        const double v = fma(2.0 * ta, up ? lo : hi, -(up ? hi : lo));
+        lo = up ? v : lo;
+        hi = up ? hi : v;
+        ta = fma(2.0 * ta, ta, -1.0);
     }
+    t[0] = lo;
+    m[0] = hi;
 #pragma unroll
     for (int a = 1; a < V; a *= 2) {
         const double two = 2.0 * ta;
@@ -87,17 +81,16 @@ __device__ __forceinline__ double group_sum(double (&p)[32 / LP]) {
 }
 
 // Coefficients of the global x-sum series held by a lane, loaded once per pair.
-template <int C>
+template <int C, int LP>
 struct PairCoef {
-    double c[Lay<C>::NX][Search<C>::V][kCoefPerLane];
+    double c[Lay<C>::NX][32 / LP][kCoefPerLane];
 };
-template <int C>
+template <int C, int LP>
 __device__ __forceinline__ void load_pair_coef(const Params& p, int64_t j, int f, int r,
-                                               PairCoef<C>& g) {
-    constexpr int LP = Search<C>::LP;
+                                               PairCoef<C, LP>& g) {
     const int64_t cp = C + p.phi;
 #pragma unroll
-    for (int v = 0; v < Search<C>::V; ++v) {
+    for (int v = 0; v < 32 / LP; ++v) {
 #pragma unroll
         for (int i = 0; i < kCoefPerLane; ++i) {
             const int64_t row = 1 + r + LP * v + 32 * i;
@@ -111,10 +104,10 @@ __device__ __forceinline__ void load_pair_coef(const Params& p, int64_t j, int f
 }
 
 // The c+2 x-dependent sums at log-lambda s; identical bits in every lane of the group.
-template <int C>
-__device__ __forceinline__ void series_xsums(const Params& p, const PairCoef<C>& g, double s, int r,
-                                             double (&xs)[Lay<C>::NX]) {
-    constexpr int LP = Search<C>::LP, V = Search<C>::V;
+template <int C, int LP>
+__device__ __forceinline__ void series_xsums(const Params& p, const PairCoef<C, LP>& g, double s,
+                                             int r, double (&xs)[Lay<C>::NX]) {
+    constexpr int V = 32 / LP;
     double t[V], m[V];
     const double t32 = cheb_group<LP>((s - p.gmid) * p.ginv, r, t, m);
     const double two = 2.0 * t32;
@@ -135,10 +128,10 @@ __device__ __forceinline__ void series_xsums(const Params& p, const PairCoef<C>&
 }
 
 // The same sums at grid point k, its Chebyshev values from the table p.tgrid.
-template <int C>
-__device__ __forceinline__ void grid_xsums(const Params& p, const PairCoef<C>& g, int k, int r,
+template <int C, int LP>
+__device__ __forceinline__ void grid_xsums(const Params& p, const PairCoef<C, LP>& g, int k, int r,
                                            double (&xs)[Lay<C>::NX]) {
-    constexpr int LP = Search<C>::LP, V = Search<C>::V;
+    constexpr int V = 32 / LP;
     const double* __restrict__ tg = p.tgrid + (int64_t)k * kChebG + r;
     double w[Lay<C>::NX][V];
 #pragma unroll
@@ -153,36 +146,58 @@ __device__ __forceinline__ void grid_xsums(const Params& p, const PairCoef<C>& g
 }
 
 // log|H^-1| and the x-free sums of phenotype f at log-lambda s, from the expansions over the
-// golden bracket of grid index `best` (degree 24, coefficients in virtual lanes 0..24).
-template <int C>
-__device__ __forceinline__ void bracket_sums(const Params& p, int best, int f, double s, int r,
-                                             double& logdet, double (&shared)[Lay<C>::NS]) {
-    using L = Lay<C>;
-    constexpr int LP = Search<C>::LP, V = Search<C>::V;
-    const double* __restrict__ cb =
-        p.cheb + (int64_t)best * (1 + (int64_t)p.phi * L::NS) * kChebN + r;
-    double t[V], m[V];
-    cheb_group<LP>((s - __ldg(p.cheb_mid + best)) * (1.0 / __ldg(p.cheb_half + best)), r, t, m);
-#pragma unroll
-    for (int k = -1; k < L::NS; ++k) {
-        const double* __restrict__ ck = cb + (k < 0 ? 0 : (int64_t)(1 + f * L::NS + k) * kChebN);
-        double w[V];
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const bool in = LP * v + LP <= kChebN || r + LP * v < kChebN;
-            w[v] = LP * v < kChebN && in ? __dmul_rn(__ldg(ck + LP * v), t[v]) : 0.0;
-        }
-        const double v = group_sum<LP>(w);
-        if (k < 0)
-            logdet = v;
-        else
-            shared[k] = v;
+// golden bracket of grid index `best` (degree 24, coefficients in virtual lanes 0..24).  With
+// 16 lanes a pair's coefficients stay in registers; fewer lanes have none left and read them
+// (through L1) at every probe.
+template <int C, int LP>
+struct Bracket {
+    static constexpr int V = 32 / LP;
+    static constexpr bool kHold = LP == 16;
+    double mid, inv_half;
+    const double* __restrict__ cb;  // of this lane
+    double c[kHold ? 1 + Lay<C>::NS : 1][V];
+    __device__ __forceinline__ double coef(const Params& p, int f, int k, int v, int r) const {
+        const bool in = LP * v + LP <= kChebN || r + LP * v < kChebN;
+        const double* __restrict__ ck = cb + (k < 0 ? 0 : (int64_t)(1 + f * Lay<C>::NS + k) * kChebN);
+        return LP * v < kChebN && in ? __ldg(ck + LP * v) : 0.0;
     }
-}
+    __device__ __forceinline__ void load(const Params& p, int best, int f, int r) {
+        cb = p.cheb + (int64_t)best * (1 + (int64_t)p.phi * Lay<C>::NS) * kChebN + r;
+        mid = __ldg(p.cheb_mid + best);
+        inv_half = 1.0 / __ldg(p.cheb_half + best);
+        if constexpr (kHold) {
+#pragma unroll
+            for (int k = -1; k < Lay<C>::NS; ++k)
+#pragma unroll
+                for (int v = 0; v < V; ++v) c[1 + k][v] = coef(p, f, k, v, r);
+        }
+    }
+    __device__ __forceinline__ void sums(const Params& p, int f, double s, int r, double& logdet,
+                                         double (&shared)[Lay<C>::NS]) const {
+        double t[V], m[V];
+        cheb_group<LP>((s - mid) * inv_half, r, t, m);
+#pragma unroll
+        for (int k = -1; k < Lay<C>::NS; ++k) {
+            double w[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                if constexpr (kHold)
+                    w[v] = __dmul_rn(c[1 + k][v], t[v]);
+                else
+                    w[v] = __dmul_rn(coef(p, f, k, v, r), t[v]);
+            }
+            const double v = group_sum<LP>(w);
+            if (k < 0)
+                logdet = v;
+            else
+                shared[k] = v;
+        }
+    }
+};
 
 // REML and MLE log-likelihoods of one Pab result with the logarithms shared out: lane i <= C
 // takes log of pivot i, lane C + 1 the one of P_yy; the sums are those of reml_logl / mle_logl.
-template <int C>
+template <int C, int LP>
 __device__ __forceinline__ double group_reml(const PabOut<C>& pb, const double (&log_iab)[C + 1],
                                              double logdet_h, const Params& p, int r) {
     const double pyy = clamp_pyy(pb.yy1);
@@ -194,10 +209,10 @@ __device__ __forceinline__ double group_reml(const PabOut<C>& pb, const double (
     double ldw = 0.0;
 #pragma unroll
     for (int i = 0; i <= C; ++i) {
-        ldw = __dadd_rn(ldw, __shfl_sync(kFull, lg, i, Search<C>::LP));
+        ldw = __dadd_rn(ldw, __shfl_sync(kFull, lg, i, LP));
         ldw = __dsub_rn(ldw, log_iab[i]);
     }
-    const double lpyy = __shfl_sync(kFull, lg, C + 1, Search<C>::LP);
+    const double lpyy = __shfl_sync(kFull, lg, C + 1, LP);
     double f = __dsub_rn(p.c_reml, __dmul_rn(0.5, logdet_h));
     f = __dsub_rn(f, __dmul_rn(0.5, ldw));
     return __dsub_rn(f, __dmul_rn(__dmul_rn(0.5, p.df), lpyy));
@@ -314,14 +329,14 @@ struct Golden {
 // of `whole` (one rounding against ~1e-13) and the direct sums' own, a few ulp of a value of
 // size 1.4 n.  Anything not finite, or a bound that no longer tells golden steps apart, makes
 // the pair's search direct from the grid on.
-template <int C>
-__device__ __forceinline__ GuideTau guide_tau(const Params& p, const PairCoef<C>& g, int best,
+template <int C, int LP>
+__device__ __forceinline__ GuideTau guide_tau(const Params& p, const PairCoef<C, LP>& g, int best,
                                               int f, int r) {
     using L = Lay<C>;
     const int64_t srow = (int64_t)p.phi * L::NS;
     const double* s0 = p.S + (int64_t)best * srow + (int64_t)f * L::NS;
     double xs[L::NX], row0[L::NI];
-    grid_xsums<C>(p, g, best, r, xs);
+    grid_xsums<C, LP>(p, g, best, r, xs);
     assemble<C>(row0, s0, xs);
     const PabOut<C> pb = pab_reduce<C>(row0);
     const double A = p.S[(int64_t)p.n_grid * srow + (int64_t)f * L::NS] / s0[0];
@@ -375,11 +390,9 @@ struct ArgMaxLead {
 // GUIDE = false: the mixed form, search and statistics.  GUIDE = true: the plain form's
 // decisions, as far as they are certain (modes 1, 2 and 4); lmm_open_kernel and
 // lmm_finish_kernel take over.
-template <int C, bool GUIDE>
-__global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
-    lmm_search_kernel(const Params p) {
+template <int C, int LP, bool GUIDE>
+__global__ void __launch_bounds__(kSearchThreads, 2) lmm_search_kernel(const Params p) {
     using L = Lay<C>;
-    constexpr int LP = Search<C>::LP;
     const int64_t npairs = p.m * p.phi;
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if ((tid & ~31ll) / LP >= npairs) return;  // the whole warp is idle
@@ -396,8 +409,8 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
     const int64_t srow = (int64_t)p.phi * L::NS;  // stride of one S row
     const bool writer = r == 0 && valid_pair;
 
-    PairCoef<C> g;
-    load_pair_coef<C>(p, j, f, r, g);
+    PairCoef<C, LP> g;
+    load_pair_coef<C, LP>(p, j, f, r, g);
 
     // ---------------- H = 1 (Iab) and H = H0 (score)
     double log_iab[C + 1];
@@ -417,7 +430,7 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
     }
     if (need_score) {
         double xs[L::NX], row0[L::NI];
-        series_xsums<C>(p, g, log(p.lam0[f]), r, xs);
+        series_xsums<C, LP>(p, g, log(p.lam0[f]), r, xs);
         assemble<C>(row0, p.S + (int64_t)(p.n_grid + 1 + f) * srow + (int64_t)f * L::NS, xs);
         const PabOut<C> pb = pab_reduce<C>(row0);
         bool valid;
@@ -447,7 +460,7 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
 #pragma unroll 1
         for (int e = 0; e < LP; ++e) {
             double xe[L::NX];
-            grid_xsums<C>(p, g, g0 + e < p.n_grid ? g0 + e : p.n_grid - 1, r, xe);
+            grid_xsums<C, LP>(p, g, g0 + e < p.n_grid ? g0 + e : p.n_grid - 1, r, xe);
 #pragma unroll
             for (int q = 0; q < L::NX; ++q) xs[q] = e == r || e == 0 ? xe[q] : xs[q];
         }
@@ -470,6 +483,9 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
     Golden<GUIDE> gm, gr;
     gm.start(p, bm);
     gr.start(p, br);
+    Bracket<C, LP> km, kr;
+    km.load(p, bm, f, r);
+    kr.load(p, br, f, r);
     SearchReport out_m, out_r;
     if constexpr (GUIDE) {
         if (writer) {
@@ -478,7 +494,7 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
         }
         // the grid's decision: its values are as certain as the probes'
         auto settle = [&](Golden<GUIDE>& gs, const ArgMaxLead& best, int at, const SearchReport& out) {
-            gs.tau = guide_tau<C>(p, g, at, f, r);
+            gs.tau = guide_tau<C, LP>(p, g, at, f, r);
             gs.certain = !best.nan && best.v - best.v2 > 4.0 * (gs.tau.whole + gs.tau.floor);
             if (!gs.certain) out.put(SearchState{0.0, 0.0, 0.0, 0.0, -1.0}, true);
         };
@@ -490,13 +506,13 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
 #pragma unroll 1
     for (int it = 0;; ++it) {
         if (need_mle) {
-            series_xsums<C>(p, g, gm.s, r, xs_m);
-            bracket_sums<C>(p, bm, f, gm.s, r, ld_m, sh_m);
+            series_xsums<C, LP>(p, g, gm.s, r, xs_m);
+            km.sums(p, f, gm.s, r, ld_m, sh_m);
         }
         if (need_reml) {
             if (!need_mle || __any_sync(kFull, gm.s != gr.s || bm != br)) {
-                series_xsums<C>(p, g, gr.s, r, xs_r);
-                bracket_sums<C>(p, br, f, gr.s, r, ld_r, sh_r);
+                series_xsums<C, LP>(p, g, gr.s, r, xs_r);
+                kr.sums(p, f, gr.s, r, ld_r, sh_r);
             } else {
 #pragma unroll
                 for (int q = 0; q < L::NX; ++q) xs_r[q] = xs_m[q];
@@ -513,7 +529,7 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
         }
         if (need_reml) {
             assemble<C>(row0, sh_r, xs_r);
-            gr.take(group_reml<C>(pab_reduce<C>(row0), log_iab, ld_r, p, r), it, p.n_iter, out_r);
+            gr.take(group_reml<C, LP>(pab_reduce<C>(row0), log_iab, ld_r, p, r), it, p.n_iter, out_r);
         }
         if (GUIDE && it == p.n_iter + 1) return;
     }
@@ -541,7 +557,7 @@ __global__ void __launch_bounds__(Search<C>::kThreads, Search<C>::kMinBlocks)
 // ---------------------------------------------------------------- plain form, guided
 // The plain form's golden sections would take a direct FP64 pass over x per probe (46 passes
 // with a logarithm and a reciprocal per sample and pair in mode 4), although nearly every
-// decision is far from a tie.  So lmm_search_kernel<C, true> takes the decisions that its
+// decision is far from a tie.  So lmm_search_kernel<.., true> takes the decisions that its
 // series approximations settle beyond their error (guide_tau), lmm_open_kernel takes the few
 // others by direct evaluations (lmm_close_kernel when they are many), and lmm_finish_kernel
 // makes one direct pass per pair for the
