@@ -291,8 +291,8 @@ int32_t jb_rotate_status(const void* workspace, int32_t* out, uintptr_t stream);
  * FP64 rotation of genotype calls on INT8 tensor cores: X = U^T G to FP64 accuracy, for calls
  * that are small integers (decoded codes, 3 = missing, mean-imputed with mean[j] without
  * centring).  jb_split_f64_prepare writes U (n x n, column-major, ldu) once per cohort as
- * seven exact int8 digit planes (base 254, a power-of-two scale per eigenvector; remainder
- * below 3e-17 max|U_col|); jb_rotate_codes_f64 sums every digit product exactly in int32
+ * seven int8 digit planes (signed base 256, a power-of-two scale per eigenvector; rounded to
+ * 2.8e-17 max|U_col|); jb_rotate_codes_f64 sums every digit product exactly in int32
  * and adds the seven in FP64.  has_missing = 0 says that the chunk holds no missing call and
  * halves the work; a missing call found all the same is imputed as with has_missing = 1.
  * Workspace: jb_rotate_codes_f64_workspace_size(n, m) bytes, its first int32 a pipeline status

@@ -1,13 +1,13 @@
 // FP64 eigenvector rotation x~ = U^T g of genotype calls on INT8 tensor cores.
 //
 // Calls are small integers, so U^T g needs no FP64 multiplier: each eigenvector u_i (column i
-// of U) is scaled by a power of two s_i (s_i 127 >= max |u_i| > s_i 63.5) and written in seven
-// signed base-254 digits, U_ki = s_i sum_{t<7} q_t(k,i) 254^-t.  Every step of the split is
-// exact in FP64; what is left over is below s_i 254^-6 / 2, i.e. 3e-17 of max |u_i| -- less
-// than the rounding of U itself.  Each digit product accumulates exactly in int32 on tcgen05
-// (kind::i8) and the epilogue adds the seven products in FP64, so the result carries a few
-// roundings of its own size, where an FP64 GEMM carries those of n partial sums (measured
-// against exact sums, n = 20 000: see jb_rotate_codes_f64's test).
+// of U) is scaled by a power of two s_i and rounded to a 56-bit integer, U_ki = s_i X_ki with
+// 63.5 2^48 < max |X| <= 127 2^48, which is off by at most s_i / 2 -- 2.8e-17 of max |u_i|,
+// less than the rounding of its larger elements to doubles.  The seven signed base-256 digits of X are
+// its bytes after adding 128 to each (int8 digits in [-128, 127]).  Each digit product
+// accumulates exactly in int32 on tcgen05 (kind::i8) and the epilogue adds the seven products
+// in FP64, so the result carries a few roundings of its own size, where an FP64 GEMM carries
+// those of n partial sums.
 //
 // Missing calls are mean-imputed without centring (src/jamma/lmm/runner_streaming.py:
 // 427-434), g_j = z_j + mu_j m_j with m_j the missing mask: x~ = U^T z + mu_j U^T m.
@@ -37,59 +37,112 @@ constexpr int kXBN = 32 * kXDigits;   // digit rows of 32 eigenvectors
 constexpr int kXStages = 4;
 constexpr int kXLd = 33;              // padded row of the epilogue's output tile
 constexpr int kXEpiSmem = 128 * kXLd * 8;
-constexpr double kXBase = 254.0;
 using XSmem = GemmSmem<kXBN, kXStages, kXEpiSmem>;
 
 // ---------------------------------------------------------------- digit split
-// One CTA per eigenvector: its scale, then its seven digit rows.  scale[i] = s_i, 0 for a
-// zero eigenvector (no digits), NaN if an element is not finite (every output of that row
-// becomes NaN, as in a GEMM).
-__global__ void __launch_bounds__(256) xsplit_kernel(const double* __restrict__ U, int64_t n,
-                                                     int64_t ldu, int8_t* __restrict__ A,
-                                                     int64_t lda, double* __restrict__ scale) {
+// Digits of four consecutive samples k..k+3 of one eigenvector (X = U f1 f2), one 32-bit word
+// per digit row; rows 32 lda apart.
+__device__ __forceinline__ void xsplit_store(const double (&u)[4], double f1, double f2,
+                                             int8_t* __restrict__ at, int64_t lda) {
+    uint32_t lo[4], hi[4];  // low and high bytes of the four samples' digits
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const long long x = __double2ll_rn(u[q] * f1 * f2);
+        // bytes of X + 128 (1 + 256 + ...): digit + 128; then flip back to signed digits
+        const unsigned long long b = ((unsigned long long)x + 0x0080808080808080ull) ^
+                                     0x0080808080808080ull;
+        lo[q] = (uint32_t)b;
+        hi[q] = (uint32_t)(b >> 32);
+    }
+#pragma unroll
+    for (int t = 0; t < kXDigits; ++t) {  // digit t: byte 6 - t
+        const int by = kXDigits - 1 - t;
+        const uint32_t* w = by < 4 ? lo : hi;
+        const uint32_t sel = (uint32_t)((by & 3) | (((by & 3) + 4) << 4));
+        const uint32_t p01 = __byte_perm(w[0], w[1], sel), p23 = __byte_perm(w[2], w[3], sel);
+        *reinterpret_cast<uint32_t*>(at + 32 * t * lda) = __byte_perm(p01, p23, 0x5410);
+    }
+}
+
+// One CTA per eigenvector: its scale, then its seven digit rows (bound by HBM: U read, its
+// planes written).  STEPS > 0: each thread keeps its 4 STEPS elements in registers between
+// the two, n <= 4 kXSplitThreads STEPS; 0: the column is read twice.  scale[i] = s_i 256^6
+// (the leading digit's weight), 0 for a zero eigenvector (no digits), NaN if an element is
+// not finite (every output of that row becomes NaN, as in a GEMM).
+constexpr int kXSplitThreads = 512;
+template <int STEPS>
+__global__ void __launch_bounds__(kXSplitThreads)
+    xsplit_kernel(const double* __restrict__ U, int64_t n, int64_t ldu, int8_t* __restrict__ A,
+                  int64_t lda, double* __restrict__ scale) {
     const int64_t i = blockIdx.x;
     const double* __restrict__ col = U + i * ldu;
+    const bool vec = (reinterpret_cast<uintptr_t>(col) & 15) == 0;
+    auto load = [&](int64_t k, double (&u)[4]) {
+        if (vec && k + 4 <= n) {
+            const double2 a = __ldg(reinterpret_cast<const double2*>(col + k));
+            const double2 b = __ldg(reinterpret_cast<const double2*>(col + k + 2));
+            u[0] = a.x;
+            u[1] = a.y;
+            u[2] = b.x;
+            u[3] = b.y;
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) u[q] = k + q < n ? __ldg(col + k + q) : 0.0;
+        }
+    };
     double mx = 0.0;
     bool bad = false;
-    for (int64_t k = threadIdx.x; k < n; k += blockDim.x) {
-        const double a = fabs(col[k]);
-        bad = bad || !(a <= 1.7976931348623157e308);
-        mx = fmax(mx, a);
+    auto look = [&](const double (&u)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const double a = fabs(u[q]);
+            bad = bad || !(a <= 1.7976931348623157e308);
+            mx = fmax(mx, a);
+        }
+    };
+    const int64_t k0 = 4 * (int64_t)threadIdx.x, dk = 4 * (int64_t)kXSplitThreads;
+    double keep[STEPS > 0 ? STEPS : 1][4];
+    if (STEPS > 0) {
+#pragma unroll
+        for (int s = 0; s < STEPS; ++s) load(k0 + s * dk, keep[s]);
+#pragma unroll
+        for (int s = 0; s < STEPS; ++s) look(keep[s]);
+    } else {
+        for (int64_t k = k0; k < n; k += dk) {
+            load(k, keep[0]);
+            look(keep[0]);
+        }
     }
-    __shared__ double red[8];
+    __shared__ double red[kXSplitThreads / 32];
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
     bad = __syncthreads_or(bad);
-    for (int w = 0; w < 8; ++w) mx = fmax(mx, red[w]);
-    // 2^e with 63.5 < mx 2^e <= 127
-    int e = 0;
+    for (int w = 0; w < kXSplitThreads / 32; ++w) mx = fmax(mx, red[w]);
+    int e = 0;  // X = U 2^e
     const bool zero = bad || !(mx > 0.0);
     if (!zero) {
         frexp(mx, &e);  // mx = f 2^e, f in [1/2, 1)
-        e = 7 - e;      // mx 2^e in [64, 128)
-        if (scalbn(mx, e) > 127.0) --e;
+        e = 55 - e;     // mx 2^e in [2^54, 2^55)
+        if (scalbn(mx, e) > 127.0 * 281474976710656.0) --e;  // the top digit holds 127 at most
     }
     if (threadIdx.x == 0)
-        scale[i] = bad ? __longlong_as_double(0x7ff8000000000000ll) : (zero ? 0.0 : scalbn(1.0, -e));
+        scale[i] = bad ? __longlong_as_double(0x7ff8000000000000ll) : (zero ? 0.0 : scalbn(1.0, 48 - e));
+    // 2^e as two factors, each a normal double for every e (|e| < 1140); none without digits
+    const double f1 = zero ? 0.0 : scalbn(1.0, e / 2), f2 = scalbn(1.0, e - e / 2);
     int8_t* __restrict__ rows = A + ((i / 32) * kXBN + (i % 32)) * lda;
-    for (int64_t k = 4 * (int64_t)threadIdx.x; k < lda; k += 4 * (int64_t)blockDim.x) {
-        uint32_t w[kXDigits];
+    if (STEPS > 0) {
 #pragma unroll
-        for (int t = 0; t < kXDigits; ++t) w[t] = 0u;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (k + q >= n || zero) continue;
-            double a = scalbn(col[k + q], e);  // |a| <= 127, exact
-#pragma unroll
-            for (int t = 0; t < kXDigits; ++t) {
-                const double r = rint(a);
-                w[t] |= (uint32_t)(uint8_t)(int8_t)(int)r << (8 * q);
-                a = (a - r) * kXBase;  // exact: |a - r| <= 1/2 drops 7 leading bits, 254 adds 7
+        for (int s = 0; s < STEPS; ++s)
+            if (k0 + s * dk < lda) {
+                if (bad) keep[s][0] = keep[s][1] = keep[s][2] = keep[s][3] = 0.0;
+                xsplit_store(keep[s], f1, f2, rows + k0 + s * dk, lda);
             }
+    } else {
+        for (int64_t k = k0; k < lda; k += dk) {
+            load(k, keep[0]);
+            if (bad) keep[0][0] = keep[0][1] = keep[0][2] = keep[0][3] = 0.0;
+            xsplit_store(keep[0], f1, f2, rows + k, lda);
         }
-#pragma unroll
-        for (int t = 0; t < kXDigits; ++t)
-            *reinterpret_cast<uint32_t*>(rows + 32 * t * lda + k) = w[t];
     }
 }
 
@@ -164,10 +217,10 @@ struct XEpi {
                                         uint8_t* smem) const {
         double* S = reinterpret_cast<double*>(smem);  // [row][kXLd]
         constexpr int kRows = PAIRED ? 64 : 128;      // SNPs of the tile
-        constexpr double w1 = 1.0 / kXBase;
+        constexpr double w1 = 1.0 / 256.0;
         const int row = 32 * q + lane;                // TMEM lane
         const int i0 = nb * 32;
-        // V[e] = sum_t C_t 254^-t, smallest digit first (Horner's rule from the last digit)
+        // V[e] = sum_t C_t 256^-t, smallest digit first (Horner's rule from the last digit)
         double v[32];
         {
             uint32_t c[32];
@@ -303,8 +356,15 @@ int32_t jb_split_f64_prepare(const double* U, int64_t n, int64_t ldu, void* plan
         const int64_t first = (P.rows - kXBN) * P.lda;
         JB_CUDA(cudaMemsetAsync(ws + P.a_off + first, 0, (size_t)(kXBN * P.lda), st));
     }
-    xsplit_kernel<<<(unsigned)n, 256, 0, st>>>(U, n, ldu, reinterpret_cast<int8_t*>(ws + P.a_off), P.lda,
-                                               reinterpret_cast<double*>(ws + P.s_off));
+    // P.lda is the span a CTA writes, so the register forms are chosen by it
+    const int64_t step = 4 * (int64_t)kXSplitThreads;
+    auto kern = P.lda <= 2 * step ? xsplit_kernel<2>
+                : P.lda <= 4 * step ? xsplit_kernel<4>
+                : P.lda <= 8 * step ? xsplit_kernel<8>
+                : P.lda <= 12 * step ? xsplit_kernel<12>
+                                     : xsplit_kernel<0>;
+    kern<<<(unsigned)n, kXSplitThreads, 0, st>>>(U, n, ldu, reinterpret_cast<int8_t*>(ws + P.a_off), P.lda,
+                                                 reinterpret_cast<double*>(ws + P.s_off));
     JB_LAUNCH_CHECK("xsplit_kernel");
     return JB_OK;
 }

@@ -131,6 +131,20 @@ class DeviceCohort:
                   else colmajor(np.asarray(eigenvectors, dtype=np.float64)))
         if self.U.shape != (n, n) or self.evals.shape != (n,):
             raise ValueError("eigendecomposition does not match the number of samples")
+        # the smallest eigenvalue decides the search's form: read before other work is queued
+        ev_min = float(np.min(eigenvalues) if not isinstance(eigenvalues, torch.Tensor)
+                       else self.evals.min().item())
+        # digit planes of U for the rotation of calls: four in the mixed form, seven exact
+        # ones in the FP64 form (where U^T G is a GEMM without them), which the first chunk of
+        # calls makes: chunks of other genotypes never need them
+        self.ozaki = None
+        self.exact = precision == "fp64" and n <= EXACT_MAX_SAMPLES
+        if precision == "mixed":
+            self.ozaki = ozaki if ozaki is not None else ozaki_split(self.U)
+        elif (self.exact and ozaki is not None
+              and ozaki.numel() == _native.load().jb_split_f64_workspace_size(n)):
+            self.ozaki = ozaki
+        self.code_ld = (n + 127) // 128 * 128 if precision == "mixed" or self.exact else n
         self.UtW = rotate(self.U, colmajor(W))
         self.Uty = rotate(self.U, colmajor(y))
         self.lam0 = self.logl0 = None
@@ -141,16 +155,6 @@ class DeviceCohort:
             _native.call("jb_null_mle", n, c, phi, ptr(self.evals), ptr(self.UtW), n, ptr(self.Uty),
                          n, NULL_L_MIN, NULL_L_MAX, NULL_N_GRID, NULL_N_ITER, ptr(self.lam0),
                          ptr(self.logl0), st)
-        # digit planes of U for the rotation of calls: four in the mixed form, seven exact
-        # ones in the FP64 form (where U^T G is a GEMM without them)
-        self.ozaki = None
-        if precision == "mixed":
-            self.ozaki = ozaki if ozaki is not None else ozaki_split(self.U)
-        elif n <= EXACT_MAX_SAMPLES:
-            shared = (ozaki is not None
-                      and ozaki.numel() == _native.load().jb_split_f64_workspace_size(n))
-            self.ozaki = ozaki if shared else exact_split(self.U)
-        self.code_ld = (n + 127) // 128 * 128 if self.ozaki is not None else n
         self._rot_ws = None
         self._chunk_ws = None
         # The interpolated search expands 1/(lambda*eval + 1) in log lambda over the fixed
@@ -159,7 +163,6 @@ class DeviceCohort:
         # The FP64 form stays a search of direct evaluations (search 0), with the decisions
         # that are far from a tie taken on the same series where these hold and its golden
         # brackets are narrow enough for their expansions to reach rounding level.
-        ev_min = float(self.evals.min().item())
         series = (1.0 + SERIES_L_MAX * ev_min > 0.5
                   and self.l_min >= SERIES_L_MIN and self.l_max <= SERIES_L_MAX)
         self.search = 1 if precision == "mixed" and series else 0
@@ -250,6 +253,8 @@ class DeviceCohort:
                          out: torch.Tensor | None = None) -> torch.Tensor:
         """FP64 form: U^T G (m, n) of decoded codes from the exact digit planes."""
         m, ld = codes.shape
+        if self.ozaki is None:
+            self.ozaki = exact_split(self.U)
         need = _native.load().jb_rotate_codes_f64_workspace_size(self.n, m)
         if self._rot_ws is None or self._rot_ws.numel() < need:
             self._rot_ws = workspace(need)
@@ -274,7 +279,7 @@ class DeviceCohort:
         UtG = UtG[:m] if UtG is not None and UtG.shape[0] >= m else None
         if self.precision == "mixed":
             return self.associate_rotated(self.rotate_codes_i8(codes, means, has_missing, UtG), out)
-        if self.ozaki is not None:
+        if self.exact:
             return self.associate_rotated(self.rotate_codes_f64(codes, means, has_missing, UtG), out)
         G = bufs.get("G")
         if G is None or G.shape[0] < m:
@@ -321,7 +326,7 @@ class ChunkGraph:
         self.counts = torch.zeros((m, 4), dtype=torch.int32, device="cuda")
         self.out = cohort.alloc_out(m)
         self.bufs = {"UtG": empty((m, n))}
-        if cohort.ozaki is None:
+        if cohort.precision != "mixed" and not cohort.exact:
             self.bufs["G"] = empty((m, n))
         caller = torch.cuda.current_stream()
         side = torch.cuda.Stream()
