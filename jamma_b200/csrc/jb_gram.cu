@@ -18,6 +18,7 @@
 #include "jb_rotate_i8.cuh"
 
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 namespace jb {
@@ -245,74 +246,82 @@ __global__ void kin_vectors_reduce_kernel(int64_t n, int64_t nblk, const double*
 // Missing-call terms for one SNP chunk (at most kSpMaxChunk SNPs):
 //   Q[i, k] += R_ik + T_ik / 2,   R_ik = sum_{j in miss(k)} mu_j z_ij,
 //                                 T_ik = sum_{j in miss(k) and miss(i)} mu_j^2
-// (z_ij the 0/1/2 call, 0 where missing).  R is n x nnz(M) multiply-adds: with 1 % of calls
-// missing that is 1 % of a dense Z diag(mu) M^T, so it runs on the FP64 pipe from
-// registers rather than densely on the tensor cores.
+// (z_ij the 0/1/2 call, 0 where missing).  With 1 % of calls missing that is 1 % of a dense
+// product with FP64 weights, and each sample k has its own list of SNPs, so it runs on the
+// CUDA cores.
 //
-// kin_sp_words_kernel (one warp per SNP): the chunk's calls as "dosage words", 16 samples
-// per uint32, 2 bits each: the call 0/1/2, or 3 where it is missing.
+// kin_sp_words_kernel: the chunk's calls as "dosage words", 16 samples per uint32, 2 bits
+// each: the call 0/1/2, or 3 where it is missing.
 //
-// kin_sp_kernel: one CTA per (sample k, block b of 4096 samples i).  The CTA turns k's
-// missing-SNP bitmask into an increasing list in shared memory, then walks it once with
-// every thread owning 16 consecutive samples i: per SNP j one dosage word, and per sample
-// one FMA of mu_j with the word's 2-bit value c as the double 4 + c.  A missing call
-// (c = 3) adds 3 mu_j more than R wants; it also marks the (i, k, j) triple of T.  Two
-// bit operations per word find the missing calls, and for each of them a rare branch adds
-// mu_j^2/2 - 3 mu_j into the sample's slot in shared memory (thread-private, summed in SNP
-// order).  So R + T/2 comes out of one walk with no per-SNP lists and no atomics.
-constexpr int kSpThreads = 256;
-constexpr int kSpSpt = 16;                      // samples per thread = one dosage word
-constexpr int kSpBlock = kSpThreads * kSpSpt;  // samples per CTA
-constexpr int kSpWords = kSpBlock / 16;        // dosage words per CTA
-constexpr int kSpMaxChunk = 16384;             // SNPs per call (list in shared memory)
+// kin_sp_kernel: one CTA per (sample k, block of samples i).  The CTA turns k's missing-SNP
+// bitmask into an increasing list in shared memory and takes the list's SNPs kG at a time
+// (the method of the Four Russians): the kG 2-bit values of a sample are one index into a
+// table of the 4^kG sums of their terms -- c mu_j for a call c, mu_j^2 / 2 for a missing one,
+// so the missing x missing term needs no branch -- and every sample adds one table entry per
+// kG SNPs.  Bound by shared memory: per thread and 16 samples 16 table reads, 16 additions
+// and ~50 integer instructions to transpose the words' 2-bit fields into indexes (an FMA per
+// sample and SNP took ~5.7 instructions).  The table is replicated for each lane of a
+// half-warp, [entry][16], so that a read of any 16 entries has no bank conflict; it is built
+// for the next kG SNPs while the current one is read.
+// kG = 4 pays for its 256-entry table with two words per thread (n > 5120); smaller cohorts take
+// 3 (n > 2048) or 2.  Two CTAs per SM, so that one's table, list and result phases run beside
+// the other's reads (one CTA of 640 threads: 31.5 against 28.0 ms below).
+// Measured against one FMA per sample and SNP from registers, a chunk of 16 384 SNPs with 1 %
+// missing, all of its terms: n = 20 000 19.3 -> 13.2 ms, n = 8001 3.8 -> 3.0 ms, n = 1940
+// 1.2 -> 0.66 ms; 30 011 SNPs at n = 20 000 in chunks of 10 000, this kernel 36.5 -> 24.2 ms.
+constexpr int kSpMaxThreads = 320;
+constexpr int kSpMaxChunk = 16384;  // SNPs per call (list in shared memory)
+constexpr int kSpMinThreads = 256;  // the list is built by the first 256 threads
 
-struct SpSmem {
-    double corr[kSpSpt][kSpThreads];  // per-thread missing-call terms, [sample][thread]
-    uint16_t jl[kSpMaxChunk];         // k's missing SNPs, increasing
-    int warp_sum[kSpThreads / 32];
+// Launch shape for `words` dosage words (16 samples each) per SNP.
+struct SpShape {
+    int g;        // SNPs per table
+    int wpt;      // words per thread
+    int threads, blocks;
 };
-
-// 16 samples s0..s0+15 of one SNP row of int8 codes (0/1/2 calls, 3 missing; samples at
-// or beyond n read as call 0): z = the calls, 2 bits each (missing -> 0); miss = bit 2q
-// set where sample s0 + q is missing.
-__device__ __forceinline__ void sp_load16(const int8_t* __restrict__ row, int64_t s0, int64_t n,
-                                          bool vec, uint32_t& z, uint32_t& miss) {
-    uint32_t x[4] = {0u, 0u, 0u, 0u};
-    if (vec && s0 + 16 <= n) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + s0));
-        x[0] = v.x;
-        x[1] = v.y;
-        x[2] = v.z;
-        x[3] = v.w;
-    } else {
-        for (int q = 0; q < 16; ++q)
-            if (s0 + q < n) x[q >> 2] |= (uint32_t)(uint8_t)row[s0 + q] << (8 * (q & 3));
-    }
-    z = 0u;
-    miss = 0u;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const uint32_t m3 = __vcmpeq4(x[e], 0x03030303u);  // 0xff in each missing byte
-        const uint32_t c = x[e] & ~m3 & 0x03030303u;
-        const uint32_t pz = (c & 0x3u) | ((c >> 6) & 0xCu) | ((c >> 12) & 0x30u) | ((c >> 18) & 0xC0u);
-        const uint32_t pm = (m3 & 0x1u) | ((m3 >> 6) & 0x4u) | ((m3 >> 12) & 0x10u) | ((m3 >> 18) & 0x40u);
-        z |= pz << (8 * e);
-        miss |= pm << (8 * e);
-    }
+inline SpShape sp_shape(int64_t words) {
+    SpShape s;
+    s.wpt = words > kSpMaxThreads ? 2 : 1;
+    s.g = s.wpt == 2 ? 4 : (words >= 128 ? 3 : 2);
+    s.blocks = (int)ceil_div(words, (int64_t)kSpMaxThreads * s.wpt);
+    const int64_t per = ceil_div(ceil_div(words, s.blocks), s.wpt);
+    s.threads = (int)(ceil_div(per, 32) * 32);
+    if (s.threads < kSpMinThreads) s.threads = kSpMinThreads;
+    return s;
+}
+constexpr int kSpPad = 16;        // list entries past the end that name the row of zero words
+constexpr int sp_smem(int g) {  // two tables, the list, the warp counts
+    return 2 * (1 << (2 * g)) * 16 * 8 + (kSpMaxChunk + kSpPad) * 2 + 64;
 }
 
+// Dosage words of one SNP per warp: word w of a row of wpr (a multiple of 4) holds samples
+// w, w + wpr, ..., w + 15 wpr, so that the threads of kin_sp_kernel, one word each, own
+// consecutive samples and reach Q along its columns.  A lane makes four words from four codes
+// at a time.
 __global__ void __launch_bounds__(256) kin_sp_words_kernel(const int8_t* __restrict__ codes,
                                                            int64_t ldc, int64_t n, int64_t m,
                                                            int64_t wpr, int vec,
                                                            uint32_t* __restrict__ zb) {
     const int64_t j = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    if (j >= m) return;  // warp-uniform
+    if (j > m) return;  // warp-uniform; row m holds zero words
     const int8_t* row = codes + j * ldc;
-    for (int64_t wi = lane; wi < wpr; wi += 32) {
-        uint32_t z, miss;
-        sp_load16(row, wi * 16, n, vec != 0, z, miss);
-        zb[j * wpr + wi] = z | miss | (miss << 1);  // missing -> 3
+    for (int64_t w = 4 * lane; w < wpr; w += 128) {
+        uint32_t o[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            if (j == m) break;
+            const int64_t s = q * wpr + w;  // samples s .. s + 3
+            uint32_t x = 0u;
+            if (vec && s + 4 <= n)
+                x = __ldg(reinterpret_cast<const uint32_t*>(row + s));
+            else
+                for (int e = 0; e < 4; ++e)
+                    if (s + e < n) x |= (uint32_t)(uint8_t)row[s + e] << (8 * e);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] |= ((x >> (8 * e)) & 3u) << (2 * q);
+        }
+        *reinterpret_cast<uint4*>(zb + j * wpr + w) = make_uint4(o[0], o[1], o[2], o[3]);
     }
 }
 
@@ -353,43 +362,36 @@ __global__ void __launch_bounds__(256) kin_mask_kernel(const int8_t* __restrict_
     if (s0 + lane < n) mask[(s0 + lane) * words + jt] = out;
 }
 
-// One SNP for a thread's 16 samples.  A word value c (0..3) becomes the double 4 + c built
-// in one 64-bit integer multiply-add: the two bits, masked at bit position pos (20..30) of
-// w or of w shifted by 10 or 20, times 2^(50 - pos) land at bits 50-51 -- the top two
-// mantissa bits -- of the bit pattern of 4.0 (exponent 2, so they weigh 1 and 2), and the
-// result is already the register pair the FMA with mu_j reads.  The offset 4 sum_j mu_j is
-// removed afterwards (4 mu is exact, so a sample with only zero calls ends with exactly
-// 4 x the plain sum).
-__device__ __forceinline__ double sp_call_double(uint32_t masked, uint32_t mult) {
-    unsigned long long d;
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(masked), "r"(mult), "l"(0x4010000000000000ull));
-    return __longlong_as_double((long long)d);
+// Indexes of 16 samples from the words of four SNPs: byte b of out[h] is that of sample
+// 4 b + h, its bits 2 e, 2 e + 1 the value of SNP e.
+__device__ __forceinline__ void sp_indexes(const uint32_t (&w)[4], uint32_t (&out)[4]) {
+    const uint32_t m2 = 0x33333333u, m4 = 0x0f0f0f0fu;
+    const uint32_t a = (w[0] & m2) | ((w[1] << 2) & ~m2), b = ((w[0] >> 2) & m2) | (w[1] & ~m2);
+    const uint32_t c = (w[2] & m2) | ((w[3] << 2) & ~m2), d = ((w[2] >> 2) & m2) | (w[3] & ~m2);
+    // nibbles of a, c: even samples; of b, d: odd samples
+    out[0] = (a & m4) | ((c << 4) & ~m4);
+    out[2] = ((a >> 4) & m4) | (c & ~m4);
+    out[1] = (b & m4) | ((d << 4) & ~m4);
+    out[3] = ((b >> 4) & m4) | (d & ~m4);
 }
 
-__device__ __forceinline__ void sp_word(uint32_t w, double u, double (&r)[kSpSpt]) {
-    const uint32_t g[3] = {w << 20, w << 10, w};  // samples 0-4, 5-9, 10-15 at bits 20-31
-#pragma unroll
-    for (int q = 0; q < kSpSpt; ++q) {
-        const int gi = q < 5 ? 0 : (q < 10 ? 1 : 2);
-        const int pos = 2 * q + (gi == 0 ? 20 : (gi == 1 ? 10 : 0));
-        r[q] = fma(u, sp_call_double(g[gi] & (3u << pos), 1u << (50 - pos)), r[q]);
-    }
-}
-
-template <bool kR>
-__global__ void __launch_bounds__(kSpThreads, 3) kin_sp_kernel(
+template <bool kR, int kG, int kWpt>
+__global__ void __launch_bounds__(kSpMaxThreads, 2) kin_sp_kernel(
     const uint32_t* __restrict__ zb, int64_t wpr, const uint32_t* __restrict__ mask,
-    int64_t words, const double* __restrict__ mu, int64_t n, double* __restrict__ Q,
+    int64_t words, const double* __restrict__ mu, int64_t n, int64_t m, double* __restrict__ Q,
     int64_t ldq) {
+    constexpr int kRows = 1 << (2 * kG);
+    // the tables, [entry][buffer][16 copies]: 256 bytes an entry, so that one byte permutation
+    // makes an address of an index byte and the lane's copy of the current buffer
     extern __shared__ __align__(16) unsigned char sp_smem_raw[];
-    SpSmem& S = *reinterpret_cast<SpSmem*>(sp_smem_raw);
+    uint16_t* jl = reinterpret_cast<uint16_t*>(sp_smem_raw + kRows * 256);
+    int* warp_cnt = reinterpret_cast<int*>(jl + kSpMaxChunk + kSpPad);
     const int64_t k = blockIdx.x;
-    const int b = blockIdx.y;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // k's missing SNPs in increasing order: thread t owns mask words 2t, 2t+1
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
+    // k's missing SNPs in increasing order: thread t < 256 owns mask words 2t, 2t+1
     const uint32_t* __restrict__ mk = mask + k * words;
-    uint32_t m0 = 2 * tid < words ? __ldg(mk + 2 * tid) : 0u;
-    uint32_t m1 = 2 * tid + 1 < words ? __ldg(mk + 2 * tid + 1) : 0u;
+    uint32_t m0 = tid < 256 && 2 * tid < words ? __ldg(mk + 2 * tid) : 0u;
+    uint32_t m1 = tid < 256 && 2 * tid + 1 < words ? __ldg(mk + 2 * tid + 1) : 0u;
     const int c = __popc(m0) + __popc(m1);
     int incl = c;
 #pragma unroll
@@ -397,84 +399,114 @@ __global__ void __launch_bounds__(kSpThreads, 3) kin_sp_kernel(
         const int t = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += t;
     }
-    if (lane == 31) S.warp_sum[warp] = incl;
-#pragma unroll
-    for (int q = 0; q < kSpSpt; ++q) S.corr[q][tid] = 0.0;  // this thread's own slots
+    if (lane == 31 && warp < 8) warp_cnt[warp] = incl;
     __syncthreads();
     int pos = incl - c, cnt = 0;
 #pragma unroll
-    for (int w = 0; w < kSpThreads / 32; ++w) {
-        pos += w < warp ? S.warp_sum[w] : 0;
-        cnt += S.warp_sum[w];
+    for (int w = 0; w < 8; ++w) {
+        pos += w < warp ? warp_cnt[w] : 0;
+        cnt += warp_cnt[w];
     }
     while (m0) {
-        S.jl[pos++] = (uint16_t)(64 * tid + __ffs(m0) - 1);
+        jl[pos++] = (uint16_t)(64 * tid + __ffs(m0) - 1);
         m0 &= m0 - 1u;
     }
     while (m1) {
-        S.jl[pos++] = (uint16_t)(64 * tid + 32 + __ffs(m1) - 1);
+        jl[pos++] = (uint16_t)(64 * tid + 32 + __ffs(m1) - 1);
         m1 &= m1 - 1u;
     }
+    if (tid < kSpPad) jl[cnt + tid] = (uint16_t)m;
     __syncthreads();
-    double r[kSpSpt];
-#pragma unroll
-    for (int q = 0; q < kSpSpt; ++q) r[q] = 0.0;
-    double s = 0.0;
-    const int64_t wi = (int64_t)b * kSpWords + tid;
-    const bool act = wi < wpr;
-    const uint32_t* __restrict__ zc = zb + (act ? wi : 0);
-    uint32_t wn[4];
-    double un[4];
-    auto fetch = [&](int p0) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int p = p0 + e;
-            if (p < cnt) {
-                const int64_t j = S.jl[p];
-                un[e] = __ldg(mu + j);
-                wn[e] = act ? __ldg(zc + j * wpr) : 0u;
-            } else {
-                un[e] = 0.0;
-                wn[e] = 0u;
-            }
+    // The table of one group of SNPs from their mu (0 past the list's end: terms of zero).  A
+    // warp takes the 16 entries of one value of SNPs 2 and 3, two entries at a time (one per
+    // half-warp, its 16 lanes writing the 16 copies): entry 2 s + half has SNP 0's value
+    // 2 (s & 1) + half and SNP 1's s / 2.
+    auto term = [&](int x, double u) {  // of a value x = 0..3
+        const double r = kR ? u : 0.0;
+        return x == 3 ? 0.5 * u * u : (x == 2 ? 2.0 * r : (x == 1 ? r : 0.0));
+    };
+    const uint32_t copy = (uint32_t)(lane & 15) * 8;
+    auto build = [&](uint32_t buf, const double (&u)[4]) {
+        const int half = lane >> 4;
+        const double a0 = term(half, u[0]), a1 = term(2 + half, u[0]);
+        const double b1 = term(1, u[1]), b2 = term(2, u[1]), b3 = term(3, u[1]);
+        for (int hi = warp; hi < kRows / 16; hi += nthr / 32) {
+            const double f = (kG > 2 ? term(hi & 3, u[2]) : 0.0) + (kG > 3 ? term(hi >> 2, u[3]) : 0.0);
+            unsigned char* at = sp_smem_raw + (hi * 16 + half) * 256 + buf + copy;
+            const double f0 = f + a0, f1 = f + a1;
+            *reinterpret_cast<double*>(at) = f0;
+            *reinterpret_cast<double*>(at + 512) = f1;
+            *reinterpret_cast<double*>(at + 2 * 512) = f0 + b1;
+            *reinterpret_cast<double*>(at + 3 * 512) = f1 + b1;
+            *reinterpret_cast<double*>(at + 4 * 512) = f0 + b2;
+            *reinterpret_cast<double*>(at + 5 * 512) = f1 + b2;
+            *reinterpret_cast<double*>(at + 6 * 512) = f0 + b3;
+            *reinterpret_cast<double*>(at + 7 * 512) = f1 + b3;
         }
     };
-    fetch(0);
-#pragma unroll 1
-    for (int p0 = 0; p0 < cnt; p0 += 4) {
-        uint32_t w[4];
-        double u[4];
+    auto mus = [&](int p0, double (&u)[4]) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            w[e] = wn[e];
-            u[e] = un[e];
-        }
-        fetch(p0 + 4);
+        for (int e = 0; e < 4; ++e) u[e] = e < kG && p0 + e < cnt ? __ldg(mu + jl[p0 + e]) : 0.0;
+    };
+    // this thread's words: wbase + tid and, with two, wbase + tid + nthr
+    const int64_t per = (wpr + gridDim.y - 1) / gridDim.y;
+    const int64_t wbase = (int64_t)blockIdx.y * per, wend = wbase + per < wpr ? wbase + per : wpr;
+    const uint32_t* zc[kWpt];
+    bool act[kWpt];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            if (kR) {
-                s += u[e];
-                sp_word(w[e], u[e], r);
-            }
-            uint32_t mm = w[e] & (w[e] >> 1) & 0x55555555u;  // bit 2q: sample q missing
-            if (mm) {
-                const double h = kR ? fma(0.5 * u[e], u[e], -3.0 * u[e]) : 0.5 * u[e] * u[e];
-                do {
-                    const int q = (__ffs(mm) - 1) >> 1;
-                    S.corr[q][tid] += h;
-                    mm &= mm - 1u;
-                } while (mm);
-            }
-        }
+    for (int q = 0; q < kWpt; ++q) {
+        const int64_t wi = wbase + tid + (int64_t)q * nthr;
+        act[q] = wi < wend;
+        zc[q] = zb + (act[q] ? wi : 0);  // a thread without a word reads one and drops its sums
     }
-    const double s4 = 4.0 * s;
-    const int64_t i0 = (int64_t)b * kSpBlock + (int64_t)tid * kSpSpt;
+    const uint32_t row = (uint32_t)wpr;
+    uint32_t nx[kWpt][4];
+    auto fetch = [&](int p0, int q) {  // at most 2 kG past the list's end: rows of zero words
 #pragma unroll
-    for (int q = 0; q < kSpSpt; ++q) {
-        const int64_t i = i0 + q;
-        double v = S.corr[q][tid];
-        if (kR) v += r[q] - s4;
-        if (i < n && v != 0.0) Q[k * ldq + i] += v;  // Q[i, k] (column-major, column k)
+        for (int e = 0; e < 4; ++e) nx[q][e] = e < kG ? __ldg(zc[q] + (uint32_t)jl[p0 + e] * row) : 0u;
+    };
+    double acc[kWpt][16];
+#pragma unroll
+    for (int q = 0; q < kWpt; ++q)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[q][i] = 0.0;
+    double u[4];
+    mus(0, u);
+    build(0, u);
+#pragma unroll
+    for (int q = 0; q < kWpt; ++q) fetch(0, q);
+    mus(kG, u);
+    __syncthreads();
+    uint32_t buf = 0;  // byte offset of the current table within an entry: 0 or 128
+#pragma unroll 1
+    for (int p0 = 0; p0 < cnt; p0 += kG, buf ^= 128) {
+        build(buf ^ 128, u);
+        mus(p0 + 2 * kG, u);  // loaded a whole group before their table is built
+        const uint32_t low = buf + copy;
+#pragma unroll
+        for (int q = 0; q < kWpt; ++q) {
+            uint32_t ix[4];
+            sp_indexes(nx[q], ix);
+            fetch(p0 + kG, q);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const uint32_t off = __byte_perm(ix[i & 3], low, 0x5504u | ((i >> 2) << 4));
+                acc[q][i] += *reinterpret_cast<const double*>(sp_smem_raw + off);
+            }
+        }
+        __syncthreads();  // the next table is complete, this one has been read
+    }
+#pragma unroll
+    for (int q = 0; q < kWpt; ++q) {
+        const int64_t i0 = wbase + tid + (int64_t)q * nthr;
+        if (!act[q]) continue;
+        double* __restrict__ col = Q + k * ldq;  // Q[i, k]
+#pragma unroll
+        for (int s = 0; s < 16; ++s)  // all loads in flight before the first store
+            if (i0 + s * wpr < n) acc[q][s] += col[i0 + s * wpr];
+#pragma unroll
+        for (int s = 0; s < 16; ++s)
+            if (i0 + s * wpr < n) col[i0 + s * wpr] = acc[q][s];
     }
 }
 
@@ -548,20 +580,46 @@ struct KinREpi {
     }
 };
 
-// K = (C - a_i - a_j + s - b_i - b_j + Q_ij + Q_ji) / p, symmetric, column-major.
-__global__ void kin_finalize_i8_kernel(const int32_t* __restrict__ C, int64_t ldc, int64_t n,
-                                       const double* __restrict__ a, const double* __restrict__ b,
-                                       double s, const double* __restrict__ RT, int64_t ldr,
-                                       double inv_p, double* __restrict__ K, int64_t ldk) {
-    for (int64_t j = blockIdx.y; j < n; j += gridDim.y) {
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= j && i < n;
-             i += (int64_t)gridDim.x * blockDim.x) {
-            // the int32 Gram holds the upper triangle (row i <= column j) at C[j*ldc + i]
-            double v = (double)C[j * ldc + i] - a[i] - a[j] + s - b[i] - b[j];
-            if (RT) v += RT[j * ldr + i] + RT[i * ldr + j];
-            v *= inv_p;
-            K[j * ldk + i] = v;
-            K[i * ldk + j] = v;
+// K = (C - a_i - a_j + s - b_i - b_j + Q_ij + Q_ji) / p, symmetric, column-major, by tiles of
+// 32 x 32 with row block <= column block.  Bound by HBM (C's upper triangle and all of Q read,
+// K written); the mirrored halves of Q and K pass through shared memory, so that every access
+// runs along a column.
+__global__ void __launch_bounds__(256) kin_finalize_i8_kernel(
+    const int32_t* __restrict__ C, int64_t ldc, int64_t n, const double* __restrict__ a,
+    const double* __restrict__ b, double s, const double* __restrict__ RT, int64_t ldr,
+    double inv_p, double* __restrict__ K, int64_t ldk) {
+    __shared__ double t[32][33];
+    const int64_t i0 = (int64_t)blockIdx.x * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    for (int64_t jb = blockIdx.y; jb * 32 < n; jb += gridDim.y) {
+        const int64_t j0 = jb * 32;
+        if (i0 > j0) continue;  // the same decision in every thread
+        __syncthreads();
+        if (RT) {  // t[r][c] = Q[j0 + c, i0 + r], read along column i0 + r
+            for (int r = ty; r < 32; r += 8)
+                t[r][tx] = i0 + r < n && j0 + tx < n ? RT[(i0 + r) * ldr + j0 + tx] : 0.0;
+            __syncthreads();
+        }
+        double v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int64_t i = i0 + tx, j = j0 + ty + 8 * e;
+            v[e] = 0.0;
+            if (j < n && i <= j) {
+                // the int32 Gram holds the upper triangle (row i <= column j) at C[j*ldc + i]
+                double x = (double)C[j * ldc + i] - a[i] - a[j] + s - b[i] - b[j];
+                if (RT) x += RT[j * ldr + i] + t[tx][ty + 8 * e];
+                v[e] = x * inv_p;
+                K[j * ldk + i] = v[e];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 4; ++e) t[ty + 8 * e][tx] = v[e];  // t[c][r]: K[i0 + r, j0 + c]
+        __syncthreads();
+        for (int r = ty; r < 32; r += 8) {
+            const int64_t i = i0 + r, j = j0 + tx;  // K[j, i], along column i
+            if (j < n && i < j) K[i * ldk + j] = t[tx][r];
         }
     }
 }
@@ -793,7 +851,6 @@ int32_t jb_codes_to_sample_major(const int8_t* codes, int64_t ld_codes, int64_t 
 // Workspace of the correction entry points (tc: with the tensor-core R operand).
 struct KinCorrWs {
     int64_t status, pa, mask, zb, tiles, B, ldb, total, wpr, words;
-    int nb;
 };
 static KinCorrWs kin_corr_ws(int64_t n, int64_t m, bool tc) {
     KinCorrWs w;
@@ -801,8 +858,7 @@ static KinCorrWs kin_corr_ws(int64_t n, int64_t m, bool tc) {
     const int64_t nblk = ceil_div(mm, 256);
     auto a256 = [](int64_t x) { return (x + 255) / 256 * 256; };
     w.words = ceil_div(mm, 32);
-    w.wpr = ceil_div(n, 16);
-    w.nb = (int)ceil_div(n, kSpBlock);
+    w.wpr = ceil_div(n, 64) * 4;
     int64_t off = 0;
     w.status = off;
     off += 256;
@@ -811,7 +867,7 @@ static KinCorrWs kin_corr_ws(int64_t n, int64_t m, bool tc) {
     w.mask = off;
     off += a256(n * w.words * 4);
     w.zb = off;
-    off += a256(mm * w.wpr * 4);
+    off += a256((mm + 1) * w.wpr * 4);  // and a row of zero words
     w.ldb = (mm + 127) / 128 * 128;
     w.tiles = off;
     off += tc ? a256(ceil_div(n, kBM) * ceil_div(4 * n, 256) * (int64_t)sizeof(Tile)) : 0;
@@ -853,13 +909,20 @@ static int32_t kin_missing_terms(const int8_t* codes, int64_t ld_codes, int64_t 
                                  uint8_t* ws, bool with_r, cudaStream_t st) {
     const uint32_t* mask = reinterpret_cast<const uint32_t*>(ws + L.mask);
     uint32_t* zb = reinterpret_cast<uint32_t*>(ws + L.zb);
-    const int vec = ((reinterpret_cast<uintptr_t>(codes) & 15) == 0 && ld_codes % 16 == 0) ? 1 : 0;
-    kin_sp_words_kernel<<<(unsigned)ceil_div(m, 8), 256, 0, st>>>(codes, ld_codes, n, m, L.wpr, vec, zb);
+    const int vec = ((reinterpret_cast<uintptr_t>(codes) & 3) == 0 && ld_codes % 4 == 0) ? 1 : 0;
+    kin_sp_words_kernel<<<(unsigned)ceil_div(m + 1, 8), 256, 0, st>>>(codes, ld_codes, n, m, L.wpr, vec, zb);
     JB_LAUNCH_CHECK("kin_sp_words_kernel");
-    auto kern = with_r ? kin_sp_kernel<true> : kin_sp_kernel<false>;
-    JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpSmem)));
-    kern<<<dim3((unsigned)n, (unsigned)L.nb), kSpThreads, sizeof(SpSmem), st>>>(
-        zb, L.wpr, mask, L.words, mu, n, RT, ldr);
+    const SpShape sh = sp_shape(L.wpr);
+    auto pick = [&](auto r) {
+        constexpr bool R = decltype(r)::value;
+        if (sh.wpt == 2) return kin_sp_kernel<R, 4, 2>;
+        return sh.g == 3 ? kin_sp_kernel<R, 3, 1> : kin_sp_kernel<R, 2, 1>;
+    };
+    auto kern = with_r ? pick(std::true_type{}) : pick(std::false_type{});
+    const int smem = sp_smem(sh.g);
+    JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kern<<<dim3((unsigned)n, (unsigned)sh.blocks), sh.threads, smem, st>>>(zb, L.wpr, mask, L.words, mu, n,
+                                                                            m, RT, ldr);
     JB_LAUNCH_CHECK("kin_sp_kernel");
     return JB_OK;
 }
@@ -877,8 +940,7 @@ int32_t jb_kinship_i8_corrections(const int8_t* codes, int64_t ld_codes, int32_t
     if (m == 0) return JB_OK;
     JB_CHECK_ARG(m <= kSpMaxChunk, "jb_kinship_i8_corrections: at most %d SNPs per call", kSpMaxChunk);
     JB_CHECK_ARG(codes && mu && a && b, "jb_kinship_i8_corrections: null pointer");
-    JB_CHECK_ARG(n * ceil_div(n, kSpBlock) < (1ll << 31) && n < (1ll << 31),
-                 "jb_kinship_i8_corrections: n too large");
+    JB_CHECK_ARG(n < (1ll << 21), "jb_kinship_i8_corrections: n too large");
     const KinCorrWs L = kin_corr_ws(n, m, false);
     JB_CHECK_ARG(workspace && workspace_bytes >= L.total,
                  "jb_kinship_i8_corrections: workspace too small");
@@ -949,7 +1011,7 @@ int32_t jb_kinship_i8_finalize(const int32_t* C, int64_t ldc, int64_t n, const d
                                const double* b, double sum_mu2, const double* RT, int64_t ldr,
                                int64_t p_kept, double* K, int64_t ldk, uintptr_t stream) {
     JB_CHECK_ARG(n > 0 && ldc >= n && ldk >= n && p_kept > 0, "jb_kinship_i8_finalize: bad shape");
-    dim3 grid((unsigned)(ceil_div(n, 256) < 64 ? ceil_div(n, 256) : 64), grid_y(n), 1);
+    dim3 grid((unsigned)ceil_div(n, 32), grid_y(ceil_div(n, 32)), 1);
     kin_finalize_i8_kernel<<<grid, 256, 0, as_stream(stream)>>>(C, ldc, n, a, b, sum_mu2, RT, ldr,
                                                                1.0 / (double)p_kept, K, ldk);
     JB_LAUNCH_CHECK("kin_finalize_i8_kernel");
