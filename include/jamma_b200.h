@@ -203,6 +203,33 @@ int32_t jb_kinship_i8_finalize(const int32_t* C, int64_t ldc, int64_t n, const d
                                uintptr_t stream);
 
 /*
+ * The same kinship in full FP64 accuracy on the INT8 tensor cores (no reference counterpart;
+ * an evaluation of _accumulate_kinship, src/jamma/kinship/compute.py:46-57).  With r_j =
+ * rint(mu_j), z' = z - r (0 where missing) and d = mu - r:
+ *   p K = Z' Z'^T - a 1^T - 1 a^T + sum_j d_j^2 - b 1^T - 1 b^T + Q + Q^T,
+ * a = Z' d and sum d^2 as unevaluated sums of two doubles, b_i the sum of d_j^2 over i's
+ * missing SNPs, Q the missing-call terms (zeroed by the caller).
+ * jb_kinship_exact_accumulate: m <= 16384 SNPs (codes SNP-major, 3 = missing): writes columns
+ *   col0.. of the sample-major operand Zs (n x ldz) and adds to a, a_lo, b (n doubles each) and,
+ *   when has_missing, Q (n x n, ldq).  workspace: jb_kinship_exact_workspace_size(n, m) bytes.
+ * jb_gram_i8_add: jb_gram_i8 adding to C, for an operand taken block by block.
+ * jb_kinship_exact_finalize: K from the int32 Gram's upper triangle, the vectors, s + s_lo =
+ *   sum d^2 and Q (NULL without missing calls); K may be Q's buffer.
+ */
+int64_t jb_kinship_exact_workspace_size(int64_t n, int64_t m);
+int32_t jb_kinship_exact_accumulate(const int8_t* codes, int64_t ld_codes, int64_t n, int64_t m,
+                                    const double* mu, int32_t has_missing, int8_t* Zs, int64_t ldz,
+                                    int64_t col0, double* a, double* a_lo, double* b, double* Q,
+                                    int64_t ldq, void* workspace, int64_t workspace_bytes,
+                                    uintptr_t stream);
+int32_t jb_gram_i8_add(const int8_t* Z, int64_t n, int64_t p, int64_t ldz, int32_t* C, int64_t ldc,
+                       void* workspace, int64_t workspace_bytes, uintptr_t stream);
+int32_t jb_kinship_exact_finalize(const int32_t* C, int64_t ldc, int64_t n, const double* a,
+                                  const double* a_lo, const double* b, double s, double s_lo,
+                                  const double* Q, int64_t ldq, int64_t p_kept, double* K,
+                                  int64_t ldk, uintptr_t stream);
+
+/*
  * Leave-one-chromosome-out kinship (compute_loco_kinship_streaming,
  * src/jamma/kinship/compute.py:693-916): K_loco = (S_full - S_chr) / p_loco.
  * jb_kinship_i8_finalize_loco: from the full-genome and one chromosome's int32 Grams

@@ -89,6 +89,12 @@ SIGNATURES: dict[str, tuple] = {
     "jb_kinship_i8_corrections": (
         _i32, [_p, _i64, _i32, _i64, _i64, _p, _p, _p, _p, _i64, _p, _i64, _u]),
     "jb_kinship_i8_finalize": (_i32, [_p, _i64, _i64, _p, _p, _f64, _p, _i64, _i64, _p, _i64, _u]),
+    "jb_kinship_exact_workspace_size": (_i64, [_i64, _i64]),
+    "jb_kinship_exact_accumulate": (
+        _i32, [_p, _i64, _i64, _i64, _p, _i32, _p, _i64, _i64, _p, _p, _p, _p, _i64, _p, _i64, _u]),
+    "jb_gram_i8_add": (_i32, [_p, _i64, _i64, _i64, _p, _i64, _p, _i64, _u]),
+    "jb_kinship_exact_finalize": (
+        _i32, [_p, _i64, _i64, _p, _p, _p, _f64, _f64, _p, _i64, _i64, _p, _i64, _u]),
     "jb_ozaki_workspace_size": (_i64, [_i64]),
     "jb_ozaki_prepare": (_i32, [_p, _i64, _i64, _p, _i64, _u]),
     "jb_rotate_i8_workspace_size": (_i64, [_i64, _i64]),

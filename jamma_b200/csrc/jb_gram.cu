@@ -10,6 +10,12 @@
 //   p K = Z Z^T - a 1^T - 1 a^T + (sum mu^2) 1 1^T - b 1^T - 1 b^T + R + R^T + T
 //   a = Z mu,  b = M mu^2,  R = Z diag(mu) M^T,  T = M diag(mu^2) M^T
 //
+// The same identity holds for calls shifted by any integer r_j per SNP, with z - r for z, mu - r
+// for mu: the exact form (jb_kinship_exact_*) takes r_j = rint(mu_j), so that |mu - r| <= 1/2
+// and every term is of the size of the result, keeps a as an unevaluated sum of two doubles
+// and combines the terms in such sums, so that K comes out correctly rounded but for Q's
+// roundings (Q is ~1 % of the terms) -- closer to exact sums than an FP64 product.
+//
 // T is symmetric, so R + R^T + T = Q + Q^T with Q = R + T/2: one n x n buffer holds both
 // sparse terms.  The dense Z Z^T runs on tcgen05 (kind::i8); the vectors and Q are FP64
 // on the CUDA cores.
@@ -84,6 +90,7 @@ struct GramEpi {
     int32_t* C;
     int64_t ldc;
     int n;
+    bool add;  // add to C instead of overwriting it
     __device__ __forceinline__ void run(int mb, int nb, uint32_t taddr, int q, int lane,
                                         uint8_t*) const {
         const int i = mb * kBM + 32 * q + lane;
@@ -95,7 +102,10 @@ struct GramEpi {
             if (i < n) {
 #pragma unroll
                 for (int t = 0; t < 32; ++t) {
-                    if (j0 + t < n) C[(int64_t)(j0 + t) * ldc + i] = (int32_t)v[t];
+                    if (j0 + t < n) {
+                        int32_t* c = C + (int64_t)(j0 + t) * ldc + i;
+                        *c = (int32_t)v[t] + (add ? *c : 0);
+                    }
                 }
             }
         }
@@ -118,18 +128,45 @@ __host__ __device__ inline int gram_tiles(int MB, int NB, Tile* out) {
     return k;
 }
 
-__global__ void gram_tiles_kernel(int MB, int NB, Tile* out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) gram_tiles(MB, NB, out);
+// The same list on the device, one CTA: the tiles of row group gm and column nb are the rows
+// gm .. min(gm + 15, MB - 1, 2 nb + 1), so every thread writes one such run at a prefix sum of
+// the runs' lengths (one thread walking the list took 0.46 ms at n = 20 000; 6 us).
+__global__ void __launch_bounds__(1024) gram_tiles_kernel(int MB, int NB, Tile* out) {
+    __shared__ int wsum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int runs = (MB + 15) / 16 * NB;
+    int base = 0;  // tiles of the runs before this round of 1024
+    for (int r0 = 0; r0 < runs; r0 += 1024) {
+        const int r = r0 + threadIdx.x;
+        const int gm = r / NB * 16, nb = r % NB;
+        const int last = min(min(gm + 15, MB - 1), 2 * nb + 1);
+        const int c = r < runs && last >= gm ? last - gm + 1 : 0;
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        int pos = base + incl - c;
+        for (int w = 0; w < 32; ++w) {
+            pos += w < warp ? wsum[w] : 0;
+            base += wsum[w];
+        }
+        for (int k = 0; k < c; ++k) out[pos + k] = Tile{gm + k, nb};
+        __syncthreads();  // wsum is written again
+    }
 }
 
 // ---------------------------------------------------------------- layout kernels
 // SNP-major codes (m x ldc, 3 = missing) -> sample-major int8 calls Zs[i, col0 + j]
-// (missing -> 0), through 32x32 shared-memory tiles.
+// (missing -> 0), through 32x32 shared-memory tiles; with mu, less rint(mu_j).
 // Optionally also the raw codes Cs[i, j] (3 kept) of this chunk, sample-major.
 __global__ void codes_to_sample_major_kernel(const int8_t* __restrict__ codes, int64_t ldc,
                                              int64_t n, int64_t m, int8_t* __restrict__ Zs,
                                              int64_t ldz, int64_t col0, int8_t* __restrict__ Cs,
-                                             int64_t ldcs) {
+                                             int64_t ldcs, const double* __restrict__ mu) {
     __shared__ int8_t t[32][33];
     const int64_t j0 = (int64_t)blockIdx.x * 32, i0 = (int64_t)blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
@@ -142,7 +179,8 @@ __global__ void codes_to_sample_major_kernel(const int8_t* __restrict__ codes, i
         const int64_t i = i0 + r, j = j0 + tx;
         if (i < n && j < m) {
             const int8_t v = t[tx][r];
-            if (Zs) Zs[i * ldz + col0 + j] = (v == 3) ? (int8_t)0 : v;
+            const int8_t r = mu ? (int8_t)(int)rint(__ldg(mu + j)) : (int8_t)0;
+            if (Zs) Zs[i * ldz + col0 + j] = (v == 3) ? (int8_t)0 : (int8_t)(v - r);
             if (Cs) Cs[i * ldcs + j] = v;
         }
     }
@@ -153,7 +191,7 @@ __global__ void codes_to_sample_major_kernel(const int8_t* __restrict__ codes, i
 // sample as one uint32 each.
 __global__ void __launch_bounds__(256) codes_to_sample_major_vec_kernel(
     const int8_t* __restrict__ codes, int64_t ldc, int64_t n, int64_t m, int8_t* __restrict__ Zs,
-    int64_t ldz, int64_t col0) {
+    int64_t ldz, int64_t col0, const double* __restrict__ mu) {
     __shared__ uint32_t t[64][17];  // t[j][i / 4]: samples i..i+3 of SNP j
     const int64_t j0 = (int64_t)blockIdx.x * 64, i0 = (int64_t)blockIdx.y * 64;
     for (int r = threadIdx.x; r < 64 * 16; r += 256) {
@@ -178,8 +216,9 @@ __global__ void __launch_bounds__(256) codes_to_sample_major_vec_kernel(
         uint32_t w = 0u;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            uint32_t b = (t[jq + e][ii >> 2] >> (8 * (ii & 3))) & 0xffu;
-            w |= (b == 3u ? 0u : b) << (8 * e);  // missing -> 0
+            const uint32_t b = (t[jq + e][ii >> 2] >> (8 * (ii & 3))) & 0xffu;
+            const uint32_t r = mu && j + e < m ? (uint32_t)(int)rint(__ldg(mu + j + e)) : 0u;
+            w |= (b == 3u ? 0u : (b - r) & 0xffu) << (8 * e);  // missing -> 0
         }
         int8_t* q = Zs + i * ldz + col0 + j;
         if (j + 4 <= m)
@@ -240,6 +279,54 @@ __global__ void kin_vectors_reduce_kernel(int64_t n, int64_t nblk, const double*
         sb += pb[k * n + i];
     }
     a[i] += sa;
+    b[i] += sb;
+}
+
+// The exact form's vectors: a_i = sum_j (z_ij - r_j) (mu_j - r_j) over the observed calls as an
+// unevaluated sum hi + lo, b_i = sum_{j missing at i} (mu_j - r_j)^2.
+__device__ __forceinline__ void dd_add(double& hi, double& lo, double x) {
+    const double s = hi + x, t = s - hi;
+    lo += (hi - (s - t)) + (x - t);  // the exact rounding error of s
+    hi = s;
+}
+
+__global__ void kin_exact_partial_kernel(const int8_t* __restrict__ codes, int64_t ldc, int64_t n,
+                                         int64_t m, const double* __restrict__ mu,
+                                         double* __restrict__ pa, double* __restrict__ pl,
+                                         double* __restrict__ pb) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t jb = blockIdx.y, j0 = jb * 256, j1 = j0 + 256 < m ? j0 + 256 : m;
+    if (i >= n) return;
+    double hi = 0.0, lo = 0.0, sb = 0.0;
+#pragma unroll 4
+    for (int64_t j = j0; j < j1; ++j) {
+        const int c = codes[j * ldc + i];
+        const double u = __ldg(mu + j), r = rint(u), d = u - r;  // exact
+        if (c == 3)
+            sb = fma(d, d, sb);
+        else
+            dd_add(hi, lo, ((double)c - r) * d);  // |c - r| <= 2: exact
+    }
+    pa[jb * n + i] = hi;
+    pl[jb * n + i] = lo;
+    pb[jb * n + i] = sb;
+}
+
+__global__ void kin_exact_reduce_kernel(int64_t n, int64_t nblk, const double* __restrict__ pa,
+                                        const double* __restrict__ pl, const double* __restrict__ pb,
+                                        double* __restrict__ a, double* __restrict__ al,
+                                        double* __restrict__ b) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double hi = a[i], lo = al[i], sb = 0.0;
+    for (int64_t k = 0; k < nblk; ++k) {
+        dd_add(hi, lo, pa[k * n + i]);
+        lo += pl[k * n + i];
+        sb += pb[k * n + i];
+    }
+    const double s = hi + lo;  // |hi| is far above |lo| or both are small: renormalise
+    al[i] = lo - (s - hi);
+    a[i] = s;
     b[i] += sb;
 }
 
@@ -375,7 +462,7 @@ __device__ __forceinline__ void sp_indexes(const uint32_t (&w)[4], uint32_t (&ou
     out[3] = ((b >> 4) & m4) | (d & ~m4);
 }
 
-template <bool kR, int kG, int kWpt>
+template <bool kR, bool kShift, int kG, int kWpt>
 __global__ void __launch_bounds__(kSpMaxThreads, 2) kin_sp_kernel(
     const uint32_t* __restrict__ zb, int64_t wpr, const uint32_t* __restrict__ mask,
     int64_t words, const double* __restrict__ mu, int64_t n, int64_t m, double* __restrict__ Q,
@@ -421,21 +508,25 @@ __global__ void __launch_bounds__(kSpMaxThreads, 2) kin_sp_kernel(
     // warp takes the 16 entries of one value of SNPs 2 and 3, two entries at a time (one per
     // half-warp, its 16 lanes writing the 16 copies): entry 2 s + half has SNP 0's value
     // 2 (s & 1) + half and SNP 1's s / 2.
-    auto term = [&](int x, double u) {  // of a value x = 0..3
-        const double r = kR ? u : 0.0;
-        return x == 3 ? 0.5 * u * u : (x == 2 ? 2.0 * r : (x == 1 ? r : 0.0));
+    // term of a value x = 0..3: (x - r) d of a call, d^2 / 2 of a missing one, where d is mu (r =
+    // 0) or, in the exact form, mu - r with r = rint(mu)
+    auto term = [&](int x, double u) {
+        const double r = kShift ? rint(u) : 0.0, d = u - r;
+        if (x == 3) return 0.5 * d * d;
+        return kR ? ((double)x - r) * d : 0.0;
     };
     const uint32_t copy = (uint32_t)(lane & 15) * 8;
     auto build = [&](uint32_t buf, const double (&u)[4]) {
         const int half = lane >> 4;
         const double a0 = term(half, u[0]), a1 = term(2 + half, u[0]);
+        const double b0 = kShift ? term(0, u[1]) : 0.0;
         const double b1 = term(1, u[1]), b2 = term(2, u[1]), b3 = term(3, u[1]);
         for (int hi = warp; hi < kRows / 16; hi += nthr / 32) {
             const double f = (kG > 2 ? term(hi & 3, u[2]) : 0.0) + (kG > 3 ? term(hi >> 2, u[3]) : 0.0);
             unsigned char* at = sp_smem_raw + (hi * 16 + half) * 256 + buf + copy;
             const double f0 = f + a0, f1 = f + a1;
-            *reinterpret_cast<double*>(at) = f0;
-            *reinterpret_cast<double*>(at + 512) = f1;
+            *reinterpret_cast<double*>(at) = kShift ? f0 + b0 : f0;
+            *reinterpret_cast<double*>(at + 512) = kShift ? f1 + b0 : f1;
             *reinterpret_cast<double*>(at + 2 * 512) = f0 + b1;
             *reinterpret_cast<double*>(at + 3 * 512) = f1 + b1;
             *reinterpret_cast<double*>(at + 4 * 512) = f0 + b2;
@@ -584,10 +675,15 @@ struct KinREpi {
 // 32 x 32 with row block <= column block.  Bound by HBM (C's upper triangle and all of Q read,
 // K written); the mirrored halves of Q and K pass through shared memory, so that every access
 // runs along a column.
+// K may be Q's own buffer: a block reads both tiles of Q that it writes as K, each value in the
+// thread that overwrites it or before a barrier.
+// kExact: a and s are unevaluated sums with a_lo, s_lo; the terms are added in such a sum and
+// the result is divided by p once.
+template <bool kExact>
 __global__ void __launch_bounds__(256) kin_finalize_i8_kernel(
     const int32_t* __restrict__ C, int64_t ldc, int64_t n, const double* __restrict__ a,
-    const double* __restrict__ b, double s, const double* __restrict__ RT, int64_t ldr,
-    double inv_p, double* __restrict__ K, int64_t ldk) {
+    const double* __restrict__ a_lo, const double* __restrict__ b, double s, double s_lo,
+    const double* RT, int64_t ldr, double p, double* K, int64_t ldk) {
     __shared__ double t[32][33];
     const int64_t i0 = (int64_t)blockIdx.x * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
@@ -607,9 +703,20 @@ __global__ void __launch_bounds__(256) kin_finalize_i8_kernel(
             v[e] = 0.0;
             if (j < n && i <= j) {
                 // the int32 Gram holds the upper triangle (row i <= column j) at C[j*ldc + i]
-                double x = (double)C[j * ldc + i] - a[i] - a[j] + s - b[i] - b[j];
-                if (RT) x += RT[j * ldr + i] + t[tx][ty + 8 * e];
-                v[e] = x * inv_p;
+                if (kExact) {
+                    double hi = (double)C[j * ldc + i], lo = s_lo - a_lo[i] - a_lo[j];
+                    dd_add(hi, lo, s);
+                    dd_add(hi, lo, -a[i]);
+                    dd_add(hi, lo, -a[j]);
+                    double q = -b[i] - b[j];
+                    if (RT) q += RT[j * ldr + i] + t[tx][ty + 8 * e];
+                    dd_add(hi, lo, q);
+                    v[e] = (hi + lo) / p;
+                } else {
+                    double x = (double)C[j * ldc + i] - a[i] - a[j] + s - b[i] - b[j];
+                    if (RT) x += RT[j * ldr + i] + t[tx][ty + 8 * e];
+                    v[e] = x * (1.0 / p);
+                }
                 K[j * ldk + i] = v[e];
             }
         }
@@ -724,8 +831,8 @@ int64_t jb_gram_i8_workspace_size(int64_t n) {
     return gram_ws(n).total;
 }
 
-int32_t jb_gram_i8(const int8_t* Z, int64_t n, int64_t p, int64_t ldz, int32_t* C, int64_t ldc,
-                   void* workspace, int64_t workspace_bytes, uintptr_t stream) {
+static int32_t gram_i8(const int8_t* Z, int64_t n, int64_t p, int64_t ldz, int32_t* C, int64_t ldc,
+                       bool add, void* workspace, int64_t workspace_bytes, uintptr_t stream) {
     JB_CHECK_ARG(n > 0 && p > 0 && ldz >= p && ldc >= n, "jb_gram_i8: bad shape");
     JB_CHECK_ARG(n < (1ll << 31) && p < (1ll << 31), "jb_gram_i8: size too large");
     JB_CHECK_ARG(4ll * p < (1ll << 31), "jb_gram_i8: p too large for exact int32 accumulation");
@@ -743,17 +850,27 @@ int32_t jb_gram_i8(const int8_t* Z, int64_t n, int64_t p, int64_t ldz, int32_t* 
     rc = make_map_i8(&tb, Z, n, p, ldz, kGramBN);
     if (rc) return rc;
     JB_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
-    gram_tiles_kernel<<<1, 32, 0, st>>>(MB, NB, tiles);
+    gram_tiles_kernel<<<1, 1024, 0, st>>>(MB, NB, tiles);
     JB_LAUNCH_CHECK("gram_tiles_kernel");
     auto kern = i8_gemm_kernel<kGramBN, kGramStages, GramEpi>;
     JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  GramSmem::TOTAL));
-    GramEpi epi{C, ldc, (int)n};
+    GramEpi epi{C, ldc, (int)n, add};
     const int grid = n_tiles < num_sms() ? n_tiles : num_sms();
     const int num_kb = (int)ceil_div(p, kBK);
     kern<<<grid, kThreads, GramSmem::TOTAL, st>>>(ta, tb, tiles, n_tiles, num_kb, epi, status, nullptr, 0);
     JB_LAUNCH_CHECK("i8_gemm_kernel<gram>");
     return JB_OK;
+}
+
+int32_t jb_gram_i8(const int8_t* Z, int64_t n, int64_t p, int64_t ldz, int32_t* C, int64_t ldc,
+                   void* workspace, int64_t workspace_bytes, uintptr_t stream) {
+    return gram_i8(Z, n, p, ldz, C, ldc, false, workspace, workspace_bytes, stream);
+}
+
+int32_t jb_gram_i8_add(const int8_t* Z, int64_t n, int64_t p, int64_t ldz, int32_t* C, int64_t ldc,
+                       void* workspace, int64_t workspace_bytes, uintptr_t stream) {
+    return gram_i8(Z, n, p, ldz, C, ldc, true, workspace, workspace_bytes, stream);
 }
 
 int32_t jb_kinship_i8_finalize_loco(const int32_t* C_full, const int32_t* C_chr, int64_t ldc,
@@ -822,9 +939,9 @@ int32_t jb_gram_status(const void* workspace, int32_t* out, uintptr_t stream) {
     return JB_OK;
 }
 
-int32_t jb_codes_to_sample_major(const int8_t* codes, int64_t ld_codes, int64_t n, int64_t m,
-                                 int8_t* Zs, int64_t ldz, int64_t col0, int8_t* Cs, int64_t ldcs,
-                                 uintptr_t stream) {
+static int32_t sample_major(const int8_t* codes, int64_t ld_codes, int64_t n, int64_t m, int8_t* Zs,
+                            int64_t ldz, int64_t col0, int8_t* Cs, int64_t ldcs, const double* mu,
+                            uintptr_t stream) {
     JB_CHECK_ARG(n >= 0 && m >= 0 && ld_codes >= n && col0 >= 0,
                  "jb_codes_to_sample_major: bad shape");
     JB_CHECK_ARG(!Zs || ldz >= col0 + m, "jb_codes_to_sample_major: ldz too small");
@@ -837,15 +954,21 @@ int32_t jb_codes_to_sample_major(const int8_t* codes, int64_t ld_codes, int64_t 
         JB_CHECK_ARG(ceil_div(n, 64) < 65536, "jb_codes_to_sample_major: n too large");
         dim3 grid((unsigned)ceil_div(m, 64), (unsigned)ceil_div(n, 64), 1);
         codes_to_sample_major_vec_kernel<<<grid, 256, 0, as_stream(stream)>>>(codes, ld_codes, n, m, Zs,
-                                                                              ldz, col0);
+                                                                              ldz, col0, mu);
         JB_LAUNCH_CHECK("codes_to_sample_major_vec_kernel");
         return JB_OK;
     }
     dim3 grid((unsigned)ceil_div(m, 32), (unsigned)ceil_div(n, 32), 1);
     codes_to_sample_major_kernel<<<grid, dim3(32, 8), 0, as_stream(stream)>>>(codes, ld_codes, n,
-                                                                              m, Zs, ldz, col0, Cs, ldcs);
+                                                                              m, Zs, ldz, col0, Cs, ldcs, mu);
     JB_LAUNCH_CHECK("codes_to_sample_major_kernel");
     return JB_OK;
+}
+
+int32_t jb_codes_to_sample_major(const int8_t* codes, int64_t ld_codes, int64_t n, int64_t m,
+                                 int8_t* Zs, int64_t ldz, int64_t col0, int8_t* Cs, int64_t ldcs,
+                                 uintptr_t stream) {
+    return sample_major(codes, ld_codes, n, m, Zs, ldz, col0, Cs, ldcs, nullptr, stream);
 }
 
 // Workspace of the correction entry points (tc: with the tensor-core R operand).
@@ -863,7 +986,7 @@ static KinCorrWs kin_corr_ws(int64_t n, int64_t m, bool tc) {
     w.status = off;
     off += 256;
     w.pa = off;
-    off += a256(2 * nblk * n * 8);
+    off += a256(3 * nblk * n * 8);
     w.mask = off;
     off += a256(n * w.words * 4);
     w.zb = off;
@@ -906,19 +1029,21 @@ static int32_t kin_masks(const int8_t* codes, int64_t ld_codes, int64_t n, int64
 // Q += T/2 (with_r: + R) for one chunk from the masks (kin_masks) and the dosage words.
 static int32_t kin_missing_terms(const int8_t* codes, int64_t ld_codes, int64_t n, int64_t m,
                                  const double* mu, double* RT, int64_t ldr, const KinCorrWs& L,
-                                 uint8_t* ws, bool with_r, cudaStream_t st) {
+                                 uint8_t* ws, bool with_r, cudaStream_t st, bool shift = false) {
     const uint32_t* mask = reinterpret_cast<const uint32_t*>(ws + L.mask);
     uint32_t* zb = reinterpret_cast<uint32_t*>(ws + L.zb);
     const int vec = ((reinterpret_cast<uintptr_t>(codes) & 3) == 0 && ld_codes % 4 == 0) ? 1 : 0;
     kin_sp_words_kernel<<<(unsigned)ceil_div(m + 1, 8), 256, 0, st>>>(codes, ld_codes, n, m, L.wpr, vec, zb);
     JB_LAUNCH_CHECK("kin_sp_words_kernel");
     const SpShape sh = sp_shape(L.wpr);
-    auto pick = [&](auto r) {
-        constexpr bool R = decltype(r)::value;
-        if (sh.wpt == 2) return kin_sp_kernel<R, 4, 2>;
-        return sh.g == 3 ? kin_sp_kernel<R, 3, 1> : kin_sp_kernel<R, 2, 1>;
+    auto pick = [&](auto r, auto sf) {
+        constexpr bool R = decltype(r)::value, S = decltype(sf)::value;
+        if (sh.wpt == 2) return kin_sp_kernel<R, S, 4, 2>;
+        return sh.g == 3 ? kin_sp_kernel<R, S, 3, 1> : kin_sp_kernel<R, S, 2, 1>;
     };
-    auto kern = with_r ? pick(std::true_type{}) : pick(std::false_type{});
+    const std::true_type yes;
+    const std::false_type no;
+    auto kern = shift ? pick(yes, yes) : (with_r ? pick(yes, no) : pick(no, no));
     const int smem = sp_smem(sh.g);
     JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     kern<<<dim3((unsigned)n, (unsigned)sh.blocks), sh.threads, smem, st>>>(zb, L.wpr, mask, L.words, mu, n,
@@ -1012,8 +1137,59 @@ int32_t jb_kinship_i8_finalize(const int32_t* C, int64_t ldc, int64_t n, const d
                                int64_t p_kept, double* K, int64_t ldk, uintptr_t stream) {
     JB_CHECK_ARG(n > 0 && ldc >= n && ldk >= n && p_kept > 0, "jb_kinship_i8_finalize: bad shape");
     dim3 grid((unsigned)ceil_div(n, 32), grid_y(ceil_div(n, 32)), 1);
-    kin_finalize_i8_kernel<<<grid, 256, 0, as_stream(stream)>>>(C, ldc, n, a, b, sum_mu2, RT, ldr,
-                                                               1.0 / (double)p_kept, K, ldk);
+    kin_finalize_i8_kernel<false><<<grid, 256, 0, as_stream(stream)>>>(
+        C, ldc, n, a, nullptr, b, sum_mu2, 0.0, RT, ldr, (double)p_kept, K, ldk);
+    JB_LAUNCH_CHECK("kin_finalize_i8_kernel");
+    return JB_OK;
+}
+
+int64_t jb_kinship_exact_workspace_size(int64_t n, int64_t m) {
+    if (n <= 0 || m < 0) return -1;
+    return kin_corr_ws(n, m, false).total;
+}
+
+int32_t jb_kinship_exact_accumulate(const int8_t* codes, int64_t ld_codes, int64_t n, int64_t m,
+                                    const double* mu, int32_t has_missing, int8_t* Zs, int64_t ldz,
+                                    int64_t col0, double* a, double* a_lo, double* b, double* Q,
+                                    int64_t ldq, void* workspace, int64_t workspace_bytes,
+                                    uintptr_t stream) {
+    JB_CHECK_ARG(n > 0 && m >= 0 && ld_codes >= n, "jb_kinship_exact_accumulate: bad shape");
+    if (m == 0) return JB_OK;
+    JB_CHECK_ARG(codes && mu && Zs && a && a_lo && b && ldz >= col0 + m && col0 >= 0,
+                 "jb_kinship_exact_accumulate: null pointer or short operand");
+    JB_CHECK_ARG(m <= kSpMaxChunk, "jb_kinship_exact_accumulate: at most %d SNPs per call", kSpMaxChunk);
+    JB_CHECK_ARG(n < (1ll << 21), "jb_kinship_exact_accumulate: n too large");
+    JB_CHECK_ARG(!has_missing || (Q && ldq >= n), "jb_kinship_exact_accumulate: Q buffer needed");
+    const KinCorrWs L = kin_corr_ws(n, m, false);
+    JB_CHECK_ARG(workspace && workspace_bytes >= L.total,
+                 "jb_kinship_exact_accumulate: workspace too small");
+    int32_t rc = sample_major(codes, ld_codes, n, m, Zs, ldz, col0, nullptr, 0, mu, stream);
+    if (rc) return rc;
+    cudaStream_t st = as_stream(stream);
+    uint8_t* ws = static_cast<uint8_t*>(workspace);
+    const int64_t nblk = ceil_div(m, 256);
+    double* pa = reinterpret_cast<double*>(ws + L.pa);
+    kin_exact_partial_kernel<<<dim3((unsigned)ceil_div(n, 256), (unsigned)nblk), 256, 0, st>>>(
+        codes, ld_codes, n, m, mu, pa, pa + nblk * n, pa + 2 * nblk * n);
+    JB_LAUNCH_CHECK("kin_exact_partial_kernel");
+    kin_exact_reduce_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(n, nblk, pa, pa + nblk * n,
+                                                                        pa + 2 * nblk * n, a, a_lo, b);
+    JB_LAUNCH_CHECK("kin_exact_reduce_kernel");
+    if (!has_missing) return JB_OK;
+    rc = kin_masks(codes, ld_codes, n, m, L, ws, st);
+    if (rc) return rc;
+    return kin_missing_terms(codes, ld_codes, n, m, mu, Q, ldq, L, ws, true, st, true);
+}
+
+int32_t jb_kinship_exact_finalize(const int32_t* C, int64_t ldc, int64_t n, const double* a,
+                                  const double* a_lo, const double* b, double s, double s_lo,
+                                  const double* Q, int64_t ldq, int64_t p_kept, double* K,
+                                  int64_t ldk, uintptr_t stream) {
+    JB_CHECK_ARG(n > 0 && ldc >= n && ldk >= n && p_kept > 0 && a_lo,
+                 "jb_kinship_exact_finalize: bad shape");
+    dim3 grid((unsigned)ceil_div(n, 32), grid_y(ceil_div(n, 32)), 1);
+    kin_finalize_i8_kernel<true><<<grid, 256, 0, as_stream(stream)>>>(
+        C, ldc, n, a, a_lo, b, s, s_lo, Q, ldq, (double)p_kept, K, ldk);
     JB_LAUNCH_CHECK("kin_finalize_i8_kernel");
     return JB_OK;
 }

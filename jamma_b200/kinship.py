@@ -86,6 +86,115 @@ class _KinshipAccumulator:
         return self.K
 
 
+class _KinshipExact:
+    """The FP64 centered kinship through the exact INT8 tensor-core Gram of the calls less
+    rint(mean), with the centring terms in sums of two doubles (jb_kinship_exact_*): nothing
+    but the missing-call terms and the last division rounds, so that K is at least as close to
+    exact sums as the accumulated FP64 product.  SNPs fill blocks of BLOCK operand columns;
+    each full block is one Gram added to the int32 sums (at most 4 per SNP)."""
+
+    MAX_CHUNK = 16384
+    BLOCK = 65536
+
+    def __init__(self, n: int, p_kept: int, has_missing: bool):
+        self.n, self.p = n, p_kept
+        self.cols = min(self.BLOCK, p_kept)
+        self.ldz = (self.cols + 127) // 128 * 128
+        self.Zs = torch.empty((n, self.ldz), dtype=torch.int8, device="cuda")
+        self.C = torch.empty((n, n), dtype=torch.int32, device="cuda")
+        self.vec = torch.zeros((3, n), dtype=torch.float64, device="cuda")  # a, a_lo, b
+        self.Q = (torch.zeros if has_missing else torch.empty)(
+            (n, n), dtype=torch.float64, device="cuda")
+        self.has_missing = has_missing
+        lib = _native.load()
+        self.ws = workspace(lib.jb_kinship_exact_workspace_size(n, min(self.MAX_CHUNK, self.cols)))
+        self.gram_ws = workspace(lib.jb_gram_i8_workspace_size(n))
+        self._status: list[torch.Tensor] = []
+        self.col, self.blocks = 0, 0
+        self.sum_sq = np.longdouble(0.0)
+
+    @staticmethod
+    def device_bytes(n: int, p_kept: int) -> int:
+        lib = _native.load()
+        cols = min(_KinshipExact.BLOCK, p_kept)
+        return (12 * n * n + n * (cols + 128) + lib.jb_gram_i8_workspace_size(n)
+                + lib.jb_kinship_exact_workspace_size(n, min(_KinshipExact.MAX_CHUNK, cols)))
+
+    def add(self, codes: torch.Tensor, mu64_host: np.ndarray, has_missing: bool) -> None:
+        m, ld = codes.shape
+        mu = torch.from_numpy(mu64_host).to("cuda")
+        d = (mu64_host - np.rint(mu64_host)).astype(np.longdouble)
+        self.sum_sq += np.sum(d * d)
+        st, s = stream_handle(), 0
+        while s < m:
+            e = s + min(m - s, self.MAX_CHUNK, self.cols - self.col)
+            _native.call("jb_kinship_exact_accumulate", ptr(codes[s:e]), ld, self.n, e - s, ptr(mu[s:e]),
+                         int(has_missing), ptr(self.Zs), self.ldz, self.col, ptr(self.vec[0]),
+                         ptr(self.vec[1]), ptr(self.vec[2]), ptr(self.Q), self.n, ptr(self.ws),
+                         self.ws.numel(), st)
+            self.col += e - s
+            if self.col == self.cols:
+                self._gram()
+            s = e
+
+    def _gram(self) -> None:
+        entry = "jb_gram_i8_add" if self.blocks else "jb_gram_i8"
+        _native.call(entry, ptr(self.Zs), self.n, self.col, self.ldz, ptr(self.C), self.n,
+                     ptr(self.gram_ws), self.gram_ws.numel(), stream_handle())
+        self._status.append(self.gram_ws[:4].clone())
+        self.blocks += 1
+        self.col = 0
+
+    def finish(self) -> torch.Tensor:
+        if self.col:
+            self._gram()
+        hi = float(self.sum_sq)
+        _native.call("jb_kinship_exact_finalize", ptr(self.C), self.n, self.n, ptr(self.vec[0]),
+                     ptr(self.vec[1]), ptr(self.vec[2]), hi, float(self.sum_sq - np.longdouble(hi)),
+                     ptr(self.Q) if self.has_missing else None, self.n, self.p, ptr(self.Q), self.n,
+                     stream_handle())
+        status = torch.cat(self._status).view(torch.int32).cpu().numpy()
+        if np.any(status != 0):
+            raise RuntimeError(f"INT8 Gram pipeline reported status {status[status != 0][0]}")
+        return self.Q
+
+
+# Where the exact form is the faster one.  It pays ~0.25 ms of launches, the n^2 passes of its
+# int32 and missing-call sums, and a walk over the missing calls; the product runs at the FP64
+# rate.  Measured, product against exact form in ms at 0 / 1 / 5 / 10 % missing calls:
+#   n = 400,    p = 20 000   0.47 : 0.52 / 0.68 / 0.97 / 1.3
+#   n = 1200,   p =  5000    0.43 : 0.28 / 0.37 / 0.57 / 0.81
+#   n = 1940,   p = 12 226   1.70 : 0.42 / 0.71 / 1.4  / 2.4
+#   n = 4001,   p = 20 000   10.1 : 0.95 / 1.8  / 3.8  / 6.3
+#   n = 20 000, p = 30 011   340  : 7.5  / 34   / 121  / 228
+# The memory limit leaves half of what is free to the caller: the exact form holds 12 n^2 bytes
+# and the operand block where the product holds 8 n^2.
+EXACT_MIN_WORK = 1.0e10       # n^2 p
+EXACT_MIN_SAMPLES = 1000
+EXACT_MAX_SAMPLES = 65536
+EXACT_MIN_SNPS = 1000         # below, the n^2 passes weigh more than the product
+EXACT_MISSING_DENSITY = 0.03  # of all calls
+EXACT_MISSING_DENSITY_WIDE = 0.1  # from EXACT_WIDE_SAMPLES samples on
+EXACT_WIDE_SAMPLES = 4000
+
+
+def exact_form_pays(n: int, p_kept: int, n_missing: int) -> bool:
+    """Whether the FP64 centered kinship of n samples and p_kept SNPs takes the exact form."""
+    density = EXACT_MISSING_DENSITY_WIDE if n >= EXACT_WIDE_SAMPLES else EXACT_MISSING_DENSITY
+    return (EXACT_MIN_SAMPLES <= n <= EXACT_MAX_SAMPLES and EXACT_MIN_SNPS <= p_kept < 1 << 29
+            and float(n) * n * p_kept >= EXACT_MIN_WORK and n_missing <= density * n * p_kept)
+
+
+def _fp64_accumulator(n: int, p_kept: int, n_missing: int, batch: int):
+    """Accumulator of the FP64 centered kinship: exact form or FP64 product."""
+    if exact_form_pays(n, p_kept, n_missing):
+        free = (torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved()
+                - torch.cuda.memory_allocated())
+        if _KinshipExact.device_bytes(n, p_kept) <= free // 2:
+            return _KinshipExact(n, p_kept, n_missing > 0)
+    return _KinshipAccumulator(n, batch)
+
+
 # Missing-call density (fraction of a chunk's calls) above which the correction terms run
 # on the INT8 tensor cores instead of the FP64 walk over each sample's missing SNPs.
 TC_MISSING_DENSITY = 0.03
@@ -207,8 +316,12 @@ def _kinship_from_packed(packed_dev: torch.Tensor, n: int, batch_size: int, maf_
                 n_missing=int((n - c[:, 0]).sum()))
         acc.add_sum_mu2(c[:, 1] / np.maximum(c[:, 0], 1))
         return acc.finish(), idx.size
-    acc = _KinshipAccumulator(n, max(1, min(batch_size, 8192)))
-    acc.add(codes.index_select(0, sel), mu64)
+    n_missing = int((n - c[:, 0]).sum())
+    acc = _fp64_accumulator(n, idx.size, n_missing, max(1, min(batch_size, 8192)))
+    if isinstance(acc, _KinshipExact):
+        acc.add(codes.index_select(0, sel), c[:, 1] / np.maximum(c[:, 0], 1), n_missing > 0)
+    else:
+        acc.add(codes.index_select(0, sel), mu64)
     return acc.finish(), idx.size
 
 
@@ -239,7 +352,8 @@ def compute_centered_kinship(genotypes: np.ndarray, batch_size: int = 10000,
                              check_memory: bool = True, precision: str = "fp64") -> np.ndarray:
     """GEMMA -gk 1 relatedness matrix of an in-memory (n, p) genotype matrix.
 
-    ``precision="fp64"`` accumulates the centred FP64 Gram (cuBLAS DSYRK);
+    ``precision="fp64"`` forms the centred Gram to FP64 accuracy: through the exact integer
+    Gram of the shifted calls where ``exact_form_pays``, else as an FP64 product (cuBLAS DSYRK);
     ``precision="int8"`` runs the exact INT8 tensor-core Gram with FP64 corrections.
     """
     if precision not in ("fp64", "int8"):
@@ -283,7 +397,13 @@ def compute_kinship_from_bed(bfile, maf_threshold: float = 0.0, miss_threshold: 
     if idx.size == 0:
         raise ValueError("No SNPs passed filtering")
     i8 = precision == "int8"
-    acc = _KinshipI8(n, idx.size) if i8 else _KinshipAccumulator(n, min(chunk_size, 8192))
+    if i8:
+        acc = _KinshipI8(n, idx.size)
+    elif kinship_mode == 2:
+        acc = _KinshipAccumulator(n, min(chunk_size, 8192))
+    else:
+        acc = _fp64_accumulator(n, idx.size, int((n - counts[idx, 0]).sum()), min(chunk_size, 8192))
+    exact = isinstance(acc, _KinshipExact)
     for s in range(0, idx.size, chunk_size):
         sub = idx[s : s + chunk_size]
         rec = torch.from_numpy(bed.take(sub)).to("cuda")
@@ -295,6 +415,8 @@ def compute_kinship_from_bed(bfile, maf_threshold: float = 0.0, miss_threshold: 
             acc.add_sum_mu2(c[:, 1] / np.maximum(c[:, 0], 1))
         elif kinship_mode == 2:
             acc.add(codes, mu64, torch.from_numpy(snp_sd_from_counts(c, n)).to("cuda"))
+        elif exact:
+            acc.add(codes, c[:, 1] / np.maximum(c[:, 0], 1), bool(np.any(c[:, 0] < n)))
         else:
             acc.add(codes, mu64)
     K = acc.finish()
