@@ -59,6 +59,17 @@ int32_t jb_decode_bed(const uint8_t* packed, int64_t bytes_per_snp, int64_t m,
                       const int32_t* sample_idx, int64_t n, int8_t* codes,
                       int64_t ld_codes, int32_t* counts, uintptr_t stream);
 
+/*
+ * Dense genotypes (allele counts 0/1/2, NaN = missing) to count-A1 .bed records: element (i, j)
+ * of `rows` samples and m SNPs at g[i*ld + j] (along_snps) or g[j*ld + i], float (is_f32) or
+ * double; packed: the byte of the first sample (a multiple of four into the record) in the
+ * first SNP's record, records bytes_per_snp apart.  *invalid (device int32, zeroed by the
+ * caller) becomes 1 when an element is neither a count nor NaN.
+ */
+int32_t jb_pack_dense(const void* g, int32_t is_f32, int32_t along_snps, int64_t ld, int64_t rows,
+                      int64_t m, uint8_t* packed, int64_t bytes_per_snp, int32_t* invalid,
+                      uintptr_t stream);
+
 /* Re-pack decoded codes (m x ld_codes) into count-A1 .bed records (m x bytes_per_snp). */
 int32_t jb_pack_codes(const int8_t* codes, int64_t ld_codes, int64_t n, int64_t m,
                       uint8_t* packed, int64_t bytes_per_snp, uintptr_t stream);

@@ -44,6 +44,7 @@ SIGNATURES: dict[str, tuple] = {
     "jb_device_arch": (_i32, []),
     "jb_decode_bed": (_i32, [_p, _i64, _i64, _p, _i64, _p, _i64, _p, _u]),
     "jb_impute_f64": (_i32, [_p, _i64, _i64, _i64, _p, _p, _i64, _u]),
+    "jb_pack_dense": (_i32, [_p, _i32, _i32, _i64, _i64, _i64, _p, _i64, _p, _u]),
     "jb_pack_codes": (_i32, [_p, _i64, _i64, _i64, _p, _i64, _u]),
     "jb_kinship_f64_workspace_size": (_i64, [_i64, _i64]),
     "jb_kinship_accumulate_f64": (_i32, [_p, _i64, _i64, _i64, _p, _p, _i64, _p, _i64, _u]),

@@ -64,6 +64,20 @@ def _read_pool():
     return _READ_POOL
 
 
+def parallel_copy(src: np.ndarray, dst: np.ndarray) -> None:
+    """dst[...] = src over the leading axis, split over a few threads when large (NumPy's copy
+    releases the GIL): one thread fills pinned memory at ~8 GB/s, PCIe takes ~50."""
+    parts = min(_READ_THREADS, dst.nbytes // (1 << 20), len(dst))
+    if parts <= 1:
+        np.copyto(dst, src)
+        return
+    step = -(-len(dst) // parts)
+    futs = [_read_pool().submit(np.copyto, dst[a:a + step], src[a:a + step])
+            for a in range(0, len(dst), step)]
+    for f in futs:
+        f.result()
+
+
 class BedFile:
     """Memory-mapped SNP-major .bed records: ``records[j]`` is SNP j's packed bytes."""
 

@@ -14,8 +14,8 @@ import torch
 
 from jamma_b200 import _native
 from jamma_b200.device import empty, ptr, require_cuda, stream_handle, workspace
-from jamma_b200.engine import decode_packed, pass1_counts
-from jamma_b200.io import BedFile, apply_snp_list_mask, pack_genotypes
+from jamma_b200.engine import decode_packed, pack_on_device, pass1_counts
+from jamma_b200.io import BedFile, apply_snp_list_mask
 
 
 def snp_stats_from_counts(counts: np.ndarray, n: int, dtype=np.float32):
@@ -341,7 +341,7 @@ def compute_standardized_kinship(genotypes: np.ndarray, batch_size: int = 10000,
     g = np.asarray(genotypes)
     n = g.shape[0]
     stat_dtype = np.float32 if g.dtype == np.float32 else np.float64
-    packed = torch.from_numpy(pack_genotypes(g)).to("cuda")
+    packed = pack_on_device(g)
     K, _ = _kinship_from_packed(packed, n, batch_size, maf_threshold, miss_threshold, stat_dtype,
                                 "fp64", standardized=True)
     return K.cpu().numpy()
@@ -362,7 +362,7 @@ def compute_centered_kinship(genotypes: np.ndarray, batch_size: int = 10000,
     g = np.asarray(genotypes)
     n = g.shape[0]
     stat_dtype = np.float32 if g.dtype == np.float32 else np.float64
-    packed = torch.from_numpy(pack_genotypes(g)).to("cuda")
+    packed = pack_on_device(g)
     K, _ = _kinship_from_packed(packed, n, batch_size, maf_threshold, miss_threshold, stat_dtype,
                                 precision)
     return K.cpu().numpy()

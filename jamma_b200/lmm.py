@@ -25,7 +25,6 @@ from jamma_b200.io import (
     apply_snp_list_mask,
     format_assoc_line,
     get_plink_metadata,
-    pack_genotypes,
     snp_info_from_meta,
 )
 from jamma_b200.kinship import filter_mask, snp_stats_from_counts
@@ -335,8 +334,8 @@ def run_lmm_association_jax(
         if covariates is not None:
             covariates = np.asarray(covariates)[valid]
     n = y.shape[0]
-    packed = pack_genotypes(g)
-    packed_d = torch.from_numpy(packed).to("cuda")
+    packed_d = eng.pack_on_device(g)
+    packed = packed_d.cpu().numpy()
     _, c = eng.decode_packed(packed_d, n, None, n)
     mean_dtype = np.float32 if g.dtype == np.float32 else np.float64
     st = _Stats(c.cpu().numpy(), n, mean_dtype, maf_threshold, miss_threshold)
