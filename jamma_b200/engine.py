@@ -425,21 +425,30 @@ def pack_on_device(genotypes: np.ndarray) -> torch.Tensor:
     return packed
 
 
-def pass1_counts(bed, sample_idx: torch.Tensor | None, n: int, chunk: int = 16384) -> np.ndarray:
+# Bytes per pinned buffer of a pass over a .bed file: four reading threads' worth, and pinned
+# memory that costs 10 ms to allocate rather than the 50 of a whole 16 384-SNP chunk.
+READ_STAGE_BYTES = 32 << 20
+
+
+def pass1_counts(bed, sample_idx: torch.Tensor | None, n: int, chunk: int = 16384,
+                 keep: torch.Tensor | None = None) -> np.ndarray:
     """Per-SNP counts {n_obs, sum, n_het, n_hom2} of every SNP of a .bed file over the
     analysed samples (jamma's pass-1 statistics loop, src/jamma/lmm/runner_streaming.py:
     224-284), pipelined: while the device decodes chunk k, the host reads chunk k+1 into the
-    other pinned buffer; counts return by asynchronous copies collected one chunk behind."""
+    other pinned buffer; counts return by asynchronous copies collected one chunk behind.
+    ``keep`` (n_snps, bytes_per_snp) receives the records on the device."""
     p, bps = bed.n_snps, bed.bytes_per_snp
     out = np.empty((p, 4), dtype=np.int32)
     if p == 0:
         return out
-    step = min(chunk, p)
+    step = min(chunk, p, max(1, READ_STAGE_BYTES // max(bps, 1)))
     st = torch.cuda.current_stream()
     pin = [torch.empty((step, bps), dtype=torch.uint8, pin_memory=True) for _ in range(2)]
     pin_cnt = [torch.empty((step, 4), dtype=torch.int32, pin_memory=True) for _ in range(2)]
-    dev = [torch.empty((step, bps), dtype=torch.uint8, device="cuda") for _ in range(2)]
-    codes = torch.empty((step, n), dtype=torch.int8, device="cuda")
+    dev = [torch.empty((step, bps), dtype=torch.uint8, device="cuda") for _ in range(2)] \
+        if keep is None else None
+    ld = (n + 15) // 16 * 16  # whole words of codes per store
+    codes = torch.empty((step, ld), dtype=torch.int8, device="cuda")
     cnt = torch.empty((step, 4), dtype=torch.int32, device="cuda")
     done = [None, None]   # counts of the chunk in buffer b are in pin_cnt[b]
     rng = [None, None]    # SNP range of the chunk in buffer b, not yet collected
@@ -456,8 +465,9 @@ def pass1_counts(bed, sample_idx: torch.Tensor | None, n: int, chunk: int = 1638
         if rng[b] is not None:
             collect(b)  # chunk ci-2: its upload has read pin[b], its counts are back
         bed.read_into(s, e, pin[b].numpy())
-        dev[b][: e - s].copy_(pin[b][: e - s], non_blocking=True)
-        _native.call("jb_decode_bed", ptr(dev[b]), bps, e - s, ptr(sample_idx), n, ptr(codes), n,
+        rec = dev[b][: e - s] if keep is None else keep[s:e]
+        rec.copy_(pin[b][: e - s], non_blocking=True)
+        _native.call("jb_decode_bed", ptr(rec), bps, e - s, ptr(sample_idx), n, ptr(codes), ld,
                      ptr(cnt), stream_handle())
         pin_cnt[b][: e - s].copy_(cnt[: e - s], non_blocking=True)
         done[b] = torch.cuda.Event()

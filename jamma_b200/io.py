@@ -41,6 +41,32 @@ def get_plink_metadata(bfile) -> dict:
     }
 
 
+def _count_samples(bfile) -> int:
+    with open(Path(f"{bfile}.fam")) as f:
+        return len([r[1] for r in map(str.split, f) if r])
+
+
+def _count_snps(bfile) -> int:
+    p = 0
+    with open(Path(f"{bfile}.bim")) as f:
+        for line in f:
+            r = line.split()
+            if r:
+                int(r[3]), r[5]
+                p += 1
+    return p
+
+
+def get_plink_dimensions(bfile) -> tuple[int, int]:
+    """(n_samples, n_snps): the same checks of every .fam and .bim line as
+    ``get_plink_metadata`` without its arrays, which cost twice the parsing."""
+    try:
+        return _count_samples(bfile), _count_snps(bfile)
+    except (IndexError, ValueError):
+        get_plink_metadata(bfile)  # raises the error of the fields' own order
+        raise
+
+
 def snp_info_from_meta(meta: dict) -> list[dict]:
     """``snp_info`` dicts as the streaming runner builds them (runner_streaming.py:172-182)."""
     return [
@@ -86,8 +112,7 @@ class BedFile:
         if not self.path.exists():
             raise FileNotFoundError(f"PLINK .bed file not found: {self.path}")
         if n_samples is None or n_snps is None:
-            meta = get_plink_metadata(bfile)
-            n_samples, n_snps = meta["n_samples"], meta["n_snps"]
+            n_samples, n_snps = get_plink_dimensions(bfile)
         self.n_samples, self.n_snps = int(n_samples), int(n_snps)
         self.bytes_per_snp = (self.n_samples + 3) // 4
         # copy-on-write: the views handed to torch.from_numpy are writable, the file is never
@@ -151,6 +176,36 @@ class BedFile:
         ends = np.concatenate((cut, [idx.size]))
         for a, b in zip(starts.tolist(), ends.tolist()):
             self.read_into(int(idx[a]), int(idx[a]) + (b - a), out[a:b])
+
+
+def open_bed(bfile):
+    """(BedFile, check): the file opened with the SNP count that its length gives, and the check
+    of the .bim that ``BedFile(bfile)`` begins with, for the caller to run while the device is
+    busy.  A caller that fails before it runs it lets its error come first."""
+    path = Path(f"{bfile}.bed")
+    try:
+        n = _count_samples(bfile) if path.exists() else 0
+    except (IndexError, ValueError):
+        n = 0
+    records = path.stat().st_size - 3 if n else 0
+    bps = (n + 3) // 4
+    if records <= 0 or records % bps:
+        return BedFile(bfile), lambda: None
+    try:
+        bed = BedFile(bfile, n, records // bps)
+    except ValueError:
+        get_plink_dimensions(bfile)
+        raise
+
+    def check() -> None:
+        try:
+            ok = _count_snps(bfile) == bed.n_snps
+        except (IndexError, ValueError):
+            ok = False
+        if not ok:
+            BedFile(bfile)  # raises
+
+    return bed, check
 
 
 def read_snp_list_file(path) -> set[str]:

@@ -15,7 +15,7 @@ import torch
 from jamma_b200 import _native
 from jamma_b200.device import empty, ptr, require_cuda, stream_handle, workspace
 from jamma_b200.engine import decode_packed, pack_on_device, pass1_counts
-from jamma_b200.io import BedFile, apply_snp_list_mask
+from jamma_b200.io import BedFile, apply_snp_list_mask, open_bed
 
 
 def snp_stats_from_counts(counts: np.ndarray, n: int, dtype=np.float32):
@@ -120,9 +120,10 @@ class _KinshipExact:
         return (12 * n * n + n * (cols + 128) + lib.jb_gram_i8_workspace_size(n)
                 + lib.jb_kinship_exact_workspace_size(n, min(_KinshipExact.MAX_CHUNK, cols)))
 
-    def add(self, codes: torch.Tensor, mu64_host: np.ndarray, has_missing: bool) -> None:
+    def add(self, codes: torch.Tensor, mu64_host: np.ndarray, mu: torch.Tensor,
+            has_missing: bool) -> None:
+        """Add a chunk of decoded codes (m, ld) with its means on the host and the device."""
         m, ld = codes.shape
-        mu = torch.from_numpy(mu64_host).to("cuda")
         d = (mu64_host - np.rint(mu64_host)).astype(np.longdouble)
         self.sum_sq += np.sum(d * d)
         st, s = stream_handle(), 0
@@ -294,7 +295,7 @@ class _KinshipI8:
 def _kinship_from_packed(packed_dev: torch.Tensor, n: int, batch_size: int, maf_threshold: float,
                          miss_threshold: float, stat_dtype, precision: str = "fp64",
                          standardized: bool = False) -> tuple[torch.Tensor, int]:
-    codes, counts = decode_packed(packed_dev, n, None, n)
+    codes, counts = decode_packed(packed_dev, n, None, n, (n + 15) // 16 * 16)
     mean, miss, poly = snp_stats_from_counts(counts.cpu().numpy(), n, stat_dtype)
     keep, _ = filter_mask(mean, miss, poly, n, maf_threshold, miss_threshold)
     idx = np.where(keep)[0]
@@ -319,10 +320,46 @@ def _kinship_from_packed(packed_dev: torch.Tensor, n: int, batch_size: int, maf_
     n_missing = int((n - c[:, 0]).sum())
     acc = _fp64_accumulator(n, idx.size, n_missing, max(1, min(batch_size, 8192)))
     if isinstance(acc, _KinshipExact):
-        acc.add(codes.index_select(0, sel), c[:, 1] / np.maximum(c[:, 0], 1), n_missing > 0)
+        acc.add(codes.index_select(0, sel), c[:, 1] / np.maximum(c[:, 0], 1), mu64, n_missing > 0)
     else:
         acc.add(codes.index_select(0, sel), mu64)
     return acc.finish(), idx.size
+
+
+def _resident_records(bed: BedFile) -> torch.Tensor | None:
+    """Device buffer for all records of the file, or None when they would take more than a
+    quarter of the free memory."""
+    free = (torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved()
+            - torch.cuda.memory_allocated())
+    if bed.n_snps * bed.bytes_per_snp > free // 4:
+        return None
+    return torch.empty((bed.n_snps, bed.bytes_per_snp), dtype=torch.uint8, device="cuda")
+
+
+def _selected_records(bed: BedFile, idx: np.ndarray, step: int, kept: torch.Tensor | None):
+    """Yield the records of SNPs ``idx`` on the device, ``step`` at a time: from the records that
+    pass 1 left there, else read again through two pinned buffers."""
+    pin = [None, None]
+    done = [None, None]
+    for ci, s in enumerate(range(0, idx.size, step)):
+        sub = idx[s:s + step]
+        if kept is not None:
+            if sub[-1] - sub[0] + 1 == sub.size:  # idx increases
+                yield kept[int(sub[0]):int(sub[-1]) + 1]
+            else:
+                yield kept.index_select(0, torch.from_numpy(sub).to("cuda"))
+            continue
+        b = ci % 2
+        if pin[b] is None:
+            pin[b] = torch.empty((min(step, idx.size), bed.bytes_per_snp), dtype=torch.uint8,
+                                 pin_memory=True)
+        if done[b] is not None:
+            done[b].synchronize()
+        bed.take_into(sub, pin[b].numpy()[: sub.size])
+        rec = pin[b][: sub.size].to("cuda", non_blocking=True)
+        done[b] = torch.cuda.Event()
+        done[b].record()
+        yield rec
 
 
 def compute_standardized_kinship(genotypes: np.ndarray, batch_size: int = 10000,
@@ -383,12 +420,29 @@ def compute_kinship_from_bed(bfile, maf_threshold: float = 0.0, miss_threshold: 
         raise ValueError(f"invalid kinship mode {kinship_mode}; use 1 or 2")
     if kinship_mode == 2 and precision != "fp64":
         raise ValueError("standardized kinship (-gk 2) is computed in FP64 only")
+    if chunk_size < 1:
+        raise ValueError("chunk_size must be positive")
     require_cuda()
-    bed = BedFile(bfile)
+    bed, check = open_bed(bfile)
+    try:
+        acc = _accumulate_from_bed(bed, maf_threshold, miss_threshold, chunk_size, sample_idx,
+                                   precision, kinship_mode, ksnps_indices)
+    except Exception:
+        check()
+        raise
+    check()  # the device is still busy with the accumulation
+    K = acc.finish()
+    return K if as_device else K.cpu().numpy()
+
+
+def _accumulate_from_bed(bed: BedFile, maf_threshold, miss_threshold, chunk_size, sample_idx,
+                         precision, kinship_mode, ksnps_indices):
+    """Both passes over the file; the accumulator, its last launches still running."""
     n = bed.n_samples if sample_idx is None else len(sample_idx)
     sidx = None if sample_idx is None else torch.from_numpy(
         np.asarray(sample_idx, dtype=np.int32)).to("cuda")
-    counts = pass1_counts(bed, sidx, n, max(chunk_size, 16384))
+    kept = _resident_records(bed)
+    counts = pass1_counts(bed, sidx, n, max(chunk_size, 16384), kept)
     mean, miss, poly = snp_stats_from_counts(counts, n, np.float32)
     keep, _ = filter_mask(mean, miss, poly, n, maf_threshold, miss_threshold)
     if ksnps_indices is not None:
@@ -404,20 +458,24 @@ def compute_kinship_from_bed(bfile, maf_threshold: float = 0.0, miss_threshold: 
     else:
         acc = _fp64_accumulator(n, idx.size, int((n - counts[idx, 0]).sum()), min(chunk_size, 8192))
     exact = isinstance(acc, _KinshipExact)
-    for s in range(0, idx.size, chunk_size):
-        sub = idx[s : s + chunk_size]
-        rec = torch.from_numpy(bed.take(sub)).to("cuda")
-        codes, _ = decode_packed(rec, bed.n_samples, sidx, n)
-        c = counts[sub]
-        mu64 = torch.from_numpy(c[:, 1] / np.maximum(c[:, 0], 1)).to("cuda")
+    c = counts[idx]
+    mu_host = c[:, 1] / np.maximum(c[:, 0], 1)
+    mu_dev = torch.from_numpy(mu_host).to("cuda")
+    sd_dev = torch.from_numpy(snp_sd_from_counts(c, n)).to("cuda") if kinship_mode == 2 else None
+    # chunks of the missing-call walk: its n^2 sums are read and written once per chunk
+    step, s = max(chunk_size, 16384), 0
+    for rec in _selected_records(bed, idx, step, kept):
+        codes, _ = decode_packed(rec, bed.n_samples, sidx, n, (n + 15) // 16 * 16)
+        e = s + rec.shape[0]
+        n_missing = int((n - c[s:e, 0]).sum())
         if i8:
-            acc.add(codes, mu64, bool(np.any(c[:, 0] < n)), n_missing=int((n - c[:, 0]).sum()))
-            acc.add_sum_mu2(c[:, 1] / np.maximum(c[:, 0], 1))
+            acc.add(codes, mu_dev[s:e], n_missing > 0, n_missing=n_missing)
+            acc.add_sum_mu2(mu_host[s:e])
         elif kinship_mode == 2:
-            acc.add(codes, mu64, torch.from_numpy(snp_sd_from_counts(c, n)).to("cuda"))
+            acc.add(codes, mu_dev[s:e], sd_dev[s:e])
         elif exact:
-            acc.add(codes, c[:, 1] / np.maximum(c[:, 0], 1), bool(np.any(c[:, 0] < n)))
+            acc.add(codes, mu_host[s:e], mu_dev[s:e], n_missing > 0)
         else:
-            acc.add(codes, mu64)
-    K = acc.finish()
-    return K if as_device else K.cpu().numpy()
+            acc.add(codes, mu_dev[s:e])
+        s = e
+    return acc

@@ -45,8 +45,9 @@ def test_exact_form_against_extended_precision(n, p, miss, block, chunk, monkeyp
     has_missing = bool((c == 3).any())
     acc = kk._KinshipExact(n, p, has_missing)
     cut = p // 3 + 1
+    mu_d = torch.from_numpy(mu).cuda()
     for s in range(0, p, cut):
-        acc.add(codes[s:s + cut], mu[s:s + cut], has_missing)
+        acc.add(codes[s:s + cut], mu[s:s + cut], mu_d[s:s + cut], has_missing)
     K = acc.finish().cpu().numpy()
     assert np.array_equal(K, K.T)
     rows = np.unique(np.linspace(0, n - 1, min(n, 40)).astype(int))
