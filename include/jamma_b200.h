@@ -147,7 +147,7 @@ int32_t jb_kinship_finalize(double* K, int64_t n, int64_t ldk, double scale,
  * whose A operand is the chunk's columns col0..col0+m of the sample-major Gram operand Zs
  * (col0 and ldz multiples of 16); T/2 = M diag(mu^2/2) M^T from the same dosage-word walk
  * as jb_kinship_i8_corrections without its FMAs.  Faster than the FP64 walk of
- * jb_kinship_i8_corrections only when several per cent of the calls are missing (the
+ * jb_kinship_i8_corrections only when a fifth of the calls or more are missing (the
  * dense GEMM costs the same at any density).  workspace: jb_kinship_i8_tc_workspace_size(n,
  * m) bytes, first int32 a status word read with jb_gram_status (non-zero after a pipeline
  * timeout).

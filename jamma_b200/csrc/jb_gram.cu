@@ -228,6 +228,13 @@ __global__ void __launch_bounds__(256) codes_to_sample_major_vec_kernel(
     }
 }
 
+// hi + lo += x, exactly but for lo's own rounding.
+__device__ __forceinline__ void dd_add(double& hi, double& lo, double x) {
+    const double s = hi + x, t = s - hi;
+    lo += (hi - (s - t)) + (x - t);  // the exact rounding error of s
+    hi = s;
+}
+
 // a_i = sum_j Z_ij mu_j and b_i = sum_{j missing at i} mu_j^2 from SNP-major codes, in
 // two deterministic stages: block (256 samples) x (256 SNPs) partial sums, then an
 // ordered sum over the SNP blocks (no atomics, so results are bit-reproducible).
@@ -273,23 +280,17 @@ __global__ void kin_vectors_reduce_kernel(int64_t n, int64_t nblk, const double*
                                           double* __restrict__ b) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double sa = 0.0, sb = 0.0;
+    double sa = a[i], la = 0.0, sb = 0.0;  // one rounding of a however many blocks
     for (int64_t k = 0; k < nblk; ++k) {
-        sa += pa[k * n + i];
+        dd_add(sa, la, pa[k * n + i]);
         sb += pb[k * n + i];
     }
-    a[i] += sa;
+    a[i] = sa + la;
     b[i] += sb;
 }
 
 // The exact form's vectors: a_i = sum_j (z_ij - r_j) (mu_j - r_j) over the observed calls as an
 // unevaluated sum hi + lo, b_i = sum_{j missing at i} (mu_j - r_j)^2.
-__device__ __forceinline__ void dd_add(double& hi, double& lo, double x) {
-    const double s = hi + x, t = s - hi;
-    lo += (hi - (s - t)) + (x - t);  // the exact rounding error of s
-    hi = s;
-}
-
 __global__ void kin_exact_partial_kernel(const int8_t* __restrict__ codes, int64_t ldc, int64_t n,
                                          int64_t m, const double* __restrict__ mu,
                                          double* __restrict__ pa, double* __restrict__ pl,
@@ -677,8 +678,8 @@ struct KinREpi {
 // runs along a column.
 // K may be Q's own buffer: a block reads both tiles of Q that it writes as K, each value in the
 // thread that overwrites it or before a barrier.
-// kExact: a and s are unevaluated sums with a_lo, s_lo; the terms are added in such a sum and
-// the result is divided by p once.
+// The terms are added in an unevaluated sum of two doubles, since they are far larger than K;
+// kExact: a and s are such sums, with a_lo and s_lo.
 template <bool kExact>
 __global__ void __launch_bounds__(256) kin_finalize_i8_kernel(
     const int32_t* __restrict__ C, int64_t ldc, int64_t n, const double* __restrict__ a,
@@ -703,20 +704,14 @@ __global__ void __launch_bounds__(256) kin_finalize_i8_kernel(
             v[e] = 0.0;
             if (j < n && i <= j) {
                 // the int32 Gram holds the upper triangle (row i <= column j) at C[j*ldc + i]
-                if (kExact) {
-                    double hi = (double)C[j * ldc + i], lo = s_lo - a_lo[i] - a_lo[j];
-                    dd_add(hi, lo, s);
-                    dd_add(hi, lo, -a[i]);
-                    dd_add(hi, lo, -a[j]);
-                    double q = -b[i] - b[j];
-                    if (RT) q += RT[j * ldr + i] + t[tx][ty + 8 * e];
-                    dd_add(hi, lo, q);
-                    v[e] = (hi + lo) / p;
-                } else {
-                    double x = (double)C[j * ldc + i] - a[i] - a[j] + s - b[i] - b[j];
-                    if (RT) x += RT[j * ldr + i] + t[tx][ty + 8 * e];
-                    v[e] = x * (1.0 / p);
-                }
+                double hi = (double)C[j * ldc + i], lo = kExact ? s_lo - a_lo[i] - a_lo[j] : 0.0;
+                dd_add(hi, lo, s);
+                dd_add(hi, lo, -a[i]);
+                dd_add(hi, lo, -a[j]);
+                double q = -b[i] - b[j];
+                if (RT) q += RT[j * ldr + i] + t[tx][ty + 8 * e];
+                dd_add(hi, lo, q);
+                v[e] = (hi + lo) / p;
                 K[j * ldk + i] = v[e];
             }
         }
