@@ -3,15 +3,16 @@
 //   D (tile BM x BN, int32 in TMEM) = A_tile (BM x K) * B_tile (BN x K)^T
 //
 // A and B are K-major int8 matrices described by TMA tensor maps (128-byte K boxes,
-// 128B swizzle).  One CTA per SM walks a tile list; its 6 warps split the work:
+// 128B swizzle).  One CTA per SM walks a tile list; its warps split the work:
 //   warp 0      TMA producer: fills a STAGES-deep ring of (A, B) K-slices;
 //   warp 1      allocates TMEM (2 accumulators of BN <= 256 columns) and, from one thread,
 //               issues tcgen05.mma (M=128, N=BN, K=32) into the current accumulator,
 //               committing each consumed stage back to the producer and each finished
 //               tile to the epilogue;
-//   warps 2-5   epilogue: wait for a finished accumulator, read it with tcgen05.ld
-//               (warp w owns TMEM lanes 32*(w%4)..+31 = tile rows), hand the values to
-//               the Epi functor, then release the accumulator.
+//   warps 2..   epilogue, Epi::kWarps of them: wait for a finished accumulator and run the
+//               Epi functor, which reads it with tcgen05.ld (warp w reaches TMEM lanes
+//               32*(w%4)..+31 = tile rows) and releases it once it is read.
+// The tile list's next entry is loaded a tile ahead.
 // Integer accumulation is exact, so results do not depend on K order or tiling.
 // A launch with a gate returns at once unless *gate == gate_value.
 #pragma once
@@ -23,7 +24,16 @@ namespace tc {
 
 constexpr int kBM = 128;
 constexpr int kBK = 128;  // bytes of K per stage (one 128B swizzle row)
-constexpr int kThreads = 192;
+constexpr int kThreads = 192;  // producer, MMA issuer, four epilogue warps
+
+// An epilogue takes Epi::kWarps warps, 4 or 8: warps 2.., a multiple of four so that every TMEM
+// lane quarter (warp & 3) has as many.
+template <class Epi>
+constexpr int gemm_threads = 64 + 32 * Epi::kWarps;
+template <class Epi>
+__device__ __forceinline__ void epi_sync() {
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * Epi::kWarps) : "memory");
+}
 
 // Test hooks of the bounded pipeline waits, one copy per translation unit that launches
 // these kernels: the deadline of every wait and a switch that makes the producer issue no
@@ -54,7 +64,7 @@ struct Tile {
 };
 
 template <int BN, int STAGES, class Epi>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(gemm_threads<Epi>, 1)
     i8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const Tile* __restrict__ tiles, int n_tiles, int num_kb, Epi epi, int* err,
                    const int* gate = nullptr, int gate_value = 0) {
@@ -85,7 +95,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&tfull[a], 1);
-            mbar_init(&tempty[a], 128);
+            mbar_init(&tempty[a], 32 * Epi::kWarps);
         }
         *abort = 0;
         fence_mbar_init();
@@ -104,8 +114,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) {  // ---------------- TMA producer
             int stage = 0;
             uint32_t phase = 0;
+            Tile next = blockIdx.x < n_tiles ? tiles[blockIdx.x] : Tile{0, 0};
             for (int t = blockIdx.x; t < n_tiles && !*abort; t += gridDim.x) {
-                const Tile tl = tiles[t];
+                const Tile tl = next;  // the next tile's entry arrives during this one's loads
+                if (t + (int)gridDim.x < n_tiles) next = tiles[t + gridDim.x];
                 for (int kb = 0; kb < num_kb; ++kb) {
                     if (!mbar_wait(&empty[stage], phase ^ 1, abort, err, 1, wait_ns)) break;
                     uint8_t* sa = smem + stage * S::STAGE_BYTES;
@@ -153,25 +165,28 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (acc == 0) acc_phase ^= 1;
             }
         }
-    } else {  // ---------------- epilogue warps 2..5
-        // One thread waits for the accumulator and broadcasts the outcome, so the four
+    } else {  // ---------------- epilogue warps 2..
+        // One thread waits for the accumulator and broadcasts the outcome, so the
         // warps always take the same branch (their named barriers stay matched).
         volatile int* go = reinterpret_cast<volatile int*>(tmem_slot + 2);
         const int q = warp & 3;  // TMEM lane quarter this warp may access
         int acc = 0;
         uint32_t acc_phase = 0;
+        Tile next = blockIdx.x < n_tiles ? tiles[blockIdx.x] : Tile{0, 0};
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
             if (threadIdx.x == 64) *go = mbar_wait(&tfull[acc], acc_phase, abort, err, 4, wait_ns) ? 1 : 0;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            epi_sync<Epi>();
             const int proceed = *go;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            epi_sync<Epi>();
             if (!proceed) break;
             tc_fence_after();
-            const Tile tl = tiles[t];
+            const Tile tl = next;
+            if (t + (int)gridDim.x < n_tiles) next = tiles[t + gridDim.x];
             epi.run(tl.mb, tl.nb, tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(acc * kAcc), q,
-                    lane, epi_smem);
-            tc_fence_before();
-            mbar_arrive(&tempty[acc]);
+                    lane, epi_smem, [&] {
+                        tc_fence_before();
+                        mbar_arrive(&tempty[acc]);
+                    });
             acc ^= 1;
             if (acc == 0) acc_phase ^= 1;
         }
@@ -313,10 +328,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             const Tile tl = tiles[t];
             epi.run(2 * tl.mb + (int)rank, tl.nb,
                     tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(acc * BN), q, lane,
-                    epi_smem);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_remote(&tempty[acc], 0);
+                    epi_smem, [&] {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_remote(&tempty[acc], 0);
+                    });
             acc ^= 1;
             if (acc == 0) acc_phase ^= 1;
         }

@@ -86,13 +86,15 @@ int num_sms() {
 
 // ---------------------------------------------------------------- Gram epilogue
 struct GramEpi {
+    static constexpr int kWarps = 4;
     static constexpr int kSmem = 0;
     int32_t* C;
     int64_t ldc;
     int n;
     bool add;  // add to C instead of overwriting it
+    template <class Release>
     __device__ __forceinline__ void run(int mb, int nb, uint32_t taddr, int q, int lane,
-                                        uint8_t*) const {
+                                        uint8_t*, Release release) const {
         const int i = mb * kBM + 32 * q + lane;
 #pragma unroll 1
         for (int c0 = 0; c0 < 256; c0 += 32) {
@@ -109,6 +111,7 @@ struct GramEpi {
                 }
             }
         }
+        release();
     }
 };
 
@@ -643,12 +646,14 @@ __global__ void kin_rmask_kernel(const uint32_t* __restrict__ mask, int64_t word
 }
 
 struct KinREpi {
+    static constexpr int kWarps = 4;
     static constexpr int kSmem = 0;
     double* Q;
     int64_t ldq;
     int n;
+    template <class Release>
     __device__ __forceinline__ void run(int mb, int nb, uint32_t taddr, int q, int lane,
-                                        uint8_t*) const {
+                                        uint8_t*, Release release) const {
         const int i = mb * kBM + 32 * q + lane;
 #pragma unroll 1
         for (int c0 = 0; c0 < 256; c0 += 32) {
@@ -669,6 +674,7 @@ struct KinREpi {
                 }
             }
         }
+        release();
     }
 };
 

@@ -18,9 +18,14 @@
 // Tiles: SNPs on M, digits on N.  An A tile is 128 rows: the calls of 64 SNPs and their masks,
 // or the calls of 128 SNPs; a B tile is the 7 x 32 = 224 digit rows of 32 eigenvectors (digit
 // t of eigenvector 32 b + e at row 224 b + 32 t + e).  All digits of an output then lie in one
-// TMEM lane, 32 columns apart, and the epilogue thread of that lane adds them in registers;
+// TMEM lane, 32 columns apart, and an epilogue thread of that lane adds them in registers;
 // only the mask sums cross between lanes, through shared memory, on the way to the transposed
 // store.  N = 224 runs at the full rate of M = 128 tiles.
+// Up to n ~ 3000 a tile's products take less time than its epilogue does beside them, so eight
+// warps share it (two per TMEM lane quarter, half of the eigenvectors each), the accumulator
+// is released once it is read, and int32 becomes FP64 by an addition.  Paired tiles with four
+// warps that released at the end -> now, 8192 SNPs: n = 1024 151 -> 115 us, n = 1940 396 -> 319,
+// n = 3000 787 -> 669, n = 10 000 7.2 -> 7.2 ms; without any epilogue 78, 272, 634 us.
 #include "jb_common.cuh"
 #include "jb_gemm_i8.cuh"
 #include "jb_rotate_i8.cuh"
@@ -207,64 +212,62 @@ __global__ void __launch_bounds__(256) xfind_missing_kernel(const int8_t* __rest
 // ---------------------------------------------------------------- epilogue
 template <bool PAIRED>
 struct XEpi {
+    static constexpr int kWarps = 8;
     static constexpr int kSmem = kXEpiSmem;
     double* X;            // x~ (n x m, column-major, ld ldx)
     int64_t ldx;
     const double* scale;  // per eigenvector
     const double* mu;     // per SNP (PAIRED)
     int n, m;
+    template <class Release>
     __device__ __forceinline__ void run(int mb, int nb, uint32_t taddr, int q, int lane,
-                                        uint8_t* smem) const {
+                                        uint8_t* smem, Release release) const {
         double* S = reinterpret_cast<double*>(smem);  // [row][kXLd]
         constexpr int kRows = PAIRED ? 64 : 128;      // SNPs of the tile
+        constexpr int kPer = kRows / kWarps;          // and of a warp's stores
         constexpr double w1 = 1.0 / 256.0;
+        const int warp = (int)(threadIdx.x >> 5) - 2;
         const int row = 32 * q + lane;                // TMEM lane
-        const int i0 = nb * 32;
-        // V[e] = sum_t C_t 256^-t, smallest digit first (Horner's rule from the last digit)
-        double v[32];
-        {
-            uint32_t c[32];
-            tmem_ld32(taddr + 32 * (kXDigits - 1), c);
+        const int half = 16 * (warp >> 2);            // eigenvectors half .. half + 15 of the tile
+        const int i = nb * 32 + lane;                 // eigenvector of this lane's stores
+        const double sc = i < n ? __ldg(scale + i) : 0.0;
+        const int64_t j0 = (int64_t)mb * kRows + warp * kPer;
+        const double ml = PAIRED && lane < kPer && j0 + lane < m ? __ldg(mu + j0 + lane) : 0.0;
+        // int32 to double by an addition: a conversion has a quarter of its rate
+        auto dbl = [](uint32_t c) {
+            return __hiloint2double(0x43300000, (int)(c ^ 0x80000000u)) - 4503601774854144.0;
+        };
+        // v[e] = sum_t C_t 256^-t, smallest digit first (Horner's rule from the last digit)
+        static_assert(kXDigits == 7, "digits 5 and 6, 3 and 4, 1 and 2, then 0");
+        double v[16];
+        uint32_t c0[16], c1[16];
+        const uint32_t at = taddr + (uint32_t)half;
+        tmem_ld16x2(at + 5 * 32, at + 6 * 32, c0, c1);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = (double)(int32_t)c[e];
+        for (int e = 0; e < 16; ++e) v[e] = fma(dbl(c1[e]), w1, dbl(c0[e]));
+#pragma unroll
+        for (int t = 3; t > 0; t -= 2) {
+            tmem_ld16x2(at + 32 * t, at + 32 * (t + 1), c0, c1);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[e] = fma(fma(v[e], w1, dbl(c1[e])), w1, dbl(c0[e]));
         }
-#pragma unroll 1
-        for (int t = kXDigits - 2; t >= 0; --t) {
-            uint32_t c[32];
-            tmem_ld32(taddr + (uint32_t)(32 * t), c);
+        tmem_ld16(at, c0);
+        release();  // the accumulator has been read
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = fma(v[e], w1, (double)(int32_t)c[e]);
-        }
-        if (PAIRED) {
-            if (q >= 2) {  // mask sums of SNP row - 64
-#pragma unroll
-                for (int e = 0; e < 32; ++e) S[(row - 64) * kXLd + e] = v[e];
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (q < 2) {
-                const int j = mb * 64 + row;
-                const double u = j < m ? __ldg(mu + j) : 0.0;
-#pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                    const double vm = S[row * kXLd + e];
-                    const double sc = i0 + e < n ? __ldg(scale + i0 + e) : 0.0;
-                    S[row * kXLd + e] = sc * (vm != 0.0 ? fma(u, vm, v[e]) : v[e]);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < 32; ++e)
-                S[row * kXLd + e] = (i0 + e < n ? __ldg(scale + i0 + e) : 0.0) * v[e];
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        for (int e = 0; e < 16; ++e) S[row * kXLd + half + e] = fma(v[e], w1, dbl(c0[e]));
+        epi_sync<XEpi>();
         // row by row: 32 consecutive eigenvectors of one SNP per warp store
-#pragma unroll 4
-        for (int s = 0; s < kRows / 4; ++s) {
-            const int rr = q * (kRows / 4) + s;
-            const int64_t j = (int64_t)mb * kRows + rr;
-            if (j < m && i0 + lane < n) X[j * ldx + i0 + lane] = S[rr * kXLd + lane];
+#pragma unroll
+        for (int s = 0; s < kPer; ++s) {
+            const int rr = warp * kPer + s;
+            double x = S[rr * kXLd + lane];
+            if (PAIRED) {  // row 64 + rr: the mask sums of this SNP
+                const double vm = S[(64 + rr) * kXLd + lane], u = __shfl_sync(0xffffffffu, ml, s);
+                x = vm != 0.0 ? fma(u, vm, x) : x;
+            }
+            if (j0 + s < m && i < n) X[(j0 + s) * ldx + i] = sc * x;
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");  // the next tile rewrites S
+        epi_sync<XEpi>();  // the next tile rewrites S
     }
 };
 
@@ -324,7 +327,8 @@ int32_t launch_x(const int8_t* A, int64_t a_rows, int64_t lda, const int8_t* dig
     JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XSmem::TOTAL));
     const int64_t n_tiles = (int64_t)MB * NB;
     XEpi<PAIRED> epi{X, ldx, scale, mean, (int)n, (int)m};
-    kern<<<(unsigned)(n_tiles < num_sms() ? n_tiles : num_sms()), kThreads, XSmem::TOTAL, st>>>(
+    kern<<<(unsigned)(n_tiles < num_sms() ? n_tiles : num_sms()), gemm_threads<XEpi<PAIRED>>,
+           XSmem::TOTAL, st>>>(
         ta, tb, tiles, (int)n_tiles, (int)ceil_div(n, kBK), epi, status, gate, gate_value);
     JB_LAUNCH_CHECK("i8_gemm_kernel<rotate f64>");
     return JB_OK;

@@ -119,6 +119,7 @@ __global__ void rot_pack_pairs_kernel(const int8_t* __restrict__ codes, int64_t 
 // ---------------------------------------------------------------- epilogue
 template <bool PAIRED>
 struct RotEpi {
+    static constexpr int kWarps = 4;
     static constexpr int kSmem = kRotEpiSmem;
     double* X;             // x~ (n x m, column-major, ld ldx)
     int64_t ldx;
@@ -126,8 +127,9 @@ struct RotEpi {
     const double* mu;      // per-SNP imputation mean (PAIRED only)
     int n;
     int m;
+    template <class Release>
     __device__ __forceinline__ void run(int mb, int nb, uint32_t taddr, int q, int lane,
-                                        uint8_t* smem) const {
+                                        uint8_t* smem, Release release) const {
         double* S = reinterpret_cast<double*>(smem);  // [4][32][32]
         const int i = mb * 32 + lane;                 // eigenvector of this lane (any digit)
         constexpr int kCols = PAIRED ? 128 : 256;
@@ -167,6 +169,7 @@ struct RotEpi {
             }
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
+        release();
     }
 };
 
