@@ -294,6 +294,9 @@ __global__ void kin_vectors_reduce_kernel(int64_t n, int64_t nblk, const double*
 
 // The exact form's vectors: a_i = sum_j (z_ij - r_j) (mu_j - r_j) over the observed calls as an
 // unevaluated sum hi + lo, b_i = sum_{j missing at i} (mu_j - r_j)^2.
+// One thread per sample and block of 256 SNPs, blocks added in order by the second kernel.
+// Bound by the chain of dependent additions (6 per SNP): 0.27 + 0.05 ms for 20 000 SNPs at n =
+// 8001, 7 % of that kinship's device time.
 __global__ void kin_exact_partial_kernel(const int8_t* __restrict__ codes, int64_t ldc, int64_t n,
                                          int64_t m, const double* __restrict__ mu,
                                          double* __restrict__ pa, double* __restrict__ pl,

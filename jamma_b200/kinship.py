@@ -330,12 +330,15 @@ def _kinship_from_packed(packed_dev: torch.Tensor, n: int, batch_size: int, maf_
     return acc.finish(), idx.size
 
 
-def _resident_records(bed: BedFile) -> torch.Tensor | None:
+def _resident_records(bed: BedFile, n: int, int8: bool) -> torch.Tensor | None:
     """Device buffer for all records of the file, or None when they would take more than a
-    quarter of the free memory."""
+    quarter of the memory that the accumulation over n samples leaves free."""
     free = (torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved()
             - torch.cuda.memory_allocated())
-    if bed.n_snps * bed.bytes_per_snp > free // 4:
+    # n x n: int32 Gram, missing-call terms and result; per SNP: the whole INT8 operand, or the
+    # chunk buffers of either form
+    need = 20 * n * n + n * (bed.n_snps if int8 else 65536) + 10 * n * 16384
+    if bed.n_snps * bed.bytes_per_snp > (free - need) // 4:
         return None
     return torch.empty((bed.n_snps, bed.bytes_per_snp), dtype=torch.uint8, device="cuda")
 
@@ -445,7 +448,7 @@ def _accumulate_from_bed(bed: BedFile, maf_threshold, miss_threshold, chunk_size
     n = bed.n_samples if sample_idx is None else len(sample_idx)
     sidx = None if sample_idx is None else torch.from_numpy(
         np.asarray(sample_idx, dtype=np.int32)).to("cuda")
-    kept = _resident_records(bed)
+    kept = _resident_records(bed, n, precision == "int8")
     counts = pass1_counts(bed, sidx, n, max(chunk_size, 16384), kept)
     mean, miss, poly = snp_stats_from_counts(counts, n, np.float32)
     keep, _ = filter_mask(mean, miss, poly, n, maf_threshold, miss_threshold)

@@ -86,7 +86,7 @@ def test_resident_and_reread_records_give_the_same_matrix(tmp_path, precision, m
     real = kk._selected_records
     monkeypatch.setattr(kk, "_selected_records", lambda b, i, s, kept: real(b, i, 150, kept))
     K = run()
-    monkeypatch.setattr(kk, "_resident_records", lambda bed: None)
+    monkeypatch.setattr(kk, "_resident_records", lambda *a: None)
     assert np.array_equal(run(), K)
     X = g if sidx is None else g[sidx]
     X = X - np.nanmean(X, axis=0)
