@@ -1531,10 +1531,13 @@ int32_t launch_sq_sums(const double* AT, int64_t rows, const double* X, int64_t 
 // Lanes per pair of the series search: the most with which all pairs are resident at once (2
 // CTAs per SM), where the chain of steps of one pair sets the time; beyond one wave the
 // fewest, which do the least work.  Measured, every test, one covariate column, 16 / 8 / 4
-// lanes: 1000 pairs 76 / 80 / 105 us, 4000 pairs 144 / 87 / 108 us, 8192 pairs 259 / 158 /
-// 118 us; two columns, 16 / 8 lanes: 2000 pairs 91 / 101 us, 8192 pairs 298 / 204 us.
+// lanes: 1000 pairs 57 / 80 / 105 us, 4000 pairs 144 / 87 / 108 us, 8192 pairs 259 / 158 /
+// 118 us; two columns, 16 / 8 lanes: 2000 pairs 80 / 101 us, 8192 pairs 298 / 204 us.  32
+// lanes pay where 16 hold too many coefficients, for three and four columns: 1000 pairs and
+// three columns 102 -> 91 us (one column, with one point at a time, 64 -> 70 us).
 inline int search_lanes(int64_t pairs, int c) {
     const int64_t threads = (int64_t)2 * tc::num_sms() * kSearchThreads;
+    if (c > 2 && pairs * 32 <= threads) return 32;
     if (pairs * 16 <= threads) return 16;
     return c > 1 || pairs * 8 <= threads ? 8 : 4;
 }
@@ -1549,7 +1552,9 @@ void launch_search_as(const Params& p, cudaStream_t st) {
 template <int C, bool GUIDE>
 void launch_search(const Params& p, cudaStream_t st) {
     const int lanes = search_lanes(p.m * p.phi, C);
-    if (lanes == 16)
+    if (C > 2 && lanes == 32)
+        launch_search_as<C, (C > 2 ? 32 : 16), GUIDE>(p, st);
+    else if (lanes == 16)
         launch_search_as<C, 16, GUIDE>(p, st);
     else if (C == 1 && lanes == 4)
         launch_search_as<C, C == 1 ? 4 : 8, GUIDE>(p, st);

@@ -10,8 +10,8 @@
 // the per-probe scalar work (Pab recursion, golden-section steps) is repeated by every lane.
 //   * LP = 4 for one covariate column (72 coefficient doubles, 8 pairs per warp) and 8 for
 //     two to four (48 to 72 doubles, 4 pairs per warp) do the least work per pair; LP = 16
-//     (12 to 36 doubles) has the shortest chain of steps per pair, for chunks whose pairs
-//     cannot fill the GPU otherwise (search_lanes);
+//     (12 to 36 doubles), 32 for three and four columns, has the shortest chain of steps per
+//     pair, for chunks whose pairs cannot fill the GPU otherwise (search_lanes);
 //   * offsets of the butterfly that stay within a lane need no shuffle;
 //   * the logarithms of one likelihood are taken by different lanes of the group;
 //   * grid points are shared out one per lane after their sums, so that their Pab recursions
@@ -36,7 +36,7 @@ template <int LP>
 __device__ __forceinline__ double cheb_group(double x, int r, double (&t)[32 / LP],
                                              double (&m)[32 / LP]) {
     constexpr int V = 32 / LP;
-    static_assert(LP == 4 || LP == 8 || LP == 16, "group of 4, 8 or 16 lanes");
+    static_assert(LP == 4 || LP == 8 || LP == 16 || LP == 32, "group of 4, 8, 16 or 32 lanes");
     const double t2 = fma(2.0 * x, x, -1.0);
     const double t3 = fma(2.0 * t2, x, -x);
     double ta = fma(2.0 * t2, t2, -1.0);  // T_4
@@ -147,12 +147,12 @@ __device__ __forceinline__ void grid_xsums(const Params& p, const PairCoef<C, LP
 
 // log|H^-1| and the x-free sums of phenotype f at log-lambda s, from the expansions over the
 // golden bracket of grid index `best` (degree 24, coefficients in virtual lanes 0..24).  With
-// 16 lanes a pair's coefficients stay in registers; fewer lanes have none left and read them
+// 16 or 32 lanes a pair's coefficients stay in registers; fewer lanes have none left and read them
 // (through L1) at every probe.
 template <int C, int LP>
 struct Bracket {
     static constexpr int V = 32 / LP;
-    static constexpr bool kHold = LP == 16;
+    static constexpr bool kHold = LP >= 16;
     double mid, inv_half;
     const double* __restrict__ cb;  // of this lane
     double c[kHold ? 1 + Lay<C>::NS : 1][V];
@@ -457,7 +457,9 @@ __global__ void __launch_bounds__(kSearchThreads, 2) lmm_search_kernel(const Par
 #pragma unroll 1
     for (int g0 = 0; g0 < p.n_grid; g0 += LP) {
         double xs[L::NX];
-#pragma unroll 1
+        // 16 lanes and more: few pairs, so the chain of loads and shuffles of a point sets the
+        // time, and four points run beside each other (200 pairs 44 -> 35 us)
+#pragma unroll (LP >= 16 ? 4 : 1)
         for (int e = 0; e < LP; ++e) {
             double xe[L::NX];
             grid_xsums<C, LP>(p, g, g0 + e < p.n_grid ? g0 + e : p.n_grid - 1, r, xe);
