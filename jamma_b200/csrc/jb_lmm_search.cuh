@@ -313,76 +313,143 @@ struct Golden {
     }
 };
 
-// GUIDE: how far a probe's log-likelihood can be from its direct evaluation, over the golden
-// bracket of grid index `best`.  The series leave an absolute error in the x-dependent sums
-// (~1e-13 of the size that they have at lambda -> 0), which counts
-//   * by A = sum w0^2 / sum h w0^2, the factor by which the weighted sums have shrunk there,
-//   * by G = sum h x^2 / P_xx, the cancellation against the covariates (an uncentred, nearly
-//     constant genotype): sqrt(G) in P_xy, G in P_xx; 1 for a genotype of zeros, whose
-//     series vanish,
-//   * by the SNP's z score, through xy^2 / xx.
-// Measured over n = 500 to 20 000, h2 = 0 to 0.9 and allele frequencies 0.01 to 0.99 the
-// difference of series and direct log-likelihoods stays below 1/15 of `whole`.  It is the
-// truncated terms of degree 96 and up, so between close probes it cancels: its slope in log
-// lambda is at most 96 / 11.5 per sqrt(1 - t^2) (t the point in the domain scaled to
-// [-1, 1]), 27 for |t| < 0.95 and 96^2 / 11.5 = 801 anywhere.  What stays is rounding: 1/100
-// of `whole` (one rounding against ~1e-13) and the direct sums' own, a few ulp of a value of
-// size 1.4 n.  Anything not finite, or a bound that no longer tells golden steps apart, makes
-// the pair's search direct from the grid on.
-template <int C, int LP>
-__device__ __forceinline__ GuideTau guide_tau(const Params& p, const PairCoef<C, LP>& g, int best,
-                                              int f, int r) {
+// GUIDE: how far a series log-likelihood can be from its direct evaluation, to first order.
+// Two kinds of error enter the sums:
+//   * the truncated series: every weight 1/(lambda e + 1) is off by at most kSeriesEps at any
+//     log-lambda of the domain and any eigenvalue (the largest error over eigenvalues from
+//     -5e-6 to 1e9 is 7.3e-12, at eigenvalues near 1), so a sum of x z terms is off by at most
+//     kSeriesEps |x| |z|, with the unweighted norms: these stay what they are where the
+//     weights have shrunk the sums themselves (to 1e-5 of their size at lambda = 1e5);
+//   * rounding: `kappa` of the size of a sum's terms, weighted in the direct evaluations and
+//     in the x-free expansions, unweighted for a series.
+// Both are carried through the elimination of the covariates, whichever of them the sums
+// cancel against: G holds the weighted products of the residuals, U their unweighted ones, q
+// and q1 the sizes of the terms that make up a residual's square.  With x_r, y_r the residuals
+// at level c and b = P_xy / P_xx,
+//   |dP_xx| <= eps (|x_r|^2 + (|x| + |x_r|)^2) <= eps (3 |x_r|^2 + 2 |x|^2),
+//   |dP_xy| <= eps |x| |y_r|,   |dP_yy'| <= 2 |b| |dP_xy| + b^2 |dP_xx|,
+// and the log-likelihoods change by half of dP_xx / P_xx (REML) and n / 2 of dP_yy' / P_yy'.
+// `whole` is the series' part, `floor` the rounding.  Compared with direct evaluations in
+// double and in 80 bits, differences of probes stay below 0.15 of the bound that GuideTau
+// makes of it (n = 400 to 4000, one to four covariate columns, spread and centred-kinship
+// spectra, where the intercept keeps its weight at every lambda while all else shrinks, h2 = 0
+// to 1, allele frequencies 0.01 to 0.99, phenotypes and covariates 0 to 100 standard
+// deviations off zero).
+constexpr double kSeriesEps = 1e-11;
+struct GuideErr {
+    double whole_mle, floor_mle, whole_reml, floor_reml;
+};
+template <int C>
+__device__ __forceinline__ GuideErr guide_err(const Params& p, const double (&row0)[Lay<C>::NI],
+                                              int64_t j, int f, double ldh) {
     using L = Lay<C>;
-    const int64_t srow = (int64_t)p.phi * L::NS;
-    const double* s0 = p.S + (int64_t)best * srow + (int64_t)f * L::NS;
-    double xs[L::NX], row0[L::NI];
-    grid_xsums<C, LP>(p, g, best, r, xs);
-    assemble<C>(row0, s0, xs);
-    const PabOut<C> pb = pab_reduce<C>(row0);
-    const double A = p.S[(int64_t)p.n_grid * srow + (int64_t)f * L::NS] / s0[0];
-    const double xx = row0[L::idx(C, C)];
-    const double G = xx == 0.0 ? 1.0 : xx / pb.xx;
-    const double z2 = p.n_d * fmax(pb.yy - pb.yy1, 0.0) / pb.yy1;
-    double whole = 2.0 * A * (1e-9 * sqrt(G) * (1.0 + 0.05 * sqrt(z2)) + 2e-13 * G * (1.0 + z2));
-    if (!(A > 0.0 && G >= 0.5 && whole < 1e-2)) whole = __longlong_as_double(0x7ff0000000000000ll);
-    const double t = (p.loglam[best] - p.gmid) * p.ginv;
-    return GuideTau{whole, whole * (fabs(t) < 0.95 ? 30.0 : 900.0), 0.01 * whole + 1e-14 * p.n_d};
-}
-
-// Maximum of the grid's values with its lead over the next largest.
-struct ArgMaxLead {
-    int idx = -1;
-    double v = 0.0, v2 = 0.0;
-    bool nan = false;
-    __device__ __forceinline__ void push(int i, double x) {
-        nan = nan || isnan(x);
-        if (idx < 0) {
-            idx = i;
-            v = x;
-            v2 = -__longlong_as_double(0x7ff0000000000000ll);
-        } else if (x > v) {
-            idx = i;
-            v2 = v;
-            v = x;
-        } else {
-            v2 = x > v2 ? x : v2;
+    constexpr int R = L::R;
+    const double inf = __longlong_as_double(0x7ff0000000000000ll);
+    const double kappa = 2.2e-16 * (4.0 + sqrt(p.n_d / 32.0));
+    double G[L::NI], U[L::NI], xs[L::NX], q[R], q1[R];
+    const double* cl = p.CL + j * p.ldcl;
+#pragma unroll
+    for (int a = 0; a < C; ++a) xs[a] = __ldg(cl + a);
+    xs[C] = __ldg(p.CQ + j * p.ldcq);
+    xs[C + 1] = __ldg(cl + C + f);
+    assemble<C>(U, p.S + ((int64_t)p.n_grid * p.phi + f) * L::NS, xs);
+    const double x1 = xs[C];  // |x|^2
+#pragma unroll
+    for (int k = 0; k < L::NI; ++k) G[k] = row0[k];
+#pragma unroll
+    for (int a = 0; a < R; ++a) {
+        q[a] = fabs(G[L::idx(a, a)]);
+        q1[a] = U[L::idx(a, a)];
+    }
+    double piv = 0.0;
+    bool ok = true;
+#pragma unroll
+    for (int w = 0; w < C; ++w) {
+        const double ww = G[L::idx(w, w)], inv = 1.0 / ww, uw = U[L::idx(w, w)];
+        ok = ok && ww > 0.0;
+        piv = fma(q[w], inv, piv);
+        double l[R];
+#pragma unroll
+        for (int a = w + 1; a < R; ++a) l[a] = G[L::idx(a, w)] * inv;
+#pragma unroll
+        for (int a = w + 1; a < R; ++a) {
+            q[a] = fma(l[a] * l[a], q[w], q[a]);
+            q1[a] = fma(l[a] * l[a], q1[w], q1[a]);
+#pragma unroll
+            for (int b = a; b < R; ++b) {
+                G[L::idx(a, b)] = fma(-l[a], G[L::idx(b, w)], G[L::idx(a, b)]);
+                U[L::idx(a, b)] = fma(-l[a], U[L::idx(b, w)], fma(-l[b], fma(-l[a], uw, U[L::idx(a, w)]),
+                                                                 U[L::idx(a, b)]));
+            }
         }
     }
+    const bool none = x1 == 0.0;  // a genotype of zeros: its sums are exact
+    const double xx = none ? 1.0 : G[L::idx(C, C)], ix = 1.0 / xx;
+    const double b = fabs(G[L::idx(C, C + 1)]) * ix;
+    const double yy1 = fma(-b * b, xx, G[L::idx(C + 1, C + 1)]), ny = 0.5 * p.n_d / yy1;
+    const double xr = fmax(U[L::idx(C, C)], 0.0) + kappa * q1[C];
+    const double yr = fmax(U[L::idx(C + 1, C + 1)], 0.0) + kappa * q1[C + 1];
+    const double exx = kSeriesEps * (3.0 * xr + 2.0 * x1), exy = kSeriesEps * sqrt(x1 * yr);
+    const double fxx = kappa * sqrt(x1 * q1[C]), fxy = kappa * sqrt(x1 * q1[C + 1]);
+    GuideErr e;
+    e.whole_mle = ny * b * (2.0 * exy + b * exx);
+    e.floor_mle = ny * (kappa * (q[C + 1] + b * b * q[C]) + b * (2.0 * fxy + b * fxx)) +
+                  kappa * (p.n_d + fabs(ldh));
+    e.whole_reml = e.whole_mle + 0.5 * exx * ix;
+    e.floor_reml = e.floor_mle + 0.5 * (kappa * piv + fxx * ix);
+    // first order needs errors well below what they are errors of
+    if (!(ok && xx > 0.0 && yy1 > 0.0 && exx + fxx < 0.25 * xx)) e = GuideErr{inf, inf, inf, inf};
+    return e;
+}
+
+// The bound over the golden bracket of grid index `best`, from the two at that point: across
+// the bracket every weighted sum shrinks by at most exp(d), d the distance to its far end, so
+// `whole` (through P_xx and P_yy') grows by at most exp(2 d) and `floor` by exp(d); both
+// twice, for a difference of two probes.  The series' error is a combination of terms of degree
+// 96 and up, so between close probes it cancels: its slope is at most 96 / 11.5 per unit of
+// log-lambda within 0.95 of the domain (8.4 of the largest error, 68 at the ends, over the
+// eigenvalues above), and 1 and 2 more for P_xx and P_yy' in the denominators.
+__device__ __forceinline__ GuideTau guide_tau(const Params& p, int best, double whole, double floor) {
+    const double s = p.loglam[best];
+    const int lo = best - 1 > 0 ? best - 1 : 0;
+    const int hi = best + 1 < p.n_grid - 1 ? best + 1 : p.n_grid - 1;
+    const double d = fmax(p.loglam[hi] - s, s - p.loglam[lo]), f = exp(d);
+    const double w = 2.0 * whole * f * f;
+    return GuideTau{w, w * ((fabs(s - p.gmid) + d) * p.ginv < 0.95 ? 12.0 : 72.0), 2.0 * floor * f};
+}
+
+// Maximum of the grid's values, with the largest value that another point can have: each
+// value comes with its error bound (the same at no two points: it grows with lambda).
+struct ArgMaxLead {
+    int idx = -1;
+    double v = 0.0, e = 0.0, other = -INFINITY;
+    bool nan = false;
+    __device__ __forceinline__ void push(int i, double x, double err) {
+        nan = nan || isnan(x + err) || isnan(x - err);
+        if (idx >= 0) other = fmax(other, x > v ? v + e : x + err);
+        if (idx < 0 || x > v) {
+            idx = i;
+            v = x;
+            e = err;
+        }
+    }
+    // the point is the one that exact values would give
+    __device__ __forceinline__ bool certain() const { return !nan && v - e > other; }
     template <int GW>
     __device__ __forceinline__ void warp_reduce() {  // over groups of GW lanes
 #pragma unroll
         for (int o = GW / 2; o > 0; o >>= 1) {
             const int oi = __shfl_xor_sync(kFull, idx, o);
-            const double ov = __shfl_xor_sync(kFull, v, o), ov2 = __shfl_xor_sync(kFull, v2, o);
+            const double ov = __shfl_xor_sync(kFull, v, o), oe = __shfl_xor_sync(kFull, e, o);
+            const double oo = __shfl_xor_sync(kFull, other, o);
             nan = __shfl_xor_sync(kFull, (int)nan, o) != 0 || nan;
             if (oi < 0) continue;
-            if (idx < 0 || ov > v || (ov == v && oi < idx)) {
-                v2 = idx >= 0 && v > ov2 ? v : ov2;
-                v = ov;
-                idx = oi;
-            } else {
-                v2 = ov > v2 ? ov : v2;
-            }
+            const bool take = idx < 0 || ov > v || (ov == v && oi < idx);
+            if (idx >= 0) other = fmax(other, take ? v + e : ov + oe);
+            other = fmax(other, oo);
+            v = take ? ov : v;
+            e = take ? oe : e;
+            idx = take ? oi : idx;
         }
     }
 };
@@ -472,8 +539,17 @@ __global__ void __launch_bounds__(kSearchThreads, 2) lmm_search_kernel(const Par
             assemble<C>(row0, p.S + (int64_t)k * srow + (int64_t)f * L::NS, xs);
             const PabOut<C> pb = pab_reduce<C>(row0);
             const double ldh = p.logdet[k];
-            if (need_reml) best_reml.push(k, reml_logl<C>(pb, log_iab, ldh, p));
-            if (need_mle) best_mle.push(k, mle_logl<C>(pb, ldh, p));
+            if constexpr (GUIDE) {
+                const GuideErr er = guide_err<C>(p, row0, j, f, ldh);
+                if (need_reml)
+                    best_reml.push(k, reml_logl<C>(pb, log_iab, ldh, p),
+                                   2.0 * (er.whole_reml + er.floor_reml));
+                if (need_mle)
+                    best_mle.push(k, mle_logl<C>(pb, ldh, p), 2.0 * (er.whole_mle + er.floor_mle));
+            } else {
+                if (need_reml) best_reml.push(k, reml_logl<C>(pb, log_iab, ldh, p));
+                if (need_mle) best_mle.push(k, mle_logl<C>(pb, ldh, p));
+            }
         }
     }
     best_reml.template warp_reduce<LP>();
@@ -494,14 +570,22 @@ __global__ void __launch_bounds__(kSearchThreads, 2) lmm_search_kernel(const Par
             out_m = SearchReport{p.state + 2 * wid, 2 * wid, p.open_list, p.open_count};
             out_r = SearchReport{p.state + 2 * wid + 1, 2 * wid + 1, p.open_list, p.open_count};
         }
-        // the grid's decision: its values are as certain as the probes'
-        auto settle = [&](Golden<GUIDE>& gs, const ArgMaxLead& best, int at, const SearchReport& out) {
-            gs.tau = guide_tau<C, LP>(p, g, at, f, r);
-            gs.certain = !best.nan && best.v - best.v2 > 4.0 * (gs.tau.whole + gs.tau.floor);
+        auto err_at = [&](int at) {
+            double xs[L::NX], row0[L::NI];
+            grid_xsums<C, LP>(p, g, at, r, xs);
+            assemble<C>(row0, p.S + (int64_t)at * srow + (int64_t)f * L::NS, xs);
+            return guide_err<C>(p, row0, j, f, p.logdet[at]);
+        };
+        auto settle = [&](Golden<GUIDE>& gs, const ArgMaxLead& best, int at, double whole,
+                          double floor, const SearchReport& out) {
+            gs.tau = guide_tau(p, at, whole, floor);
+            gs.certain = best.certain();
             if (!gs.certain) out.put(SearchState{0.0, 0.0, 0.0, 0.0, -1.0}, true);
         };
-        if (need_mle) settle(gm, best_mle, bm, out_m);
-        if (need_reml) settle(gr, best_reml, br, out_r);
+        GuideErr e = err_at(bm);
+        if (need_mle) settle(gm, best_mle, bm, e.whole_mle, e.floor_mle, out_m);
+        if (__any_sync(kFull, bm != br)) e = err_at(br);
+        if (need_reml) settle(gr, best_reml, br, e.whole_reml, e.floor_reml, out_r);
     }
     double xs_m[L::NX], xs_r[L::NX], sh_m[L::NS], sh_r[L::NS], ld_m = 0.0, ld_r = 0.0;
     PabOut<C> pb_m, pb_r;
