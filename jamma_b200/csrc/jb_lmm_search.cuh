@@ -644,12 +644,15 @@ __global__ void __launch_bounds__(kSearchThreads, 2) lmm_search_kernel(const Par
 // The plain form's golden sections would take a direct FP64 pass over x per probe (46 passes
 // with a logarithm and a reciprocal per sample and pair in mode 4), although nearly every
 // decision is far from a tie.  So lmm_search_kernel<.., true> takes the decisions that its
-// series approximations settle beyond their error (guide_tau), lmm_open_kernel takes the few
+// series approximations settle beyond their error (guide_err), lmm_open_kernel takes the few
 // others by direct evaluations (lmm_close_kernel when they are many), and lmm_finish_kernel
-// makes one direct pass per pair for the
-// evaluations at the optima, whose sums the statistics use, and the score test.  Both form
-// their sums term by term in the order of eval_full, so every decision and every value is
-// the one that a search of direct evaluations gives.
+// makes one direct pass per pair for the evaluations at the optima, whose sums the statistics
+// use, and the score test.  All three form an evaluation's sums term by term in the order of
+// eval_full, and the same values come out whichever kernel takes a search.  The decisions are
+// those of a search of direct evaluations, but for two kinds that rounding settles: near-ties
+// of grid points (lmm_pairs_kernel has their x-sums from a GEMM, in another order), and REML
+// values closer than the rounding of their H = 1 determinant, whose sums (the chunk's ones row)
+// come from GEMMs of different shapes.
 // Measured, search of direct evaluations -> search + open + close + finish: 8192 SNPs, n =
 // 1940, Wald 1976 -> 264 us; 2048 SNPs, three covariate columns, n = 10 000, every test 8294
 // -> 796 us; 2048 SNPs, n = 20 000, every test 10 536 -> 832 us (and 0.4 ms more for the 97
@@ -812,24 +815,25 @@ __device__ __forceinline__ double close_golden(const Params& p, const SearchStat
     return __dmul_rn(__dadd_rn(a, b), 0.5);
 }
 
-// The grid point of a search whose grid decision is open, from the tabulated H rows: x-sums
-// of kRun points a pass by THREADS threads, added up over the warps in `red`.
-template <int C, bool REML, int THREADS>
-__device__ __forceinline__ int direct_grid(const Params& p, const double* __restrict__ x,
-                                           const double* __restrict__ y, int f,
-                                           const double (&log_iab)[C + 1], double* red) {
+// The best of a warp's share of the grid points (groups of kRun, one in `warps` from `warp` on)
+// for a search whose grid decision is open, from the tabulated H rows.  A point's x-sums are
+// added up by one warp in one order, whichever kernel takes the search and however many warps
+// share the points.
+template <int C, bool REML>
+__device__ __forceinline__ ArgMax direct_grid(const Params& p, const double* __restrict__ x,
+                                              const double* __restrict__ y, int f,
+                                              const double (&log_iab)[C + 1], int warp, int warps) {
     using L = Lay<C>;
-    constexpr int kRun = 4, kWarps = THREADS / 32;
-    const int tid = THREADS == 32 ? threadIdx.x & 31 : threadIdx.x;
+    constexpr int kRun = 4;
     ArgMax best;
 #pragma unroll 1
-    for (int g0 = 0; g0 < p.n_grid; g0 += kRun) {
+    for (int g0 = kRun * warp; g0 < p.n_grid; g0 += kRun * warps) {
         double acc[kRun][L::NX];
 #pragma unroll
         for (int e = 0; e < kRun; ++e)
 #pragma unroll
             for (int q = 0; q < L::NX; ++q) acc[e][q] = 0.0;
-        for (int64_t i = tid; i < p.n; i += THREADS) {
+        for (int64_t i = threadIdx.x & 31; i < p.n; i += 32) {
             const double xv = x[i], yv = __ldg(y + i);
             double w[C];
 #pragma unroll
@@ -849,18 +853,6 @@ __device__ __forceinline__ int direct_grid(const Params& p, const double* __rest
             double xs[L::NX], row0[L::NI];
 #pragma unroll
             for (int q = 0; q < L::NX; ++q) xs[q] = warp_sum(acc[e][q]);
-            if (THREADS > 32) {
-                __syncthreads();
-                if ((tid & 31) == 0)
-#pragma unroll
-                    for (int q = 0; q < L::NX; ++q) red[q * kWarps + (tid >> 5)] = xs[q];
-                __syncthreads();
-#pragma unroll
-                for (int q = 0; q < L::NX; ++q) {
-                    xs[q] = red[q * kWarps];
-                    for (int w = 1; w < kWarps; ++w) xs[q] += red[q * kWarps + w];
-                }
-            }
             if (g0 + e >= p.n_grid) continue;
             assemble<C>(row0, p.S + ((int64_t)(g0 + e) * p.phi + f) * L::NS, xs);
             const PabOut<C> pb = pab_reduce<C>(row0);
@@ -868,7 +860,24 @@ __device__ __forceinline__ int direct_grid(const Params& p, const double* __rest
             best.push(g0 + e, REML ? reml_logl<C>(pb, log_iab, ldh, p) : mle_logl<C>(pb, ldh, p));
         }
     }
-    return best.idx;
+    return best;
+}
+
+// The same over all warps of a CTA.
+template <int C, bool REML>
+__device__ __forceinline__ int block_grid(const Params& p, const double* __restrict__ x,
+                                          const double* __restrict__ y, int f,
+                                          const double (&log_iab)[C + 1], OpenSmem<C>& sm) {
+    constexpr int kWarps = kOpenThreads / 32;
+    const int warp = threadIdx.x >> 5;
+    ArgMax best = direct_grid<C, REML>(p, x, y, f, log_iab, warp, kWarps);
+    if ((threadIdx.x & 31) == 0) {
+        sm.sum[warp] = best.v;
+        sm.sum[kWarps + warp] = best.idx;
+    }
+    __syncthreads();
+    for (int w = 0; w < kWarps; ++w) best.merge((int)sm.sum[kWarps + w], sm.sum[w]);
+    return best.idx;  // sum is next written after barriers of block_logl
 }
 
 // Few open searches (the usual chunk: a fraction of a percent): one CTA takes one at a time,
@@ -890,7 +899,7 @@ __device__ __noinline__ double open_search(const Params& p, int64_t wid, OpenSme
     return close_golden(
         p, p.state[2 * wid + (REML ? 1 : 0)],
         [&](double s) { return block_logl<C, REML>(p, x, y, s, log_iab, sm); },
-        [&] { return direct_grid<C, REML, kOpenThreads>(p, x, y, f, log_iab, sm.h); });
+        [&] { return block_grid<C, REML>(p, x, y, f, log_iab, sm); });
 }
 
 template <int C>
@@ -920,7 +929,7 @@ __device__ __noinline__ double close_search(const Params& p, int64_t wid) {
     return close_golden(
         p, p.state[2 * wid + (REML ? 1 : 0)],
         [&](double s) { return eval_logl<C, REML>(p, x, y, s, log_iab, nullptr); },
-        [&] { return direct_grid<C, REML, 32>(p, x, y, f, log_iab, nullptr); });
+        [&] { return direct_grid<C, REML>(p, x, y, f, log_iab, 0, 1).idx; });
 }
 
 template <int C>

@@ -53,3 +53,24 @@ def test_guided_search_with_cancelling_sums(c, h2, offset):
     same = np.abs(guided["lambda_remle"] / direct["lambda_remle"] - 1) <= 1e-13
     for k in ("beta", "se"):
         np.testing.assert_allclose(guided[k][same], direct[k][same], rtol=1e-10, atol=0)
+
+
+@pytest.mark.parametrize("c", [1, 4])
+def test_a_pair_does_not_depend_on_the_other_pairs_of_its_chunk(c):
+    """Genotypes within rounding of the covariates' span: every grid decision is a matter of
+    rounding and left open, by few pairs of a chunk (one CTA each) or by many (one warp each)."""
+    import torch
+
+    from jamma_b200 import engine as eng
+
+    n = 800
+    rng = np.random.default_rng(c)
+    q = np.linalg.qr(rng.standard_normal((n, n)))[0]
+    w = np.column_stack([np.ones(n), rng.standard_normal((n, c - 1))])
+    cohort = eng.DeviceCohort(np.sort(rng.gamma(0.7, 0.5, n)), q, w, rng.standard_normal(n), 2)
+    utg = torch.from_numpy(rng.uniform(0.3, 1.7, (1500, 1))).cuda() * cohort.UtW[:1]
+    utg = utg.contiguous()
+    many = {k: v.cpu().numpy()[:, :150] for k, v in cohort.associate_rotated(utg).items()}
+    few = {k: v.cpu().numpy() for k, v in cohort.associate_rotated(utg[:150].contiguous()).items()}
+    for k in few:
+        np.testing.assert_array_equal(many[k], few[k], err_msg=k)
