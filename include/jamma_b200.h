@@ -323,6 +323,8 @@ int32_t jb_rotate_i8(const void* ozaki_ws, int64_t n, const int8_t* codes, int64
                      int64_t m, const double* mean, int32_t has_missing, double* X,
                      int64_t ldx, void* workspace, int64_t workspace_bytes,
                      uintptr_t stream);
+/* The status of the last rotation in `workspace` (its first int32, zeroed by every call).  The
+ * int32 at byte 64 holds the first failure of any call since the caller zeroed it. */
 int32_t jb_rotate_status(const void* workspace, int32_t* out, uintptr_t stream);
 
 /*

@@ -288,7 +288,8 @@ XPlanes xplanes(int64_t n) {
     L.total = L.s_off + ((n * 8 + 255) / 256) * 256;
     return L;
 }
-// Chunk scratch: status and found words, one tile list per form, the packed A operand.
+// Chunk scratch: status and found words (the caller's kFirstFailure word behind them), one tile
+// list per form, the packed A operand.
 struct XChunk {
     int64_t status, found, tiles, tiles2, a_off, lda, total;
 };
@@ -298,7 +299,7 @@ XChunk xchunk(int64_t n, int64_t m) {
     auto a256 = [](int64_t x) { return (x + 255) / 256 * 256; };
     L.lda = (n + 127) / 128 * 128;
     L.status = 0;
-    L.found = 128;
+    L.found = 4;
     L.tiles = 256;
     L.tiles2 = L.tiles + a256(MB * NB * (int64_t)sizeof(Tile));
     L.a_off = L.tiles2 + a256(ceil_div(m, 128) * NB * (int64_t)sizeof(Tile));
@@ -398,7 +399,7 @@ int32_t jb_rotate_codes_f64(const void* planes, int64_t n, const int8_t* codes, 
     int* found = reinterpret_cast<int*>(ws + L.found);
     int8_t* A = reinterpret_cast<int8_t*>(ws + L.a_off);
     cudaStream_t st = as_stream(stream);
-    JB_CUDA(cudaMemsetAsync(ws, 0, 256, st));  // status and found
+    JB_CUDA(cudaMemsetAsync(ws, 0, 8, st));  // status and found
     const int* gate = nullptr;
     // without missing calls the codes are the A operand themselves (if TMA can read them);
     // should one be missing after all, the launches after it run instead

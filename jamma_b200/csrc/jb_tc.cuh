@@ -59,6 +59,11 @@ enum : int { kErrNone = 0, kErrTimeout = 1 };
 // Default deadline of every bounded wait.
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
 
+// A workspace's status words, both the first failure: err[0] that of one call, whose entry point
+// zeroes it, and err[kFirstFailure] that of all calls since the caller zeroed it, so that a
+// failure outlives the calls after it.
+constexpr int kFirstFailure = 16;
+
 // Bounded wait.  Returns false (and has raised *abort) if the deadline (limit_ns after the
 // call) passed or another role already aborted.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort,
@@ -71,6 +76,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
         if (globaltimer_ns() - t0 > limit_ns) {
             *abort = 1;
             atomicCAS(err, 0, kErrTimeout * 100 + where);
+            atomicCAS(err + kFirstFailure, 0, kErrTimeout * 100 + where);
             return false;
         }
     }

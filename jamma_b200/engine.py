@@ -39,6 +39,8 @@ SERIES_L_MIN, SERIES_L_MAX = 1e-5, 1e5
 # The FP64 form rotates calls from seven INT8 digit planes (7 n^2 bytes beside U's 8 n^2) up to
 # this many samples
 EXACT_MAX_SAMPLES = 65536
+# Where a rotation's workspace keeps its first failure (see jb_rotate_status)
+FAILED_AT = 64
 # The FP64 form's guided search: fewest grid points at which the degree-24 bracket expansions
 # truncate below 1e-15, and fewest samples at which it is the faster one (4000 SNPs x 2
 # phenotypes, every test, direct -> guided: n = 300 1.4 -> 2.5 ms, n = 500 1.9 -> 0.7 ms)
@@ -224,6 +226,21 @@ class DeviceCohort:
         UtG = rotate(self.U, G, out=scratch)
         return self.associate_rotated(UtG, out)
 
+    def _rotation_workspace(self, need: int) -> None:
+        old = self._rot_ws
+        if old is None or old.numel() < need:
+            self._rot_ws = workspace(need)
+            self._rot_ws[:256].zero_()
+            if old is not None:  # a failure not asked for yet
+                self.failed_word().copy_(old[FAILED_AT:FAILED_AT + 4].view(torch.int32))
+
+    def failed_word(self) -> torch.Tensor | None:
+        """Device int32 (1,) that tells the first failure of any rotation since it was last
+        cleared (:meth:`rotate_status`); None where the rotation is a GEMM, which has none."""
+        if self._rot_ws is None:
+            return None
+        return self._rot_ws[FAILED_AT:FAILED_AT + 4].view(torch.int32)
+
     def rotate_codes_i8(self, codes: torch.Tensor, means: torch.Tensor, has_missing: bool,
                         out: torch.Tensor | None = None, after_rotation=None) -> torch.Tensor:
         """Mixed form: INT8 tensor-core rotation of decoded codes -> U^T G (m, n) FP64.
@@ -231,9 +248,7 @@ class DeviceCohort:
         ``after_rotation`` (optional callable) runs between the rotation GEMM and the
         series-sum GEMM, e.g. to record a CUDA event that times the rotation alone."""
         m, ld = codes.shape
-        need = _native.load().jb_rotate_i8_workspace_size(self.n, m)
-        if self._rot_ws is None or self._rot_ws.numel() < need:
-            self._rot_ws = workspace(need)
+        self._rotation_workspace(_native.load().jb_rotate_i8_workspace_size(self.n, m))
         out = out if out is not None else empty((m, self.n))
         _native.call("jb_rotate_i8", ptr(self.ozaki), self.n, ptr(codes), ld, m, ptr(means),
                      int(bool(has_missing)), ptr(out), self.n, ptr(self._rot_ws),
@@ -256,9 +271,7 @@ class DeviceCohort:
         m, ld = codes.shape
         if self.ozaki is None:
             self.ozaki = exact_split(self.U)
-        need = _native.load().jb_rotate_codes_f64_workspace_size(self.n, m)
-        if self._rot_ws is None or self._rot_ws.numel() < need:
-            self._rot_ws = workspace(need)
+        self._rotation_workspace(_native.load().jb_rotate_codes_f64_workspace_size(self.n, m))
         out = out if out is not None else empty((m, self.n))
         _native.call("jb_rotate_codes_f64", ptr(self.ozaki), self.n, ptr(codes), ld, m, ptr(means),
                      int(bool(has_missing)), ptr(out), self.n, ptr(self._rot_ws),
@@ -266,10 +279,13 @@ class DeviceCohort:
         return out
 
     def rotate_status(self) -> int:
-        st = np.zeros(1, dtype=np.int32)
-        if self._rot_ws is not None:
-            _native.call("jb_rotate_status", ptr(self._rot_ws), st.ctypes.data, stream_handle())
-        return int(st[0])
+        """The first failure (a bounded tensor-core pipeline wait that ran out) of any rotation
+        queued on this cohort since this was last asked; 0: none.  Waits for the stream."""
+        word = self.failed_word()
+        status = 0 if word is None else int(word.item())
+        if status:
+            word.zero_()
+        return status
 
     def associate_codes(self, codes: torch.Tensor, means: torch.Tensor, out: dict | None = None,
                         bufs: dict | None = None, has_missing: bool = True) -> dict:

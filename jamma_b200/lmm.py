@@ -179,8 +179,15 @@ def associate_records(cohort: eng.DeviceCohort, records, n_file: int, sample_idx
     pin_out = [{k: torch.empty((cohort.phi, step), dtype=torch.float64, pin_memory=True)
                 for k in graph.out} for _ in range(2)]
 
+    failed = cohort.failed_word()  # None where the rotation is a GEMM
+    pin_failed = [torch.zeros(1, dtype=torch.int32, pin_memory=True) for _ in range(2)]
+
     def collect(b: int, s: int, e: int) -> None:
         returned[b].synchronize()
+        if status := int(pin_failed[b][0]):
+            cohort.rotate_status()  # the cohort can be used again
+            raise RuntimeError(f"INT8 rotation pipeline reported status {status} (a bounded "
+                               "tensor-core pipeline wait ran out)")
         for k, v in pin_out[b].items():
             res[k][:, s:e] = v[:, : e - s].numpy()
         if on_chunk is not None:
@@ -189,6 +196,8 @@ def associate_records(cohort: eng.DeviceCohort, records, n_file: int, sample_idx
     def send_back(b: int, rows: int) -> None:
         for k, v in graph.out.items():
             pin_out[b][k][:, :rows].copy_(v[:, :rows], non_blocking=True)
+        if failed is not None:
+            pin_failed[b].copy_(failed, non_blocking=True)
         returned[b] = torch.cuda.Event()
         returned[b].record(main)
 
@@ -219,9 +228,6 @@ def associate_records(cohort: eng.DeviceCohort, records, n_file: int, sample_idx
         collect(*pending)
         pending = (b, s, e)
     collect(*pending)
-    if status := cohort.rotate_status():  # 0 where the rotation was a GEMM
-        raise RuntimeError(f"INT8 rotation pipeline reported status {status} (a bounded "
-                           "tensor-core pipeline wait ran out)")
     return res
 
 

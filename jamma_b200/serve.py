@@ -344,16 +344,23 @@ class GwasServer:
                     for k, v in out.items()}
             for k, v in out.items():
                 host[k].copy_(v[:, : e - s], non_blocking=True)
+            failed = torch.zeros(1, dtype=torch.int32).pin_memory()
+            if (word := act.cohort.failed_word()) is not None:
+                failed.copy_(word, non_blocking=True)
             ev = torch.cuda.Event()
             ev.record(act.stream)
-        act.inflight.append((ev, host, s, e))
+        act.inflight.append((ev, host, s, e, failed))
 
     def _poll(self, act: _Active) -> bool:
-        """Collect finished chunks; returns True when the job is complete."""
+        """Collect finished chunks; returns True when the job is complete.  Raises when a
+        chunk's rotation failed: its results are not the job's."""
         keep = []
         for item in act.inflight:
-            ev, host, s, e = item[:4]
+            ev, host, s, e, failed = item
             if ev.query():
+                if status := int(failed[0]):
+                    raise RuntimeError(f"job {act.job.job_id}: INT8 rotation pipeline reported "
+                                       f"status {status}")
                 for k, v in host.items():
                     act.job.results[k][:, s:e] = v.numpy()
                 self.snps_done += (e - s) * act.cohort.phi
@@ -361,6 +368,14 @@ class GwasServer:
                 keep.append(item)
         act.inflight = keep
         return act.next >= len(act.chunk_starts) and not act.inflight
+
+    def _give_back(self, act: _Active) -> None:
+        """Return a job's reservation of memory and cohort."""
+        self.used -= act.bytes
+        with self._lock:
+            res = self.cohorts.get(act.job.cohort_id)
+            if res is not None:
+                res.refs -= 1
 
     def step(self) -> bool:
         """One pass of the loop; returns False when it found nothing to do."""
@@ -375,11 +390,7 @@ class GwasServer:
                 except BaseException:
                     # give back the job's reservation so that a server which catches the
                     # error and keeps running admits and evicts as before
-                    self.used -= act.bytes
-                    with self._lock:
-                        res = self.cohorts.get(act.job.cohort_id)
-                        if res is not None:
-                            res.refs -= 1
+                    self._give_back(act)
                     raise
                 act.job.ready = time.perf_counter()
                 self.active.append(act)
@@ -388,12 +399,17 @@ class GwasServer:
             if act.next < len(act.chunk_starts) and len(act.inflight) < 2:
                 self._launch_chunk(act)
                 busy = True
-            if self._poll(act):
+            try:
+                done = self._poll(act)
+            except BaseException:
+                act.stream.synchronize()  # chunks in flight use the job's buffers
+                self._give_back(act)
+                self.active.remove(act)
+                raise
+            if done:
                 act.job.done = time.perf_counter()
                 self.finished.append(act.job)
-                with self._lock:
-                    self.cohorts[act.job.cohort_id].refs -= 1
-                self.used -= act.bytes
+                self._give_back(act)
                 self.active.remove(act)
                 busy = True
         return busy
