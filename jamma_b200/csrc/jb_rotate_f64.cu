@@ -375,7 +375,7 @@ int32_t jb_split_f64_prepare(const double* U, int64_t n, int64_t ldu, void* plan
 }
 
 int64_t jb_rotate_codes_f64_workspace_size(int64_t n, int64_t m) {
-    if (n <= 0 || m <= 0) return -1;
+    if (n <= 0 || m < 0) return -1;  // no SNPs: the status words
     return xchunk(n, m).total;
 }
 
