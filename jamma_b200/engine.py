@@ -138,15 +138,17 @@ class DeviceCohort:
         ev_min = float(np.min(eigenvalues) if not isinstance(eigenvalues, torch.Tensor)
                        else self.evals.min().item())
         # digit planes of U for the rotation of calls: four in the mixed form, seven exact
-        # ones in the FP64 form (where U^T G is a GEMM without them), which the first chunk of
-        # calls makes: chunks of other genotypes never need them
+        # ones in the FP64 form (where U^T G is a GEMM without them).  Made here, on the stream
+        # that makes the rest of the cohort's state: a first chunk may be queued on another
+        # stream than the second, or captured and never replayed.
         self.ozaki = None
         self.exact = precision == "fp64" and n <= EXACT_MAX_SAMPLES
         if precision == "mixed":
             self.ozaki = ozaki if ozaki is not None else ozaki_split(self.U)
-        elif (self.exact and ozaki is not None
-              and ozaki.numel() == _native.load().jb_split_f64_workspace_size(n)):
-            self.ozaki = ozaki
+        elif self.exact:
+            shared = (ozaki is not None
+                      and ozaki.numel() == _native.load().jb_split_f64_workspace_size(n))
+            self.ozaki = ozaki if shared else exact_split(self.U)
         self.code_ld = (n + 127) // 128 * 128 if precision == "mixed" or self.exact else n
         self.UtW = rotate(self.U, colmajor(W))
         self.Uty = rotate(self.U, colmajor(y))
@@ -269,8 +271,6 @@ class DeviceCohort:
                          out: torch.Tensor | None = None) -> torch.Tensor:
         """FP64 form: U^T G (m, n) of decoded codes from the exact digit planes."""
         m, ld = codes.shape
-        if self.ozaki is None:
-            self.ozaki = exact_split(self.U)
         self._rotation_workspace(_native.load().jb_rotate_codes_f64_workspace_size(self.n, m))
         out = out if out is not None else empty((m, self.n))
         _native.call("jb_rotate_codes_f64", ptr(self.ozaki), self.n, ptr(codes), ld, m, ptr(means),
