@@ -96,7 +96,8 @@ class _KinshipExact:
     MAX_CHUNK = 16384
     BLOCK = 65536
 
-    def __init__(self, n: int, p_kept: int, has_missing: bool):
+    def __init__(self, n: int, p_kept: int, has_missing: bool, chunk: int = MAX_CHUNK):
+        """``chunk``: most SNPs that one call of :meth:`add` brings."""
         self.n, self.p = n, p_kept
         self.cols = min(self.BLOCK, p_kept)
         self.ldz = (self.cols + 127) // 128 * 128
@@ -107,7 +108,8 @@ class _KinshipExact:
             (n, n), dtype=torch.float64, device="cuda")
         self.has_missing = has_missing
         lib = _native.load()
-        self.ws = workspace(lib.jb_kinship_exact_workspace_size(n, min(self.MAX_CHUNK, self.cols)))
+        self.step = min(self.MAX_CHUNK, self.cols, chunk)
+        self.ws = workspace(lib.jb_kinship_exact_workspace_size(n, self.step))
         self.gram_ws = workspace(lib.jb_gram_i8_workspace_size(n))
         self._status: list[torch.Tensor] = []
         self.col, self.blocks = 0, 0
@@ -128,7 +130,7 @@ class _KinshipExact:
         self.sum_sq += np.sum(d * d)
         st, s = stream_handle(), 0
         while s < m:
-            e = s + min(m - s, self.MAX_CHUNK, self.cols - self.col)
+            e = s + min(m - s, self.step, self.cols - self.col)
             _native.call("jb_kinship_exact_accumulate", ptr(codes[s:e]), ld, self.n, e - s, ptr(mu[s:e]),
                          int(has_missing), ptr(self.Zs), self.ldz, self.col, ptr(self.vec[0]),
                          ptr(self.vec[1]), ptr(self.vec[2]), ptr(self.Q), self.n, ptr(self.ws),
@@ -186,13 +188,15 @@ def exact_form_pays(n: int, p_kept: int, n_missing: int) -> bool:
             and float(n) * n * p_kept >= EXACT_MIN_WORK and n_missing <= density * n * p_kept)
 
 
-def _fp64_accumulator(n: int, p_kept: int, n_missing: int, batch: int):
-    """Accumulator of the FP64 centered kinship: exact form or FP64 product."""
+def _fp64_accumulator(n: int, p_kept: int, n_missing: int, batch: int,
+                      chunk: int = _KinshipExact.MAX_CHUNK):
+    """Accumulator of the FP64 centered kinship: exact form (SNPs added ``chunk`` at a time at
+    most) or FP64 product."""
     if exact_form_pays(n, p_kept, n_missing):
         free = (torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved()
                 - torch.cuda.memory_allocated())
         if _KinshipExact.device_bytes(n, p_kept) <= free // 2:
-            return _KinshipExact(n, p_kept, n_missing > 0)
+            return _KinshipExact(n, p_kept, n_missing > 0, chunk)
     return _KinshipAccumulator(n, batch)
 
 
@@ -343,6 +347,17 @@ def _resident_records(bed: BedFile, n: int, int8: bool) -> torch.Tensor | None:
     return torch.empty((bed.n_snps, bed.bytes_per_snp), dtype=torch.uint8, device="cuda")
 
 
+# compute_kinship_from_bed: the default chunk_size, and the chunk it and larger ones stand for on
+# the device: the missing-call walk reads and writes its n^2 sums once per chunk (30 011 SNPs at
+# n = 20 000 in chunks of 10 000 or 16 384: 23.3 or 20.7 ms), and two full batches of the
+# FP64 product fit.  Smaller ones are a caller's limit on the chunk's buffers and are kept.
+KINSHIP_CHUNK, KINSHIP_DEVICE_CHUNK = 10_000, 16_384
+
+
+def _device_chunk(chunk_size: int) -> int:
+    return chunk_size if chunk_size < KINSHIP_CHUNK else max(chunk_size, KINSHIP_DEVICE_CHUNK)
+
+
 def _selected_records(bed: BedFile, idx: np.ndarray, step: int, kept: torch.Tensor | None):
     """Yield the records of SNPs ``idx`` on the device, ``step`` at a time: from the records that
     pass 1 left there, else read again through two pinned buffers."""
@@ -413,7 +428,7 @@ def compute_centered_kinship(genotypes: np.ndarray, batch_size: int = 10000,
 
 
 def compute_kinship_from_bed(bfile, maf_threshold: float = 0.0, miss_threshold: float = 1.0,
-                             chunk_size: int = 10000, sample_idx: np.ndarray | None = None,
+                             chunk_size: int = KINSHIP_CHUNK, sample_idx: np.ndarray | None = None,
                              as_device: bool = False, precision: str = "fp64",
                              kinship_mode: int = 1, ksnps_indices: np.ndarray | None = None):
     """Kinship streamed from a .bed file (``compute_kinship_streaming``,
@@ -458,19 +473,20 @@ def _accumulate_from_bed(bed: BedFile, maf_threshold, miss_threshold, chunk_size
     if idx.size == 0:
         raise ValueError("No SNPs passed filtering")
     i8 = precision == "int8"
+    step = _device_chunk(chunk_size)
     if i8:
         acc = _KinshipI8(n, idx.size)
     elif kinship_mode == 2:
         acc = _KinshipAccumulator(n, min(chunk_size, 8192))
     else:
-        acc = _fp64_accumulator(n, idx.size, int((n - counts[idx, 0]).sum()), min(chunk_size, 8192))
+        acc = _fp64_accumulator(n, idx.size, int((n - counts[idx, 0]).sum()), min(chunk_size, 8192),
+                                step)
     exact = isinstance(acc, _KinshipExact)
     c = counts[idx]
     mu_host = c[:, 1] / np.maximum(c[:, 0], 1)
     mu_dev = torch.from_numpy(mu_host).to("cuda")
     sd_dev = torch.from_numpy(snp_sd_from_counts(c, n)).to("cuda") if kinship_mode == 2 else None
-    # chunks of the missing-call walk: its n^2 sums are read and written once per chunk
-    step, s = max(chunk_size, 16384), 0
+    s = 0
     for rec in _selected_records(bed, idx, step, kept):
         codes, _ = decode_packed(rec, bed.n_samples, sidx, n, (n + 15) // 16 * 16)
         e = s + rec.shape[0]
