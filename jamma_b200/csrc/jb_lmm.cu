@@ -1545,8 +1545,12 @@ inline int search_lanes(int64_t pairs, int c) {
 template <int C, int LP, bool GUIDE>
 void launch_search_as(const Params& p, cudaStream_t st) {
     const int64_t threads = p.m * p.phi * LP;
-    lmm_search_kernel<C, LP, GUIDE>
-        <<<(unsigned)ceil_div(threads, kSearchThreads), kSearchThreads, 0, st>>>(p);
+    auto kern = lmm_search_kernel<C, LP, GUIDE, kByMode>;
+    if constexpr (C >= 2 && LP == (C > 2 ? 32 : 16)) {
+        if (p.mode == 2) kern = lmm_search_kernel<C, LP, GUIDE, kMleOnly>;
+        if (p.mode == 1) kern = lmm_search_kernel<C, LP, GUIDE, kRemlOnly>;
+    }
+    kern<<<(unsigned)ceil_div(threads, kSearchThreads), kSearchThreads, 0, st>>>(p);
 }
 
 template <int C, bool GUIDE>

@@ -145,6 +145,51 @@ __device__ __forceinline__ void grid_xsums(const Params& p, const PairCoef<C, LP
     for (int q = 0; q < Lay<C>::NX; ++q) xs[q] = group_sum<LP>(w[q]);
 }
 
+// The same sums at four grid points k0 .. k0 + 3 at once, for groups of 16 or 32 lanes: each of
+// the first two steps of the butterfly halves the points that a lane goes on with, so that four
+// sums take 6 shuffles (32 lanes) in place of 20 (the grid was most of what one warp issues for
+// a pair).  Lane r is left with point k0 + r / (LP / 4).  The additions are those of group_sum,
+// bit for bit.
+template <int C, int LP>
+__device__ __forceinline__ void grid_xsums4(const Params& p, const PairCoef<C, LP>& g, int k0, int r,
+                                            double (&xs)[Lay<C>::NX]) {
+    constexpr int V = 32 / LP;
+    static_assert(LP >= 16, "two steps of the butterfly between lanes");
+    double w[Lay<C>::NX][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int k = k0 + e < p.n_grid ? k0 + e : p.n_grid - 1;
+        const double* __restrict__ tg = p.tgrid + (int64_t)k * kChebG + r;
+        double t[V][3];
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) t[v][i] = __ldg(tg + LP * v + 32 * i);
+#pragma unroll
+        for (int q = 0; q < Lay<C>::NX; ++q) {
+            double u[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                u[v] = fma(g.c[q][v][2], t[v][2], fma(g.c[q][v][1], t[v][1],
+                                                      __dmul_rn(g.c[q][v][0], t[v][0])));
+            w[q][e] = V == 2 ? __dadd_rn(u[0], u[V - 1]) : u[0];
+        }
+    }
+    const bool up1 = (r & (LP / 2)) != 0, up2 = (r & (LP / 4)) != 0;
+#pragma unroll
+    for (int q = 0; q < Lay<C>::NX; ++q) {
+        double h[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            h[e] = (up1 ? w[q][2 + e] : w[q][e]) +
+                   __shfl_xor_sync(kFull, up1 ? w[q][e] : w[q][2 + e], LP / 2);
+        double s = (up2 ? h[1] : h[0]) + __shfl_xor_sync(kFull, up2 ? h[0] : h[1], LP / 4);
+#pragma unroll
+        for (int o = LP / 8; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+        xs[q] = s;
+    }
+}
+
 // log|H^-1| and the x-free sums of phenotype f at log-lambda s, from the expansions over the
 // golden bracket of grid index `best` (degree 24, coefficients in virtual lanes 0..24).  With
 // 16 or 32 lanes a pair's coefficients stay in registers; fewer lanes have none left and read them
@@ -454,10 +499,16 @@ struct ArgMaxLead {
     }
 };
 
+// What a kernel searches: by the mode, or one likelihood only.  The latter, for chunks that
+// cannot fill the GPU, keeps the other search's state out of the registers.  With it and
+// grid_xsums4, 200 pairs of the mixed form's likelihood-ratio test, one to four columns: 35.4,
+// 40.6, 44.8, 69.6 -> 32.2, 33.0, 35.4, 41.1 us.
+constexpr int kByMode = 0, kMleOnly = 1, kRemlOnly = 2;
+
 // GUIDE = false: the mixed form, search and statistics.  GUIDE = true: the plain form's
 // decisions, as far as they are certain (modes 1, 2 and 4); lmm_open_kernel and
 // lmm_finish_kernel take over.
-template <int C, int LP, bool GUIDE>
+template <int C, int LP, bool GUIDE, int SEARCHES>
 __global__ void __launch_bounds__(kSearchThreads, 2) lmm_search_kernel(const Params p) {
     using L = Lay<C>;
     const int64_t npairs = p.m * p.phi;
@@ -469,9 +520,9 @@ __global__ void __launch_bounds__(kSearchThreads, 2) lmm_search_kernel(const Par
     const int r = threadIdx.x & (LP - 1);
     const int64_t j = wid / p.phi;
     const int f = (int)(wid % p.phi);
-    const bool need_reml = p.mode == 1 || p.mode == 4;
-    const bool need_mle = p.mode == 2 || p.mode == 4;
-    const bool need_score = !GUIDE && (p.mode == 3 || p.mode == 4);
+    const bool need_reml = SEARCHES == kByMode ? p.mode == 1 || p.mode == 4 : SEARCHES == kRemlOnly;
+    const bool need_mle = SEARCHES == kByMode ? p.mode == 2 || p.mode == 4 : SEARCHES == kMleOnly;
+    const bool need_score = !GUIDE && SEARCHES == kByMode && (p.mode == 3 || p.mode == 4);
     const int64_t o = (int64_t)f * p.m + j;
     const int64_t srow = (int64_t)p.phi * L::NS;  // stride of one S row
     const bool writer = r == 0 && valid_pair;
@@ -524,16 +575,29 @@ __global__ void __launch_bounds__(kSearchThreads, 2) lmm_search_kernel(const Par
 #pragma unroll 1
     for (int g0 = 0; g0 < p.n_grid; g0 += LP) {
         double xs[L::NX];
-        // 16 lanes and more: few pairs, so the chain of loads and shuffles of a point sets the
-        // time, and four points run beside each other (200 pairs 44 -> 35 us)
-#pragma unroll (LP >= 16 ? 4 : 1)
-        for (int e = 0; e < LP; ++e) {
-            double xe[L::NX];
-            grid_xsums<C, LP>(p, g, g0 + e < p.n_grid ? g0 + e : p.n_grid - 1, r, xe);
+        int k = g0 + r;
+        if constexpr (LP >= 16) {
+            // few pairs, so that the instructions of one warp set the time: four points at once
+            constexpr int kPasses = LP / 4;
+            const int mine = r & (kPasses - 1);
+            k = g0 + 4 * mine + r / kPasses;
+#pragma unroll 1
+            for (int e = 0; e < kPasses; ++e) {
+                if (e > 0 && g0 + 4 * e >= p.n_grid) break;
+                double xe[L::NX];
+                grid_xsums4<C, LP>(p, g, g0 + 4 * e, r, xe);
 #pragma unroll
-            for (int q = 0; q < L::NX; ++q) xs[q] = e == r || e == 0 ? xe[q] : xs[q];
+                for (int q = 0; q < L::NX; ++q) xs[q] = e == mine || e == 0 ? xe[q] : xs[q];
+            }
+        } else {
+#pragma unroll 1
+            for (int e = 0; e < LP; ++e) {
+                double xe[L::NX];
+                grid_xsums<C, LP>(p, g, g0 + e < p.n_grid ? g0 + e : p.n_grid - 1, r, xe);
+#pragma unroll
+                for (int q = 0; q < L::NX; ++q) xs[q] = e == r || e == 0 ? xe[q] : xs[q];
+            }
         }
-        const int k = g0 + r;
         if (k < p.n_grid) {
             double row0[L::NI];
             assemble<C>(row0, p.S + (int64_t)k * srow + (int64_t)f * L::NS, xs);
