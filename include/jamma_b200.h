@@ -397,9 +397,11 @@ typedef struct jb_lmm_out {
  * 2 = as 1, with the linear series sums already placed in chunk_workspace by
  * jb_lmm_chunk_series_i8 for the same chunk (only the squared sums use a DGEMM);
  * 3 = plain form, guided: the grid's and the golden sections' decisions are taken on the
- * series of precision 1 while they differ by more than the series' error bound, the others
- * and the final evaluations by direct FP64 reductions, so the optima are those of precision
- * 0; conditions as for 1, and n_grid >= 16.
+ * series of precision 1 while they differ by more than the bound of its errors and of the direct
+ * evaluations' rounding, the others and the final evaluations by direct FP64 reductions: the
+ * optima are those of precision 0, but for decisions that rounding settles there; conditions
+ * as for 1, n_grid >= 16, and no eigenvalue below -1e-6 (beyond, wide brackets' expansions lose
+ * digits).
  */
 int64_t jb_lmm_workspace_size(int64_t n, int32_t n_cvt, int32_t phi, int32_t n_grid);
 

@@ -43,8 +43,11 @@ EXACT_MAX_SAMPLES = 65536
 FAILED_AT = 64
 # The FP64 form's guided search: fewest grid points at which the degree-24 bracket expansions
 # truncate below 1e-15, and fewest samples at which it is the faster one (4000 SNPs x 2
-# phenotypes, every test, direct -> guided: n = 300 1.4 -> 2.5 ms, n = 500 1.9 -> 0.7 ms)
-GUIDE_MIN_GRID, GUIDE_MIN_SAMPLES = 16, 400
+# phenotypes, every test, direct -> guided: n = 300 1.4 -> 2.5 ms, n = 500 1.9 -> 0.7 ms).  The
+# smallest eigenvalue: a negative one has a pole of its weight at lambda = -1 / e, and at
+# e = -4.9e-6, within a factor of two of lambda = 1e5, the expansions over the last brackets of
+# 16 grid points are off by 1.1e-10 (30 points: 3e-14); at -1e-6 by less than 1e-15.
+GUIDE_MIN_GRID, GUIDE_MIN_SAMPLES, GUIDE_MIN_EIGENVALUE = 16, 400, -1e-6
 
 
 def eigh_device(K: torch.Tensor, threshold: float = 1e-10) -> tuple[torch.Tensor, torch.Tensor]:
@@ -172,7 +175,7 @@ class DeviceCohort:
                   and self.l_min >= SERIES_L_MIN and self.l_max <= SERIES_L_MAX)
         self.search = 1 if precision == "mixed" and series else 0
         self.guided = (precision == "fp64" and series and self.n_grid >= GUIDE_MIN_GRID
-                       and n >= GUIDE_MIN_SAMPLES)
+                       and n >= GUIDE_MIN_SAMPLES and ev_min >= GUIDE_MIN_EIGENVALUE)
         self._form = 3 if self.guided else self.search  # native precision argument
         self.ws = workspace(_native.load().jb_lmm_workspace_size(n, c, phi, self.n_grid))
         _native.call("jb_lmm_prepare", lmm_mode, self._form, n, c, phi, ptr(self.evals), ptr(self.UtW), n,

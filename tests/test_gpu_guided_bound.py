@@ -74,3 +74,19 @@ def test_a_pair_does_not_depend_on_the_other_pairs_of_its_chunk(c):
     few = {k: v.cpu().numpy() for k, v in cohort.associate_rotated(utg[:150].contiguous()).items()}
     for k in few:
         np.testing.assert_array_equal(many[k], few[k], err_msg=k)
+
+
+@pytest.mark.parametrize("smallest,guided", [(0.0, True), (-9e-7, True), (-1.1e-6, False),
+                                             (-4.9e-6, False)])
+def test_no_guided_search_beside_a_pole(smallest, guided):
+    """A negative eigenvalue whose weight has its pole just above lambda = 1e5, where the
+    expansions over wide brackets lose digits: the search is direct."""
+    from jamma_b200 import engine as eng
+
+    n = 500
+    rng = np.random.default_rng(0)
+    ev = np.sort(rng.gamma(0.7, 0.5, n))
+    ev[0] = smallest
+    q = np.linalg.qr(rng.standard_normal((n, n)))[0]
+    cohort = eng.DeviceCohort(ev, q, None, rng.standard_normal(n), 4, n_grid=16)
+    assert cohort.guided is guided
