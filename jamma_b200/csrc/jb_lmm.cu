@@ -1,8 +1,10 @@
 // libjamma_b200: per-SNP LMM association (FP64) on B200.
 //
-// One warp owns one (SNP, phenotype) pair and runs its whole pipeline without
-// materialising Uab: the weighted dot products of [W_1..W_c, x, y] are formed on the
-// fly from the rotated vectors while streaming them once per likelihood evaluation.
+// Uab is never materialised: the weighted dot products of [W_1..W_c, x, y] are formed on the
+// fly.  Three forms of the search:
+//
+// Direct form (precision 0, lmm_pairs_kernel below): one warp owns one (SNP, phenotype) pair
+// and streams its rotated vectors once per likelihood evaluation.
 //
 //   phase 1  one pass with two fixed weightings: H = 1 (Iab, for REML's logdet term)
 //            and H = H0 (the null-model MLE lambda, for the score test);
@@ -13,10 +15,15 @@
 //   phase 3  JAX-style golden-section refinement for MLE and REML, per-SNP lambda;
 //   epilogue Wald (from the final REML evaluation), LRT and score statistics.
 //
-// Mixed form (precision >= 1): no likelihood evaluation streams x.  The x-dependent sums
-// come from the SNP's global Chebyshev series in log lambda (chunk GEMM rows), log|H^-1|
-// and the x-free sums from per-bracket expansions; the final evaluation at each optimum
-// is one more such probe.
+// Mixed form (precision 1 and 2, lmm_search_kernel in jb_lmm_search.cuh): a pair per group of
+// 4 to 32 lanes, and no likelihood evaluation streams x but those at large lambda
+// (direct_fix).  The x-dependent sums come from the SNP's global Chebyshev series in log lambda
+// (chunk GEMM rows), log|H^-1| and the x-free sums from per-bracket expansions; the final
+// evaluation at each optimum is one more such probe.
+//
+// Guided form (precision 3, jb_lmm_search.cuh): the FP64 form's decisions on the same series
+// where they are certain, by direct evaluations where not, and one direct pass per pair for the
+// statistics.
 //
 // The sequence of evaluations, bracket rules and NaN behaviour follow
 // src/jamma/lmm/likelihood_jax.py (148-339 likelihoods, 419-598 search, 601-798
@@ -104,9 +111,9 @@ struct Params {
 constexpr int kChebN = 25;  // interpolation nodes (degree 24) per bracket
 // Global series of the x-dependent sums: each term 1/(lambda e_i + 1) is analytic in
 // t = log lambda in the strip |Im t| < pi, so over the 23-wide domain a Chebyshev series
-// converges geometrically (Bernstein ellipse rho ~ 1.31): degree 95 leaves ~1e-13 of the
-// sum's scale, far below the ~1e-9 relative error of the INT8-rotated genotypes the sums
-// are formed from, and golden-section decisions match those of exact sums.
+// converges geometrically (Bernstein ellipse rho ~ 1.31): degree 95 leaves at most 7.3e-12 of
+// a weight and, over a kinship's eigenvalues, ~1e-13 of the sum's scale, far below the ~1e-9
+// relative error of the INT8-rotated genotypes the mixed form's sums are formed from.
 constexpr int kChebG = 96;
 constexpr int kCoefPerLane = kChebG / 32;  // coefficients k = lane + 32 i held by each lane
 static_assert(kChebG % 32 == 0, "series length must be a multiple of the warp size");
